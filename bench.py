@@ -732,11 +732,9 @@ def run_variant(args):
             launch_note = ("per substep: E/H, rho, shell, update and clamp passes, and the "
                            "E_par cleaning in the last")
         if args.workload.startswith("yee"):
-            per_call = 0 if runs[0][2].problem == 1 else 1
-            launches = objs[0][2].launches_per_step() * args.steps + per_call
+            launches = objs[0][2].launches_per_step() * args.steps
             launch_note = ("per substep: shell copy, update and clamp passes; the star problem "
-                           "adds three star passes and a guard pass (box problem: one guard pass "
-                           "per call)")
+                           "adds three star passes and a guard pass")
     else:
         roof = {"kernel": "whole batched step (stage, axis and KO launches)", "bound": "hbm",
                 "achieved": BYTES_STEP * cells / (step_ms / 1e3) / 1e9, "peak": peak,

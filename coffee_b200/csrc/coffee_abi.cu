@@ -763,7 +763,7 @@ extern "C" int coffee_solver_launches_per_step(coffee_solver* s) {
   if (s && s->variant == COFFEE_VARIANT_GR) return 6;       // + two E, H passes per call
   if (s && s->variant == COFFEE_VARIANT_YEE)
     // shell + update + clamp per substep; the star boundary adds its three
-    // passes and the guard pass (the box problem: one guard pass per call)
+    // passes and the guard pass (a box with a non-periodic axis: one guard pass per call)
     return s->env->p.problem == 1 ? 21 : 9;
   if (s && s->variant == COFFEE_VARIANT_GRYEE)
     // E, H + rho + shell + update + clamp per substep, and the cleaning

@@ -404,7 +404,7 @@ __device__ __forceinline__ int periodic_targets(const GridGeom& g, int axis, int
   if (self) { out[0] = i; n = 1; }
   if (up) { if (n == 0) out[0] = i + N; else out[1] = i + N; ++n; }
   if (down) { if (n == 0) out[0] = i - N; else out[1] = i - N; ++n; }
-  return n;
+  return n < 2 ? n : 2;  // (three only where N < 2 guard)
 }
 
 // True when index i along `axis` has no periodic guard image and is not a

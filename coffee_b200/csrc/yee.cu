@@ -132,7 +132,10 @@ int yee_steps_t(const coffee_env* env, void* const A[7], void* const B0[3], void
   // the six faces of the shell: (x, y) threads over the largest face extent
   const dim3 gface = grid3(kColBlock, std::max(nx + 2, ny), std::max(ny + 2, nz), 1);
   const dim3 gshell(gface.x, gface.y, 6);
-  const dim3 gguard = grid3(kColBlock, a.g.dims[0], a.g.dims[1], 1);
+  // the guard pass: one warp per x row of the whole grid
+  const dim3 guard_block(32, 8, 1);
+  const dim3 gguard(
+      (unsigned)(((long long)a.g.dims[1] * a.g.dims[2] + guard_block.y - 1) / guard_block.y), 1, 1);
   const dim3 gstar_b = grid3(kStarBlock, a.phi[0] - a.plo[0] + 2, a.phi[1] - a.plo[1] + 2,
                              a.phi[2] - a.plo[2] + 2);
   const dim3 gstar_e = grid3(kStarBlock, a.phi[0] - a.plo[0], a.phi[1] - a.plo[1],
@@ -143,7 +146,15 @@ int yee_steps_t(const coffee_env* env, void* const A[7], void* const B0[3], void
   const bool star_pb = env->p.problem == 1;
   const T dt = (T)env->p.dt;
   T t = (T)time;
-  bool guards_synced = false;
+  // with every axis periodic each guard point is the image of an interior
+  // point, which the clamp pass writes: nothing is left for a guard pass
+  // (256^3: 0.70 ms a call saved).  On an axis of fewer than 2 guard points a
+  // point has images on both sides, of which that pass writes one: there the
+  // guard pass follows every substep.
+  bool guards_synced = a.g.periodic[0] && a.g.periodic[1] && a.g.periodic[2];
+  bool two_images = false;
+  for (int d = 0; d < 3; ++d)
+    two_images = two_images || (a.g.periodic[d] && a.g.N[d] < 2 * a.g.guard[d]);
   for (int step = 0; step < nsteps; ++step) {
     for (int sub = 0; sub < 3; ++sub) {
       const bool last = sub == 2;
@@ -182,13 +193,13 @@ int yee_steps_t(const coffee_env* env, void* const A[7], void* const B0[3], void
           else yee_star_store_kernel<T, false><<<gstar_s, kStarBlock, 0, st>>>(a);
           COFFEE_CUDA_TRY(cudaGetLastError());
         }
-        yee_guard_kernel<T, true><<<gguard, kColBlock, 0, st>>>(a);
+        yee_guard_kernel<T, true><<<gguard, guard_block, 0, st>>>(a);
         COFFEE_CUDA_TRY(cudaGetLastError());
-      } else if (!guards_synced) {
+      } else if (!guards_synced || two_images) {
         // the clamp pass wrote the images of the interior; this pass also
         // brings the guard points whose source is a non-periodic guard point
         // (corners of a mixed box) in line, after which they never change
-        yee_guard_kernel<T, false><<<gguard, kColBlock, 0, st>>>(a);
+        yee_guard_kernel<T, false><<<gguard, guard_block, 0, st>>>(a);
         COFFEE_CUDA_TRY(cudaGetLastError());
         guards_synced = true;
       }

@@ -381,10 +381,18 @@ __global__ void yee_shell_kernel(const YeeArgs<T> a, const int e_state) {
     i = face == 4 ? lo[0] - 1 : hi[0]; j = lo[1] + u; k = lo[2] + v;
   }
   const uint32_t o = (uint32_t)k * (uint32_t)a.g.sz + (uint32_t)j * (uint32_t)a.g.sy + (uint32_t)i;
+  // loads before stores: the stores may alias for all the compiler knows, and
+  // in the x faces every access is a sector of its own
+  T e[3], b[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    a.Es[c][o] = e_state ? a.E[c][o] : (T)0;
-    a.Bs[c][o] = a.B[c][o];
+    e[c] = e_state ? a.E[c][o] : (T)0;
+    b[c] = a.B[c][o];
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a.Es[c][o] = e[c];
+    a.Bs[c][o] = b[c];
   }
 }
 
@@ -696,48 +704,50 @@ __global__ void yee_star_store_kernel(const YeeArgs<T> a) {
 // periodic coordinates wrapped into the interior (the x -> y -> z plane
 // copies of the exchange compose to exactly that).  With ZERO (star
 // boundary), a point outside the interior along a non-periodic axis holds 0,
-// as the reference's copy_from of its scratch arrays leaves it.  One thread
-// per (i, j) column; interior columns visit only their guard planes.
+// as the reference's copy_from of its scratch arrays leaves it.  One warp per
+// x row, so that rows of the guard planes are copied coalesced; a row inside
+// the box along y and z visits only its guard points.  All twelve values of a
+// point pair are independent (loads before stores), so the pass waits for
+// memory once per point.
 template <typename T, bool ZERO>
-__global__ void yee_guard_kernel(const YeeArgs<T> a) {
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y);
+__global__ void __launch_bounds__(256) yee_guard_kernel(const YeeArgs<T> a) {
   const GridGeom& g = a.g;
-  if (i >= g.dims[0] || j >= g.dims[1]) return;
-  const bool xi = i >= g.lo[0] && i < g.hi[0], yi = j >= g.lo[1] && j < g.hi[1];
+  const long long row = (long long)blockIdx.x * blockDim.y + threadIdx.y;
+  if (row >= (long long)g.dims[1] * g.dims[2]) return;
+  const int k = (int)(row / g.dims[1]), j = (int)(row - (long long)k * g.dims[1]);
+  const bool yi = j >= g.lo[1] && j < g.hi[1], zi = k >= g.lo[2] && k < g.hi[2];
   auto wrap = [&](int axis, int n) {
     if (!g.periodic[axis]) return n;
     if (n < g.lo[axis]) return n + g.N[axis];
     if (n >= g.hi[axis]) return n - g.N[axis];
     return n;
   };
-  for (int k = 0; k < g.dims[2]; ++k) {
-    const bool zi = k >= g.lo[2] && k < g.hi[2];
-    if (xi && yi && zi) {  // skip the interior of the column
-      k = g.hi[2] - 1;
-      continue;
-    }
+  const int skip = yi && zi ? g.hi[0] - g.lo[0] : 0;  // interior points of the row
+  const uint32_t src =
+      (uint32_t)wrap(2, k) * (uint32_t)g.sz + (uint32_t)wrap(1, j) * (uint32_t)g.sy;
+  const uint32_t dst = (uint32_t)k * (uint32_t)g.sz + (uint32_t)j * (uint32_t)g.sy;
+  for (int q = (int)threadIdx.x; q < g.dims[0] - skip; q += (int)blockDim.x) {
+    const int i = q < g.lo[0] ? q : q + skip;
+    const bool xi = i >= g.lo[0] && i < g.hi[0];
     const bool np_out = (!xi && !g.periodic[0]) || (!yi && !g.periodic[1]) ||
                         (!zi && !g.periodic[2]);
     const bool p_out = (!xi && g.periodic[0]) || (!yi && g.periodic[1]) || (!zi && g.periodic[2]);
-    const uint32_t o = (uint32_t)k * (uint32_t)g.sz + (uint32_t)j * (uint32_t)g.sy + (uint32_t)i;
-    if (ZERO && np_out) {
+    T e[3] = {(T)0, (T)0, (T)0}, b[3] = {(T)0, (T)0, (T)0};
+    if (!(ZERO && np_out)) {
+      if (!p_out) continue;  // a non-periodic guard point: left as it is
+      // the source has every periodic coordinate inside, so this pass never
+      // writes it
+      const uint32_t o = src + (uint32_t)wrap(0, i);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        a.Eo[c][o] = (T)0;
-        a.Bo[c][o] = (T)0;
+        e[c] = a.Eo[c][o];
+        b[c] = a.Bo[c][o];
       }
-      continue;
     }
-    if (!p_out) continue;  // a non-periodic guard point: left as it is
-    // the source has every periodic coordinate inside, so this pass never
-    // writes it
-    const uint32_t q = (uint32_t)wrap(2, k) * (uint32_t)g.sz + (uint32_t)wrap(1, j) * (uint32_t)g.sy +
-                       (uint32_t)wrap(0, i);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      a.Eo[c][o] = a.Eo[c][q];
-      a.Bo[c][o] = a.Bo[c][q];
+      a.Eo[c][dst + (uint32_t)i] = e[c];
+      a.Bo[c][dst + (uint32_t)i] = b[c];
     }
   }
 }

@@ -336,3 +336,34 @@ def test_yee_one_guard_point():
     ok, rep = fp32_parity(out, list(np32), list(np64))
     print(rep)
     assert ok, rep
+
+
+@pytest.mark.parametrize("n,periodic", [((5, 7, 6), (True, True, True)),
+                                        ((33, 4, 9), (True, False, True)),
+                                        ((4, 35, 3), (False, True, False)),
+                                        ((2, 3, 2), (True, True, True))])
+def test_yee_guard_points_of_small_boxes(n, periodic):
+    """Every point, guards included, of boxes smaller than a warp's row and
+    of all mixes of axes equals the restatement's after two steps (FP64; the
+    bound is the growth of 1e-16 roundings of O(1) terms over six substeps)."""
+    p = problems.alfven_params(N=8, guard=2)
+    p.N = list(n)
+    p.size = [m / 40 for m in n]
+    p.periodic_boundary = list(periodic)
+    p.dt = 0.2 / 40
+    rng = np.random.default_rng(11)
+    shape = tuple(m + 4 for m in reversed(n))
+    U = np.concatenate([0.05 * rng.standard_normal((3, *shape)),
+                        np.array([1.0, 0.3, -0.2]).reshape(3, 1, 1, 1) +
+                        0.05 * rng.standard_normal((3, *shape)), np.zeros((1, *shape))])
+    ref = yo.yee_evolve(p, U.copy(), 2)
+    env = SimEnvironment(p)
+    data = SimData(env, np.float64)
+    data.upload(list(U))
+    s = FieldSolver(data, env)
+    s.step(0.0, 2)
+    out = data.download()
+    for o in (s, data, env):
+        o.close()
+    for c in range(6):
+        np.testing.assert_allclose(out[c], ref[c], rtol=0, atol=1e-12)
