@@ -736,12 +736,12 @@ def run_variant(args):
             launch_note = ("per substep: shell copy, update and clamp passes; the star problem "
                            "adds three star passes and a guard pass")
     else:
-        roof = {"kernel": "whole batched step (stage, axis and KO launches)", "bound": "hbm",
+        roof = {"kernel": "whole batched step (stage and KO launches)", "bound": "hbm",
                 "achieved": BYTES_STEP * cells / (step_ms / 1e3) / 1e9, "peak": peak,
                 "unit": "GB/s", "peak_kind": peak_kind, "traffic": None,
                 "algorithmic_bytes_per_step": BYTES_STEP * cells}
         launches = 13 * args.steps + 1
-        launch_note = ("5 stage + 5 axis + 1 KO + 1 axis + 1 time-advance per step (one captured "
+        launch_note = ("5 stage + 1 KO + 1 time-advance per step (one captured "
                        "CUDA graph, replayed per step), 1 axis per call")
         cfg["autotuned"] = batch.info()
     roof["frac"] = roof["achieved"] / peak

@@ -184,8 +184,8 @@ int sph_steps(const coffee_env* env, const void* tab, void* const A_[7], void* c
   const bool has_axis = c.axis_lo >= 0 || c.axis_hi >= 0;
   const T dt = c.dt;
   T t = (T)time;
-  // boundary_axis() at the start of evolve_fields (:966); idempotent after
-  // the first step, so once per call
+  // boundary_axis() at the start of evolve_fields (:966): idempotent after
+  // the first step, whose passes apply it to what they write, so once per call
   if (has_axis && nsteps > 0) {
     sph_axis_kernel<T><<<axis_blocks, 128, 0, st>>>(c, A);
     COFFEE_CUDA_TRY(cudaGetLastError());
@@ -209,20 +209,12 @@ int sph_steps(const coffee_env* env, const void* tab, void* const A_[7], void* c
                                                            (T)kBs[s], tst, flags);
       COFFEE_CUDA_TRY(cudaGetLastError());
       if (hook && (rc = hook->after(kind))) return rc;
-      if (has_axis) {
-        sph_axis_kernel<T><<<axis_blocks, 128, 0, st>>>(c, dst);
-        COFFEE_CUDA_TRY(cudaGetLastError());
-      }
     }
     int rc = hook ? hook->before(COFFEE_KERNEL_KO) : COFFEE_OK;
     if (rc) return rc;
     sph_ko_kernel<T><<<grid, block, 0, st>>>(c, Bb, A, (T)(t + dt));
     COFFEE_CUDA_TRY(cudaGetLastError());
     if (hook && (rc = hook->after(COFFEE_KERNEL_KO))) return rc;
-    if (has_axis) {
-      sph_axis_kernel<T><<<axis_blocks, 128, 0, st>>>(c, A);
-      COFFEE_CUDA_TRY(cudaGetLastError());
-    }
     t = (T)(t + dt);
   }
   return COFFEE_OK;
@@ -427,8 +419,7 @@ int sph_batch_plan_t(const SphRun* runs, int n, bool tune, cudaStream_t st, SphB
   return COFFEE_OK;
 }
 
-// The launches of one step of every run: 5 x (stage + axis), KO + axis,
-// then t += dt.  The times come from plan->tnow / tdt.
+// The launches of one step of every run: 5 stages, KO, then t += dt.  The times come from plan->tnow / tdt.
 template <typename T>
 int sph_batch_step_launches(const SphBatchPlan* pl, cudaStream_t st) {
   const auto* tab = static_cast<const SphBatchEntry<T>*>(pl->table);
@@ -445,12 +436,8 @@ int sph_batch_step_launches(const SphBatchPlan* pl, cudaStream_t st) {
       sph_stage_batch_kernel<T, false><<<pl->nblocks, block, 0, st>>>(
           tab, n, to_b, tnow, tdt, (T)kCs[s], (T)kAs[s], (T)kBs[s], s == 4);
     COFFEE_CUDA_TRY(cudaGetLastError());
-    sph_axis_batch_kernel<T><<<pl->naxis, 128, 0, st>>>(tab, n, to_b);
-    COFFEE_CUDA_TRY(cudaGetLastError());
   }
   sph_ko_batch_kernel<T><<<pl->nblocks, block, 0, st>>>(tab, n, tnow, tdt);
-  COFFEE_CUDA_TRY(cudaGetLastError());
-  sph_axis_batch_kernel<T><<<pl->naxis, 128, 0, st>>>(tab, n, 0);
   COFFEE_CUDA_TRY(cudaGetLastError());
   sph_batch_advance_kernel<T><<<(n + 127) / 128, 128, 0, st>>>(static_cast<T*>(pl->tnow), tdt, n);
   COFFEE_CUDA_TRY(cudaGetLastError());
@@ -477,8 +464,8 @@ int sph_batch_capture(SphBatchPlan* pl) {
   return COFFEE_OK;
 }
 
-// Barriers per step of the persistent kernel: 5 x (stage, axis), KO, axis.
-constexpr int kBarriersPerStep = 12;
+// Barriers per step of the persistent kernel: 5 stages, KO.
+constexpr int kBarriersPerStep = 6;
 
 // nsteps steps of the batch as cooperative launches of the persistent
 // kernel (as many steps per launch as the 32-bit arrival count allows),
@@ -498,7 +485,7 @@ int sph_batch_persistent_t(SphBatchPlan* pl, int nsteps, cudaStream_t st) {
   T* tbuf = static_cast<T*>(pl->tnow);
   const T* tdt = static_cast<const T*>(pl->tdt);
   GridSync* gs = static_cast<GridSync*>(pl->sync);
-  int n = pl->n, nb = pl->nblocks, na = pl->naxis;
+  int n = pl->n, nb = pl->nblocks;
   for (int done = 0; done < nsteps;) {
     int steps = std::min(max_steps, nsteps - done);
     // an even count leaves the current times in row 0 for the next launch
@@ -507,9 +494,8 @@ int sph_batch_persistent_t(SphBatchPlan* pl, int nsteps, cudaStream_t st) {
     COFFEE_CUDA_TRY(cudaMemsetAsync(gs, 0, sizeof(GridSync), st));
     long long lim = pl->wait_ns;
     int stall = pl->stall_block;
-    void* args[] = {(void*)&tab, (void*)&n,     (void*)&nb,  (void*)&na,  (void*)&tbuf,
-                    (void*)&tdt, (void*)&k,     (void*)&steps, (void*)&gs, (void*)&lim,
-                    (void*)&stall};
+    void* args[] = {(void*)&tab, (void*)&n,     (void*)&nb, (void*)&tbuf, (void*)&tdt,
+                    (void*)&k,   (void*)&steps, (void*)&gs, (void*)&lim,  (void*)&stall};
     COFFEE_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)sph_batch_persistent_kernel<T>,
                                                 dim3(pl->coop_grid), dim3(pl->tx, pl->ty, 1),
                                                 args, 0, st));
@@ -526,7 +512,7 @@ int sph_batch_persistent_t(SphBatchPlan* pl, int nsteps, cudaStream_t st) {
 }
 
 // nsteps evolve_fields calls of every run of the batch, each from its own
-// time (advanced in field precision by its own dt): the stage / axis / KO
+// time (advanced in field precision by its own dt): the stage / KO
 // sequence of sph_steps with one launch per phase for the whole batch.
 template <typename T>
 int sph_batch_run_t(SphBatchPlan* pl, const SphRun* runs, double* times, int nsteps,
@@ -541,7 +527,7 @@ int sph_batch_run_t(SphBatchPlan* pl, const SphRun* runs, double* times, int nst
   // pageable source: staged at once, so the vector may go out of scope
   COFFEE_CUDA_TRY(cudaMemcpyAsync(pl->tnow, t.data(), sizeof(T) * n, cudaMemcpyHostToDevice, st));
   sph_axis_batch_kernel<T><<<pl->naxis, 128, 0, st>>>(
-      static_cast<const SphBatchEntry<T>*>(pl->table), n, 0);
+      static_cast<const SphBatchEntry<T>*>(pl->table), n);
   COFFEE_CUDA_TRY(cudaGetLastError());
   if (pl->persistent) {
     int rc = sph_batch_persistent_t<T>(pl, nsteps, st);
@@ -591,7 +577,7 @@ int sph_batch_set_persistent(SphBatchPlan* pl, bool on) {
     COFFEE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, pl->tx * pl->ty, 0));
     if (per_sm < 1) return fail(COFFEE_E_CUDA, "the persistent batch kernel does not fit an SM");
     // no more CTAs than the largest phase has tiles
-    pl->coop_grid = std::max(1, std::min(per_sm * sms, std::max(pl->nblocks, pl->naxis)));
+    pl->coop_grid = std::max(1, std::min(per_sm * sms, pl->nblocks));
     cudaError_t err = cudaMalloc(&pl->sync, sizeof(GridSync));
     if (err != cudaSuccess) {
       pl->sync = nullptr;

@@ -6,9 +6,9 @@
 // arrays (i fastest).  A stage is one launch over the update box
 // [guard - shift, dims - guard + shift) of axes 0 and 1 that reads the
 // current buffer and writes the other one (the reference's rk_step1 ->
-// rk_step2 -> clamps -> point boundaries, with no intermediate arrays), plus
-// a small launch for the non-local axis boundary of the log-spherical
-// solver.  These grids are small enough (a few million points) that the
+// rk_step2 -> clamps -> point boundaries, with no intermediate arrays); the
+// non-local axis boundaries are written by the threads that own their source
+// points.  These grids are small enough (a few million points) that the
 // stencil neighbours of a warp are served from L1/L2; the kernels read
 // global memory directly.
 #pragma once
@@ -194,6 +194,59 @@ __device__ __noinline__ V7<T> sph_absorb(const SphConst<T>& c, V7<T> v, V7<T> n,
   return v;
 }
 
+// Stores the new values w of point (i, j) together with the axis boundary
+// that follows every pass (kernel_boundary_axis_sph,
+// field_solver_EZ_spherical.cu:690-748): on the theta = 0 row E_r, B_r, P take
+// the next row's values and the other components vanish, and the three rows
+// beyond the axis mirror E and B of the rows inside with the parity of each
+// component; the theta = pi row (the first guard row) likewise.  So the
+// threads of the three rows next to an axis also write their mirror rows, the
+// one next to it also the axis row, and a thread on a row that another one
+// writes stores only what the axis boundary leaves alone: nothing on the axis,
+// P beyond it (rows that are in the box with shift_ghost > 0 only).  As a
+// launch of its own, one thread per column, the boundary cost 20 us after
+// each 80 us stage at 2048 x 1024 (one chain of dependent accesses).
+template <typename T>
+__device__ __forceinline__ void sph_store(const SphConst<T>& c, const int j, const long long o,
+                                          const V7<T>& w, const F7<T>& out) {
+  // rows above theta = 0 and below theta = pi (far from an axis not on the grid)
+  const int up = c.axis_lo >= 0 ? j - c.axis_lo : 1 << 20;
+  const int down = c.axis_hi >= 0 ? c.axis_hi - j : 1 << 20;
+  if (min(up, down) > 3) {
+#pragma unroll
+    for (int a = 0; a < 7; ++a) out.p[a][o] = w.v[a];
+    return;
+  }
+  if (up == 0 || down == 0) return;
+  out.p[6][o] = w.v[6];
+  if ((up < 0 && up >= -3) || (down < 0 && down >= -3)) return;
+#pragma unroll
+  for (int a = 0; a < 6; ++a) out.p[a][o] = w.v[a];
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const int l = side == 0 ? up : down;
+    if (l < 1 || l > 3) continue;
+    const long long d = side == 0 ? -(long long)c.d0 : (long long)c.d0;  // towards the axis
+    const long long m = o + 2 * l * d;
+    out.p[0][m] = w.v[0];
+    out.p[1][m] = -w.v[1];
+    out.p[2][m] = -w.v[2];
+    out.p[3][m] = w.v[3];
+    out.p[4][m] = -w.v[4];
+    out.p[5][m] = -w.v[5];
+    if (l == 1) {
+      const long long x = o + d;
+      out.p[0][x] = w.v[0];
+      out.p[1][x] = T(0);
+      out.p[2][x] = T(0);
+      out.p[3][x] = w.v[3];
+      out.p[4][x] = T(0);
+      out.p[5][x] = T(0);
+      out.p[6][x] = w.v[6];
+    }
+  }
+}
+
 // One LSRK stage of the log-spherical solver at point (i, j):
 // kernel_compute_ElBl + kernel_rk_step1_sph + kernel_rk_step2_sph, then
 // kernel_Epar_sph, kernel_EgtB_sph, kernel_boundary_pulsar_sph and, in the
@@ -340,8 +393,7 @@ __device__ __forceinline__ void sph_stage_point(const SphConst<T>& c, const int 
     n.v[6] = T(0);
     w = sph_absorb(c, w, n, xi, rc);
   }
-#pragma unroll
-  for (int a = 0; a < 7; ++a) out.p[a][o] = w.v[a];
+  sph_store(c, j, o, w, out);
 }
 
 template <typename T, bool FIRST>
@@ -404,8 +456,7 @@ __device__ __forceinline__ void sph_ko_point(const SphConst<T>& c, const int i, 
   for (int a = 0; a < 7; ++a) w.v[a] = v[a];
   if (rc < c.radius + c.dx)
     w = sph_pulsar(c, w, rc, sc, __ldg(c.ct + j), c.y0 + c.dy * (T)(j - c.g1), tend);
-#pragma unroll
-  for (int a = 0; a < 7; ++a) out.p[a][o] = w.v[a];
+  sph_store(c, j, o, w, out);
 }
 
 template <typename T>
@@ -418,12 +469,9 @@ __global__ void __launch_bounds__(256, kSphMinBlocks) sph_ko_kernel(const __grid
   sph_ko_point(c, i, j, u, out, tend);
 }
 
-// Axis boundary of the log-spherical solver at column i
-// (kernel_boundary_axis_sph, field_solver_EZ_spherical.cu:690-748): on the
-// theta = 0 row E_r, B_r, P take the next row's values and the other
-// components vanish; the three rows beyond the axis mirror the rows inside
-// with the parity of each component.  The theta = pi row (the first guard
-// row) likewise.
+// The axis boundary of sph_store at column i of fields as they are: once per
+// call, before the first stage (the stages and KO passes apply it to what
+// they write).
 template <typename T>
 __device__ __forceinline__ void sph_axis_column(const SphConst<T>& c, const int i,
                                                 const F7<T>& u) {
@@ -434,16 +482,23 @@ __device__ __forceinline__ void sph_axis_column(const SphConst<T>& c, const int 
     if (j < 0) continue;
     const int in = side == 0 ? 1 : -1;  // direction of the rows inside
     const long long o = i + j * d0;
-    u.p[0][o] = u.p[0][o + in * d0];
-    u.p[1][o] = T(0);
-    u.p[2][o] = T(0);
-    u.p[3][o] = u.p[3][o + in * d0];
-    u.p[4][o] = T(0);
-    u.p[5][o] = T(0);
-    u.p[6][o] = u.p[6][o + in * d0];
+    T v[3][6];  // loads before stores
+#pragma unroll
     for (int l = 1; l <= 3; ++l)
 #pragma unroll
-      for (int a = 0; a < 6; ++a) u.p[a][o - in * l * d0] = par[a] * u.p[a][o + in * l * d0];
+      for (int a = 0; a < 6; ++a) v[l - 1][a] = u.p[a][o + in * l * d0];
+    const T P = u.p[6][o + in * d0];
+    u.p[0][o] = v[0][0];
+    u.p[1][o] = T(0);
+    u.p[2][o] = T(0);
+    u.p[3][o] = v[0][3];
+    u.p[4][o] = T(0);
+    u.p[5][o] = T(0);
+    u.p[6][o] = P;
+#pragma unroll
+    for (int l = 1; l <= 3; ++l)
+#pragma unroll
+      for (int a = 0; a < 6; ++a) u.p[a][o - in * l * d0] = par[a] * v[l - 1][a];
   }
 }
 
@@ -549,26 +604,24 @@ __global__ void sph_batch_advance_kernel(T* __restrict__ tnow, const T* __restri
   if (m < n) tnow[m] = batch_time(tnow[m], T(1), tdt[m]);
 }
 
-// axis boundary of every run; `on_b`: the buffer that was just written
+// axis boundary of every run's fields, once per call
 template <typename T>
-__global__ void sph_axis_batch_kernel(const SphBatchEntry<T>* __restrict__ tab, const int n,
-                                      const int on_b) {
+__global__ void sph_axis_batch_kernel(const SphBatchEntry<T>* __restrict__ tab, const int n) {
   __shared__ __align__(16) unsigned char buf[sizeof(SphBatchEntry<T>)];
   const SphBatchEntry<T>& e = sph_batch_entry(tab, n, (int)blockIdx.x, true, buf);
   if (e.c.axis_lo < 0 && e.c.axis_hi < 0) return;
   const int i = e.c.lo0 + ((int)blockIdx.x - e.axis0) * blockDim.x + threadIdx.x;
   if (i >= e.c.hi0) return;
-  sph_axis_column(e.c, i, on_b ? e.B : e.A);
+  sph_axis_column(e.c, i, e.A);
 }
 
 // ---- the whole batch step in one persistent launch ----------------------
 // One cooperative launch (every CTA resident) runs nsteps steps of every run
-// of a batch: the phases of the per-phase launches (5 x (stage, axis), KO,
-// axis), each over all runs, separated by grid-wide barriers.  In a stage or
-// KO phase the CTAs take kTicketTiles tiles at a time from a ticket counter
-// (the tiles differ in cost: star and absorbing-layer points), asking for
-// the next ticket before working on the current one; the axis phases are
-// split evenly.  On each tile a CTA runs the single-run per-point code, so
+// of a batch: the phases of the per-phase launches (5 stages, KO), each over
+// all runs, separated by grid-wide barriers.  In a phase the CTAs take
+// kTicketTiles tiles at a time from a ticket counter (the tiles differ in
+// cost: star and absorbing-layer points), asking for the next ticket before
+// working on the current one.  On each tile a CTA runs the single-run per-point code, so
 // the results are bitwise those of the per-phase launches.  The run times alternate between two
 // rows of `tbuf`: during step s the stages read row s & 1 and CTA 0 writes
 // t + dt into the other row, which the next step reads after the
@@ -642,7 +695,7 @@ __device__ __forceinline__ bool grid_barrier(GridSync* gs, unsigned q, long long
 
 template <typename T>
 __global__ void __launch_bounds__(256, kSphBatchMinBlocks) sph_batch_persistent_kernel(
-    const SphBatchEntry<T>* __restrict__ tab, const int n, const int nblocks, const int naxis,
+    const SphBatchEntry<T>* __restrict__ tab, const int n, const int nblocks,
     T* __restrict__ tbuf, const T* __restrict__ tdt, const LsrkCoef<T> k, const int nsteps,
     GridSync* __restrict__ gs, const long long limit_ns, const int stall_block) {
   __shared__ __align__(16) unsigned char buf[sizeof(SphBatchEntry<T>)];
@@ -700,17 +753,6 @@ __global__ void __launch_bounds__(256, kSphBatchMinBlocks) sph_batch_persistent_
       base = base_s;
     }
   };
-  // the axis boundary of every run on buffer B (on_b) or A, 128 columns a tile
-  auto axis = [&](const int on_b) {
-    for (int b = blockIdx.x; b < naxis; b += gridDim.x) {
-      const SphBatchEntry<T>& e = sph_batch_entry(tab, n, b, true, buf);
-      if ((e.c.axis_lo >= 0 || e.c.axis_hi >= 0) && tid < 128) {
-        const int i = e.c.lo0 + (b - e.axis0) * 128 + tid;
-        if (i < e.c.hi0) sph_axis_column(e.c, i, on_b ? e.B : e.A);
-      }
-      __syncthreads();
-    }
-  };
   for (int step = 0; step < nsteps; ++step) {
     const T* tcur = tbuf + (step & 1) * n;
     if (blockIdx.x == 0)
@@ -719,12 +761,8 @@ __global__ void __launch_bounds__(256, kSphBatchMinBlocks) sph_batch_persistent_
     for (int s = 0; s < 5; ++s) {
       tiles(s, tcur);
       if (!barrier()) return;
-      axis((s % 2 == 0) ? 1 : 0);
-      if (!barrier()) return;
     }
     tiles(5, tcur);
-    if (!barrier()) return;
-    axis(0);
     if (!barrier()) return;
   }
 }

@@ -311,3 +311,34 @@ def test_logsph_persistent_batch_wait_limit():
     batch.step(7)
     _check_batch(runs, singles)
     _close_runs(batch, runs)
+
+
+@pytest.mark.parametrize("nr,nth,shift,theta", [(33, 4, 0, (0.0, 1.0)), (20, 7, 1, (0.0, 1.0)),
+                                                (40, 9, 0, (0.0, 0.5)), (17, 12, 2, (0.3, 0.8)),
+                                                (70, 35, 0, (0.5, 1.0))])
+def test_logsph_axis_rows(nr, nth, shift, theta):
+    """The axis boundary written by the rows next to an axis: every point,
+    guards included, equals the restatement's after three steps (FP64), with
+    both axes, either or none on the grid, rows beyond the axis in the update
+    box (shift_ghost) and as few rows between the axes as are accepted."""
+    p = problems.sph_pulsar_params(nr=nr, nth=nth, guard=4 + shift, pml=4)
+    p.shift_ghost = shift
+    p.lower[1], p.size[1] = theta[0] * np.pi, (theta[1] - theta[0]) * np.pi
+    p.dt *= 0.5
+    U = np.stack(problems.sph_pulsar_fields(p, np.float64))
+    rng = np.random.default_rng(3)
+    U[:6] += 0.02 * rng.standard_normal(U[:6].shape) * np.abs(U[3])
+    ref = axo.sph_evolve(p, U.copy(), 3)
+    env = SimEnvironment(p)
+    data = SimData(env, np.float64)
+    data.upload(list(U))
+    s = FieldSolverEZSpherical(data, env)
+    s.step(0.0, 3)
+    out = data.download()
+    for o in (s, data, env):
+        o.close()
+    for f in range(7):
+        # the metric terms of the rows beside the axis, 1 / (r^3 sin), amplify
+        # FP64 roundings by at most 1e4 on these grids
+        scale = np.abs(ref[f]).max() + 1e-30
+        np.testing.assert_allclose(out[f][0], ref[f], rtol=0, atol=1e-11 * scale)
