@@ -41,6 +41,7 @@ void fill_gr_const(const coffee_env* env, GrConst<T>* c) {
   c->a = (T)p.a;
   c->dt = (T)p.dt;
   c->tau = (T)p.tau;
+  c->inv_tau = (T)1 / c->tau;
   c->ko_c = (T)(p.KOeps / 64.0);
   c->calc_current = p.calc_current;
   c->divB_clean = p.divB_clean;
@@ -134,11 +135,11 @@ int gr_steps_t(const coffee_env* env, void* ehbuf, void* const A_[7], void* cons
   }
   if (nsteps > 0 && !per_stage) {
     // the fields may have changed since the last call (upload, pointer
-    // access): E and H of both buffers, guards included; B's interior is
-    // rewritten by the first stage
-    gr_eh_kernel<T><<<gfull, kBlock, 0, st>>>(c, A, ehA, mt);
+    // access): E and H of A, and of B's guards (the first stage writes those
+    // of its interior)
+    gr_eh_kernel<T, false><<<gfull, kBlock, 0, st>>>(c, A, ehA, mt);
     COFFEE_CUDA_TRY(cudaGetLastError());
-    gr_eh_kernel<T><<<gfull, kBlock, 0, st>>>(c, Bb, ehB, mt);
+    gr_eh_kernel<T, true><<<gfull, kBlock, 0, st>>>(c, Bb, ehB, mt);
     COFFEE_CUDA_TRY(cudaGetLastError());
   }
   for (int step = 0; step < nsteps; ++step) {
@@ -151,7 +152,7 @@ int gr_steps_t(const coffee_env* env, void* ehbuf, void* const A_[7], void* cons
       if (s == 4) flags |= AX_LAST | (aux_ ? AX_AUX : 0);
       if (s == 0) flags |= AX_WRITE_UN;
       if (per_stage) {
-        gr_eh_kernel<T><<<gfull, kBlock, 0, st>>>(c, src, ehs, mt);
+        gr_eh_kernel<T, false><<<gfull, kBlock, 0, st>>>(c, src, ehs, mt);
         COFFEE_CUDA_TRY(cudaGetLastError());
       }
       const int kind = s == 0 ? COFFEE_KERNEL_STAGE_FIRST : COFFEE_KERNEL_STAGE;
@@ -196,6 +197,13 @@ int gr_check(const coffee_env* env) {
       return fail(COFFEE_E_CONFIG, "the GR solver needs guard[%d] >= shift_ghost + 3", a);
   }
   if (!(std::fabs(p.a) < 1.0)) return fail(COFFEE_E_CONFIG, "the spin a must satisfy |a| < 1");
+  // the kernels use 32-bit element offsets: an FP32 run of 2^31 points per
+  // array would need 34 arrays of 8.6 GB, more than the GPU has
+  const coffee_grid& g = env->grid;
+  const double n = (double)g.dims[0] * g.dims[1] * g.dims[2];
+  if (n >= 2147483648.0)
+    return fail(COFFEE_E_CONFIG, "%.0f points per array: the Kerr-Schild solver takes fewer than 2^31",
+                n);
   return COFFEE_OK;
 }
 

@@ -17,6 +17,7 @@
 
 #include "axisym_kernels.cuh"
 #include "ez_common.cuh"
+#include "ez_pair.cuh"
 
 namespace coffee {
 
@@ -26,7 +27,7 @@ struct GrConst {
   int lo[3], hi[3];         // update box
   int g[3];                 // guards
   T lower[3], delta[3], inv_delta[3];
-  T a, dt, tau, ko_c;
+  T a, dt, tau, inv_tau, ko_c;
   int calc_current, divB_clean, clean_ep, check_egb;
   int absorbing;
   T xl[3], xh[3];           // outer layer edges (boundary.cu:43-54)
@@ -35,14 +36,29 @@ struct GrConst {
   int nb_lo[3], nb_n[3];    // the near-horizon box of the metric table (grid indices)
 };
 
+// Reciprocals and roots of the metric: the straight-line ones of ez_pair.cuh
+// (the IEEE operations' range branches would run the metric's eight roots and
+// quotients one after another), with the ends of the range made harmless.
+template <typename T>
+__device__ __forceinline__ T metric_rcp(T x) {
+  // an overflowed denominator (r beyond 1e9) has the reciprocal 0
+  const T y = rcp_seed(x);
+  return x < (sizeof(T) == 4 ? (T)1e37 : (T)1e300) ? sfma(sfma(-x, y, (T)1), y, y) : (T)0;
+}
+template <typename T>
+__device__ __forceinline__ T metric_sqrt(T x) {
+  constexpr T lo = sizeof(T) == 4 ? (T)1e-30 : (T)1e-60, hi = sizeof(T) == 4 ? (T)1e37 : (T)1e300;
+  return x < hi ? sqrt_mid(x > lo ? x : lo) : ::sqrt(x);
+}
+
 // r of the Kerr-Schild coordinates (metric_cks_impl.hpp:17-24)
 template <typename T>
-__device__ __forceinline__ T cks_r(T a, T x, T y, T z) {
+__device__ __forceinline__ T cks_r(T a, T x, T y, T z, T tiny = Tiny<T>::v) {
   const T R2 = x * x + y * y + z * z;
   const T q = R2 - a * a;
   T s = q * q + T(4) * (a * z) * (a * z);
-  if (s < Tiny<T>::v) s = Tiny<T>::v;
-  return sqrt((q + sqrt(s)) * T(0.5));
+  if (s < tiny) s = tiny;
+  return metric_sqrt((q + metric_sqrt(s)) * T(0.5));
 }
 
 // sqrt(gamma) = sqrt(1 + 2 r^3 / (r^4 + a^2 z^2)) (:77-83)
@@ -51,70 +67,60 @@ __device__ __forceinline__ T cks_sqrt_gamma(T a, T x, T y, T z) {
   const T r = cks_r(a, x, y, z);
   T den = r * r * r * r + a * a * z * z;
   if (den < Tiny<T>::v) den = Tiny<T>::v;
-  return sqrt(T(1) + T(2) * r * r * r / den);
+  return metric_sqrt(T(1) + T(2) * r * r * r * metric_rcp(den));
 }
 
-// All metric functions at one point (metric_cks_impl.hpp:13-181), in
-// precision T with the TINY floors of the field precision TF.
+// The Kerr-Schild metric at one point (metric_cks_impl.hpp:13-181): gamma_ij =
+// delta_ij + H l_i l_j, gamma^ij = delta_ij - H/(1+H) l_i l_j, beta^i = H/(1+H)
+// l_i, alpha = 1/sqrt(1+H), sqrt(gamma) = sqrt(1+H), with H = 2 r^3 / (r^4 +
+// a^2 z^2) and l = ((r x + a y)/(r^2 + a^2), (r y - a x)/(r^2 + a^2), z/r).
+// Eight numbers instead of the eighteen components of the metric and its
+// inverse: fewer registers in kernels that have too few, and an index is
+// lowered or raised by a dot product and three fused multiply-adds.
+// Evaluated in precision T with the TINY floors of the field precision TF.
 template <typename T, typename TF = T>
 struct Cks {
-  T r, alpha, sg;
-  T bu[3];
-  T gd11, gd12, gd13, gd22, gd23, gd33;
-  T gu11, gu12, gu13, gu22, gu23, gu33;
+  T r, H, hb, alpha, sg;  // hb = H / (1 + H)
+  T l[3];
 
   Cks() = default;
   __device__ __forceinline__ Cks(T a, T x, T y, T z) {
     constexpr T tiny = (T)Tiny<TF>::v;
-    {
-      const T R2 = x * x + y * y + z * z;
-      const T q = R2 - a * a;
-      T s = q * q + T(4) * (a * z) * (a * z);
-      if (s < tiny) s = tiny;
-      r = sqrt((q + sqrt(s)) * T(0.5));
-    }
-    const T r2 = r * r, r3 = r2 * r, r4 = r2 * r2;
-    const T aa = a * a, azz = aa * z * z;
-    T den = r4 + azz;
+    r = cks_r(a, x, y, z, tiny);
+    const T r2 = r * r, aa = a * a;
+    T den = r2 * r2 + aa * z * z;
     if (den < tiny) den = tiny;
-    T denu = T(2) * r3 + r4 + azz;
-    if (denu < tiny) denu = tiny;
     T ar = aa + r2;
-    T ar2 = ar * ar;
     if (ar < tiny) ar = tiny;
-    if (ar2 < tiny) ar2 = tiny;
-    const T lx = r * x + a * y, ly = -a * x + r * y;
-    const T iden = T(1) / den, idenu = T(1) / denu, iar = T(1) / ar, iar2 = T(1) / ar2;
-    const T gam = T(1) + T(2) * r3 * iden;
-    sg = sqrt(gam);
-    alpha = sqrt(T(1) / gam);
-    bu[0] = T(2) * r3 * lx * iar * idenu;
-    bu[1] = T(2) * r3 * ly * iar * idenu;
-    bu[2] = T(2) * r2 * z * idenu;
-    const T hd = T(2) * r3 * iar2 * iden, hu = T(2) * r3 * iar2 * idenu;
-    const T kd = T(2) * r2 * iar * iden, ku = T(2) * r2 * iar * idenu;
-    gd11 = T(1) + hd * lx * lx;
-    gd12 = hd * lx * ly;
-    gd13 = kd * lx * z;
-    gd22 = T(1) + hd * ly * ly;
-    gd23 = kd * ly * z;
-    gd33 = T(1) + T(2) * r * z * z * iden;
-    gu11 = T(1) - hu * lx * lx;
-    gu12 = -hu * lx * ly;
-    gu13 = -ku * lx * z;
-    gu22 = T(1) - hu * ly * ly;
-    gu23 = -ku * ly * z;
-    gu33 = T(1) - T(2) * r * z * z * idenu;
+    const T iar = metric_rcp(ar);
+    l[0] = (r * x + a * y) * iar;
+    l[1] = (r * y - a * x) * iar;
+    l[2] = z * metric_rcp(r);
+    H = T(2) * r2 * r * metric_rcp(den);
+    derive();
+  }
+  // alpha, sqrt(gamma) and H / (1 + H) from H
+  __device__ __forceinline__ void derive() {
+    const T gam = T(1) + H;
+    sg = metric_sqrt(gam);
+    alpha = metric_rcp(sg);
+    hb = H * metric_rcp(gam);
+  }
+  __device__ __forceinline__ T beta(int i) const { return hb * l[i]; }
+  __device__ __forceinline__ T along(const T* v) const {
+    return l[0] * v[0] + l[1] * v[1] + l[2] * v[2];
   }
   __device__ __forceinline__ void lower(const T* v, T* o) const {
-    o[0] = gd11 * v[0] + gd12 * v[1] + gd13 * v[2];
-    o[1] = gd12 * v[0] + gd22 * v[1] + gd23 * v[2];
-    o[2] = gd13 * v[0] + gd23 * v[1] + gd33 * v[2];
+    const T q = H * along(v);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) o[i] = v[i] + q * l[i];
   }
-  __device__ __forceinline__ void raise(const T* v, T* o) const {
-    o[0] = gu11 * v[0] + gu12 * v[1] + gu13 * v[2];
-    o[1] = gu12 * v[0] + gu22 * v[1] + gu23 * v[2];
-    o[2] = gu13 * v[0] + gu23 * v[1] + gu33 * v[2];
+  // of both vectors of a pair
+  __device__ __forceinline__ void lower(const Pair<T> v[3], Pair<T> o[3]) const {
+    const Pair<T> L[3] = {both(l[0]), both(l[1]), both(l[2])};
+    const Pair<T> q = pmul(both(H), pdot3(L, v));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) o[i] = pfma(q, L[i], v[i]);
   }
 };
 
@@ -131,10 +137,9 @@ __device__ __forceinline__ T gr_pos(const GrConst<T>& c, int a, int n) {
 // q = R^2 - a^2 cancels inside the horizon, giving FP32 errors of 1e-5 in r
 // and the shift against 1e-7 outside 1.5 r_H).  Elsewhere it is evaluated in
 // the field precision per point, as the reference does.  kMetricComps
-// components, component q of table point t at m[q * nt + t]: r, alpha,
-// sqrt(gamma), beta^1..3, gamma_11, _12, _13, _22, _23, _33, gamma^11, ^12,
-// ^13, ^22, ^23, ^33.
-constexpr int kMetricComps = 18;
+// components, component q of table point t at m[q * nt + t]: r, H, l_1..3,
+// alpha, sqrt(gamma).
+constexpr int kMetricComps = 7;
 constexpr double kNearRH = 3.0;
 
 template <typename T>
@@ -162,9 +167,7 @@ __global__ void gr_metric_kernel(const __grid_constant__ GrConst<T> c, T* __rest
   const long long t = near_index(c, i, j, k);
   if (t < 0) return;
   const long long nt = (long long)c.nb_n[0] * c.nb_n[1] * c.nb_n[2];
-  const double v[kMetricComps] = {q.r,    q.alpha, q.sg,   q.bu[0], q.bu[1], q.bu[2],
-                                  q.gd11, q.gd12,  q.gd13, q.gd22,  q.gd23,  q.gd33,
-                                  q.gu11, q.gu12,  q.gu13, q.gu22,  q.gu23,  q.gu33};
+  const double v[kMetricComps] = {q.r, q.H, q.l[0], q.l[1], q.l[2], q.alpha, q.sg};
 #pragma unroll
   for (int a = 0; a < kMetricComps; ++a) m[a * nt + t] = (T)v[a];
 }
@@ -179,22 +182,12 @@ __device__ __forceinline__ Cks<T> metric_at(const GrConst<T>& c, const T* __rest
   const long long nt = (long long)c.nb_n[0] * c.nb_n[1] * c.nb_n[2];
   Cks<T> q;
   q.r = __ldg(m + t);
-  q.alpha = __ldg(m + nt + t);
-  q.sg = __ldg(m + 2 * nt + t);
+  q.H = __ldg(m + nt + t);
 #pragma unroll
-  for (int a = 0; a < 3; ++a) q.bu[a] = __ldg(m + (3 + a) * nt + t);
-  q.gd11 = __ldg(m + 6 * nt + t);
-  q.gd12 = __ldg(m + 7 * nt + t);
-  q.gd13 = __ldg(m + 8 * nt + t);
-  q.gd22 = __ldg(m + 9 * nt + t);
-  q.gd23 = __ldg(m + 10 * nt + t);
-  q.gd33 = __ldg(m + 11 * nt + t);
-  q.gu11 = __ldg(m + 12 * nt + t);
-  q.gu12 = __ldg(m + 13 * nt + t);
-  q.gu13 = __ldg(m + 14 * nt + t);
-  q.gu22 = __ldg(m + 15 * nt + t);
-  q.gu23 = __ldg(m + 16 * nt + t);
-  q.gu33 = __ldg(m + 17 * nt + t);
+  for (int a = 0; a < 3; ++a) q.l[a] = __ldg(m + (2 + a) * nt + t);
+  q.alpha = __ldg(m + 5 * nt + t);
+  q.sg = __ldg(m + 6 * nt + t);
+  q.hb = q.H * q.alpha * q.alpha;
   return q;
 }
 
@@ -204,24 +197,29 @@ __device__ __forceinline__ Cks<T> metric_at(const GrConst<T>& c, const T* __rest
 // Every kernel that writes D and B at a point also writes E and H there
 // through this function, so they are computed the same way everywhere.
 template <typename T>
-__device__ __forceinline__ void gr_eh_store(const Cks<T>& m, const T* D, const T* B,
-                                            const F7<T>& eh, long long o) {
-  T Dd[3], Bd[3];
-  m.lower(D, Dd);
-  m.lower(B, Bd);
-  eh.p[0][o] = m.alpha * Dd[0] + m.sg * (m.bu[1] * B[2] - m.bu[2] * B[1]);
-  eh.p[1][o] = m.alpha * Dd[1] + m.sg * (m.bu[2] * B[0] - m.bu[0] * B[2]);
-  eh.p[2][o] = m.alpha * Dd[2] + m.sg * (m.bu[0] * B[1] - m.bu[1] * B[0]);
-  eh.p[3][o] = m.alpha * Bd[0] - m.sg * (m.bu[1] * D[2] - m.bu[2] * D[1]);
-  eh.p[4][o] = m.alpha * Bd[1] - m.sg * (m.bu[2] * D[0] - m.bu[0] * D[2]);
-  eh.p[5][o] = m.alpha * Bd[2] - m.sg * (m.bu[0] * D[1] - m.bu[1] * D[0]);
+__device__ __forceinline__ void gr_eh_store(const Cks<T>& m, const Pair<T> db[3],
+                                            const F7<T>& eh, const uint32_t o) {
+  Pair<T> low[3];
+  m.lower(db, low);
+  const T sh = m.sg * m.hb;  // sqrt(gamma) beta = sh l
+  const Pair<T> L[3] = {both(m.l[0]), both(m.l[1]), both(m.l[2])};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int b = (a + 1) % 3, c = (a + 2) % 3;
+    // (l x D, l x B)_a
+    const Pair<T> x = pfma(L[b], db[c], pmul(both(-m.l[c]), db[b]));
+    eh.p[a][o] = sfma(sh, second(x), smul(m.alpha, first(low[a])));
+    eh.p[3 + a][o] = sfma(-sh, first(x), smul(m.alpha, second(low[a])));
+  }
 }
 
 // E and H over the whole grid (guards included): once per call of the
 // solver, for both field buffers; afterwards every stage and KO pass writes
 // E and H of the points it updates (ehout), so the next kernel finds those
 // of its input.  eh[0..2] = E, eh[3..5] = H.
-template <typename T>
+// GUARDS: only the points outside the update box (the first stage writes E and
+// H of the others).
+template <typename T, bool GUARDS>
 __global__ void __launch_bounds__(256) gr_eh_kernel(const __grid_constant__ GrConst<T> c,
                                                     const F7<T> u, const F7<T> eh,
                                                     const T* __restrict__ mt) {
@@ -229,42 +227,52 @@ __global__ void __launch_bounds__(256) gr_eh_kernel(const __grid_constant__ GrCo
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
   if (i >= c.d[0] || j >= c.d[1] || k >= c.d[2]) return;
-  const long long o = i + (long long)c.d[0] * (j + (long long)c.d[1] * k);
+  if (GUARDS && i >= c.lo[0] && i < c.hi[0] && j >= c.lo[1] && j < c.hi[1] && k >= c.lo[2] &&
+      k < c.hi[2])
+    return;
+  const uint32_t o = (uint32_t)i + (uint32_t)c.d[0] * ((uint32_t)j + (uint32_t)c.d[1] * (uint32_t)k);
+  Pair<T> db[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) db[a] = pk(__ldg(u.p[a] + o), __ldg(u.p[3 + a] + o));
   const Cks<T> m =
       metric_at(c, mt, i, j, k, gr_pos(c, 0, i), gr_pos(c, 1, j), gr_pos(c, 2, k));
-  const T D[3] = {__ldg(u.p[0] + o), __ldg(u.p[1] + o), __ldg(u.p[2] + o)};
-  const T B[3] = {__ldg(u.p[3] + o), __ldg(u.p[4] + o), __ldg(u.p[5] + o)};
-  gr_eh_store(m, D, B, eh, o);
+  gr_eh_store(m, db, eh, o);
 }
 
 // clean_epar / check_eGTb with the 3-metric (kernel_clean_epar_gr,
 // kernel_check_eGTb_gr, field_solver_gr_EZ.cu:422-521)
+// Lowering is linear, so the lowered D after the cleaning is that of before
+// minus the same multiple of the lowered B.
 template <typename T>
-__device__ __forceinline__ void gr_clamps(const GrConst<T>& c, const Cks<T>& m, T* v) {
+__device__ __forceinline__ void gr_clamps(const GrConst<T>& c, const Cks<T>& m, Pair<T> db[3]) {
+  if (!c.clean_ep && !c.check_egb) return;
+  Pair<T> low[3];
+  m.lower(db, low);
+  T D[3] = {first(db[0]), first(db[1]), first(db[2])};
+  const T B[3] = {second(db[0]), second(db[1]), second(db[2])};
+  T Dd[3] = {first(low[0]), first(low[1]), first(low[2])};
+  const T Bd[3] = {second(low[0]), second(low[1]), second(low[2])};
+  const T B2 = B[0] * Bd[0] + B[1] * Bd[1] + B[2] * Bd[2];
   if (c.clean_ep) {
-    T Bd[3];
-    m.lower(v + 3, Bd);
-    T B2 = v[3] * Bd[0] + v[4] * Bd[1] + v[5] * Bd[2];
-    if (B2 < Tiny<T>::v) B2 = Tiny<T>::v;
-    const T q = fdiv(v[0] * Bd[0] + v[1] * Bd[1] + v[2] * Bd[2], B2);
-    v[0] -= q * v[3];
-    v[1] -= q * v[4];
-    v[2] -= q * v[5];
-  }
-  if (c.check_egb) {
-    T Dd[3], Bd[3];
-    m.lower(v, Dd);
-    m.lower(v + 3, Bd);
-    T D2 = v[0] * Dd[0] + v[1] * Dd[1] + v[2] * Dd[2];
-    if (D2 < Tiny<T>::v) D2 = Tiny<T>::v;
-    const T B2 = v[3] * Bd[0] + v[4] * Bd[1] + v[5] * Bd[2];
-    if (D2 > B2) {
-      const T s = sqrt(fdiv(B2, D2));
-      v[0] *= s;
-      v[1] *= s;
-      v[2] *= s;
+    const T q =
+        fdiv(D[0] * Bd[0] + D[1] * Bd[1] + D[2] * Bd[2], B2 < Tiny<T>::v ? Tiny<T>::v : B2);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      D[a] -= q * B[a];
+      Dd[a] -= q * Bd[a];
     }
   }
+  if (c.check_egb) {
+    T D2 = D[0] * Dd[0] + D[1] * Dd[1] + D[2] * Dd[2];
+    if (D2 < Tiny<T>::v) D2 = Tiny<T>::v;
+    if (D2 > B2) {
+      const T s = sqrt(fdiv(B2, D2));
+#pragma unroll
+      for (int a = 0; a < 3; ++a) D[a] *= s;
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) db[a] = pk(D[a], B[a]);
 }
 
 // Outer layer at the six faces (kernel_boundary_absorbing_thread,
@@ -321,99 +329,111 @@ __device__ __noinline__ V7<T> gr_absorb(const GrConst<T>& c, V7<T> v, V7<T> n, T
 // same.
 template <typename T, bool FIRST, typename Metric, typename Fetch, typename Own>
 __device__ __forceinline__ void gr_stage_point(const GrConst<T>& c, Metric&& metric, const T x,
-                                               const T y, const T z, const long long o,
+                                               const T y, const T z, const uint32_t o,
                                                Fetch&& f, Own&& own,
                                                const F7<T>& out, const F7<T>& du,
                                                const F7<T>& un, const F5<T>& aux, const T As,
                                                const T Bs, const int flags,
                                                const F7<T>& ehout) {
-  auto d1 = [&](auto qc, auto ac) {
-    constexpr int ax = decltype(ac)::value;
-    return d1_4w(f(qc, ac, -2), f(qc, ac, -1), f(qc, ac, 1), f(qc, ac, 2)) * c.inv_delta[ax];
-  };
   using I0 = std::integral_constant<int, 0>;
   using I1 = std::integral_constant<int, 1>;
   using I2 = std::integral_constant<int, 2>;
+  using QP = std::integral_constant<int, 12>;
+  using QS = std::integral_constant<int, 13>;
+  // diff1_4 of the pair (E_q, H_q) along an axis, times 12 / inv_delta; the
+  // factor is applied once per curl and divergence
+  auto d1 = [&](auto qc, auto ac) {
+    constexpr int q = decltype(qc)::value;
+    using H = std::integral_constant<int, q + 3>;
+    auto v = [&](int n) { return pk(f(qc, ac, n), f(H{}, ac, n)); };
+    Pair<T> t = psub(v(-2), v(2));
+    t = pfma(v(-1), both((T)-8), t);
+    return pfma(v(1), both((T)8), t);
+  };
+  const T w12[3] = {c.inv_delta[0] * T(1.0 / 12.0), c.inv_delta[1] * T(1.0 / 12.0),
+                    c.inv_delta[2] * T(1.0 / 12.0)};
   // the curls and divergences before their 1 / sqrt(gamma) factor: the
   // metric is evaluated after the stencil sums, so that its values do not
   // take registers while those are formed (the same operations either way)
-  T rotH[3] = {d1(std::integral_constant<int, 5>{}, I1{}) -
-                   d1(std::integral_constant<int, 4>{}, I2{}),
-               d1(std::integral_constant<int, 3>{}, I2{}) -
-                   d1(std::integral_constant<int, 5>{}, I0{}),
-               d1(std::integral_constant<int, 4>{}, I0{}) -
-                   d1(std::integral_constant<int, 3>{}, I1{})};
-  T rotE[3] = {d1(std::integral_constant<int, 2>{}, I1{}) -
-                   d1(std::integral_constant<int, 1>{}, I2{}),
-               d1(std::integral_constant<int, 0>{}, I2{}) -
-                   d1(std::integral_constant<int, 2>{}, I0{}),
-               d1(std::integral_constant<int, 1>{}, I0{}) -
-                   d1(std::integral_constant<int, 0>{}, I1{})};
+  Pair<T> rot[3];  // (rot E, rot H)
+  rot[0] = pfma(d1(I2{}, I1{}), both(w12[1]), pmul(d1(I1{}, I2{}), both(-w12[2])));
+  rot[1] = pfma(d1(I0{}, I2{}), both(w12[2]), pmul(d1(I2{}, I0{}), both(-w12[0])));
+  rot[2] = pfma(d1(I1{}, I0{}), both(w12[0]), pmul(d1(I0{}, I1{}), both(-w12[1])));
   // div4 (:44-86): each neighbour weighted by sqrt(gamma) there (the
   // per-solver table; the reference evaluates it at the shifted coordinates)
-  T divD = T(0), divB = T(0);
+  Pair<T> dvg = both((T)0);  // (div D, div B)
   static_for<3>([&](auto ac) {
     constexpr int ax = decltype(ac)::value;
-    using QS = std::integral_constant<int, 13>;
     using QD = std::integral_constant<int, 6 + ax>;
     using QB = std::integral_constant<int, 9 + ax>;
-    const T w[4] = {f(QS{}, ac, -2), f(QS{}, ac, -1), f(QS{}, ac, 1), f(QS{}, ac, 2)};
-    divD += d1_4w(f(QD{}, ac, -2) * w[0], f(QD{}, ac, -1) * w[1], f(QD{}, ac, 1) * w[2],
-                  f(QD{}, ac, 2) * w[3]) * c.inv_delta[ax];
-    divB += d1_4w(f(QB{}, ac, -2) * w[0], f(QB{}, ac, -1) * w[1], f(QB{}, ac, 1) * w[2],
-                  f(QB{}, ac, 2) * w[3]) * c.inv_delta[ax];
+    auto v = [&](int n) { return pk(f(QD{}, ac, n), f(QB{}, ac, n)); };
+    Pair<T> t = pmul(v(-2), both(f(QS{}, ac, -2)));
+    t = pfma(v(-1), both(T(-8) * f(QS{}, ac, -1)), t);
+    t = pfma(v(1), both(T(8) * f(QS{}, ac, 1)), t);
+    t = pfma(v(2), both(-f(QS{}, ac, 2)), t);
+    dvg = pfma(t, both(w12[ax]), dvg);
+  });
+  T Pd[3];
+  static_for<3>([&](auto ac) {
+    constexpr int ax = decltype(ac)::value;
+    const T t = sfma(f(QP{}, ac, -1), (T)-8, f(QP{}, ac, -2) - f(QP{}, ac, 2));
+    Pd[ax] = sfma(f(QP{}, ac, 1), (T)8, t) * w12[ax];
   });
   const Cks<T> m = metric();
-  const T igms = T(1) / m.sg;
+  const T igms = metric_rcp(m.sg);
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    rotH[a] *= igms;
-    rotE[a] *= igms;
-  }
-  divD *= igms;
-  divB *= igms;
-  T v[7];
+  for (int a = 0; a < 3; ++a) rot[a] = pmul(rot[a], both(igms));
+  dvg = pmul(dvg, both(igms));
+  const T divD = first(dvg), divB = second(dvg);
+  Pair<T> db[3];  // (D, B)
 #pragma unroll
-  for (int a = 0; a < 7; ++a) v[a] = own(6 + a);
-  T Bd[3], Dd[3];
-  m.lower(v + 3, Bd);
-  m.lower(v, Dd);
+  for (int a = 0; a < 3; ++a) db[a] = pk(own(6 + a), own(9 + a));
+  T P = own(12);
   T J[3] = {T(0), T(0), T(0)};
   if (c.calc_current) {
-    T B2 = v[3] * Bd[0] + v[4] * Bd[1] + v[5] * Bd[2];
+    Pair<T> low[3];
+    m.lower(db, low);
+    T B2 = second(pdot3(db, low));
     if (B2 < Tiny<T>::v) B2 = Tiny<T>::v;
-    const T Jp = (Bd[0] * rotH[0] + Bd[1] * rotH[1] + Bd[2] * rotH[2]) -
-                 (Dd[0] * rotE[0] + Dd[1] * rotE[1] + Dd[2] * rotE[2]);
-    const T e0 = own(0), e1 = own(1), e2 = own(2);
-    const T iB2 = fdiv(T(1), B2);
-    J[0] = (divD * (e1 * Bd[2] - e2 * Bd[1]) * igms + Jp * v[3]) * iB2;
-    J[1] = (divD * (e2 * Bd[0] - e0 * Bd[2]) * igms + Jp * v[4]) * iB2;
-    J[2] = (divD * (e0 * Bd[1] - e1 * Bd[0]) * igms + Jp * v[5]) * iB2;
-  }
-  using QP = std::integral_constant<int, 12>;
-  const T Pd[3] = {d1(QP{}, I0{}), d1(QP{}, I1{}), d1(QP{}, I2{})};
-  T Pu[3];
-  m.raise(Pd, Pu);
-  const T shape = T(0.5) * (T(1) - tanh((m.r - T(5)) / T(1)));  // r0 = 5, del = 1 (:276-278)
-  const T dt = c.dt;
-  T rhs[7];
+    const Pair<T> lr = pdot3(low, rot);  // (D . rot E, B . rot H)
+    const T Jp = second(lr) - first(lr);
+    const T e[3] = {own(0), own(1), own(2)};
+    const T b[3] = {second(low[0]), second(low[1]), second(low[2])};
+    const T iB2 = fdiv(T(1), B2), s = divD * igms;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    rhs[a] = dt * (rotH[a] - J[a]);
-    rhs[3 + a] = c.divB_clean ? dt * (-rotE[a] + (-m.alpha * Pu[a] + m.bu[a] * divB) * shape)
-                              : -dt * rotE[a];
+    for (int a = 0; a < 3; ++a) {
+      const int a1 = (a + 1) % 3, a2 = (a + 2) % 3;
+      J[a] = (s * (e[a1] * b[a2] - e[a2] * b[a1]) + Jp * second(db[a])) * iB2;
+    }
   }
-  rhs[6] = dt * (-m.alpha * divB + m.bu[0] * Pd[0] + m.bu[1] * Pd[1] + m.bu[2] * Pd[2]) -
-           m.alpha * v[6] / c.tau;
+  // beta . grad P = hb (l . grad P), and -alpha P^i + beta^i div B as a
+  // multiple of l^i and of P_i
+  const T lP = m.hb * m.along(Pd);
+  const T kl = m.alpha * lP + m.hb * divB;
+  // r0 = 5, del = 1 (:276-278): 0.5 (1 - tanh(r - 5)) = 1 / (1 + exp(2 (r - 5)))
+  const T shape = c.divB_clean ? T(1) / (T(1) + exp(T(2) * (m.r - T(5)))) : T(0);
+  const T dt = c.dt;
   if (flags & AX_WRITE_UN) {
 #pragma unroll
-    for (int a = 0; a < 6; ++a) un.p[a][o] = v[a];
+    for (int a = 0; a < 3; ++a) {
+      un.p[a][o] = first(db[a]);
+      un.p[3 + a][o] = second(db[a]);
+    }
   }
 #pragma unroll
-  for (int a = 0; a < 7; ++a) {
-    const T dd = FIRST ? rhs[a] : As * du.p[a][o] + rhs[a];
-    du.p[a][o] = dd;
-    v[a] += Bs * dd;
+  for (int a = 0; a < 3; ++a) {
+    const T clean = kl * m.l[a] - m.alpha * Pd[a];
+    Pair<T> d = pmul(pk(second(rot[a]) - J[a], sfma(clean, shape, -first(rot[a]))), both(dt));
+    if constexpr (!FIRST) d = pfma(pk(du.p[a][o], du.p[3 + a][o]), both(As), d);
+    du.p[a][o] = first(d);
+    du.p[3 + a][o] = second(d);
+    db[a] = pfma(d, both(Bs), db[a]);
+  }
+  {
+    T d = dt * (lP - m.alpha * divB) - m.alpha * P * c.inv_tau;
+    if constexpr (!FIRST) d = sfma(du.p[6][o], As, d);
+    du.p[6][o] = d;
+    P = sfma(d, Bs, P);
   }
   if (flags & AX_AUX) {
     aux.p[0][o] = J[0];
@@ -422,26 +442,35 @@ __device__ __forceinline__ void gr_stage_point(const GrConst<T>& c, Metric&& met
     aux.p[3][o] = divD;
     aux.p[4][o] = divB;
   }
-  gr_clamps(c, m, v);
-  V7<T> w;
-#pragma unroll
-  for (int a = 0; a < 7; ++a) w.v[a] = v[a];
+  gr_clamps(c, m, db);
   const bool in_layer = x > c.xh[0] || x < c.xl[0] || y > c.xh[1] || y < c.xl[1] ||
                         z > c.xh[2] || z < c.xl[2] || m.r < c.r1;
   if ((flags & AX_LAST) && c.absorbing && in_layer) {
-    V7<T> n;
+    V7<T> w, n;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      w.v[a] = first(db[a]);
+      w.v[3 + a] = second(db[a]);
+    }
+    w.v[6] = P;
 #pragma unroll
     for (int a = 0; a < 6; ++a) n.v[a] = un.p[a][o];
     n.v[6] = T(0);
     w = gr_absorb(c, w, n, x, y, z, m.r);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) db[a] = pk(w.v[a], w.v[3 + a]);
   }
 #pragma unroll
-  for (int a = 0; a < 7; ++a) out.p[a][o] = w.v[a];
-  if (ehout.p[0]) gr_eh_store(m, w.v, w.v + 3, ehout, o);
+  for (int a = 0; a < 3; ++a) {
+    out.p[a][o] = first(db[a]);
+    out.p[3 + a][o] = second(db[a]);
+  }
+  out.p[6][o] = P;
+  if (ehout.p[0]) gr_eh_store(m, db, ehout, o);
 }
 
 template <typename T, bool FIRST>
-__global__ void __launch_bounds__(256, COFFEE_GR_STAGE_MIN_BLOCKS) gr_stage_kernel(const __grid_constant__ GrConst<T> c,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? COFFEE_GR_STAGE_MIN_BLOCKS : 3) gr_stage_kernel(const __grid_constant__ GrConst<T> c,
                                                        const F7<T> u, const F7<T> eh,
                                                        const F7<T> out, const F7<T> du,
                                                        const F7<T> un, const F5<T> aux,
@@ -453,20 +482,22 @@ __global__ void __launch_bounds__(256, COFFEE_GR_STAGE_MIN_BLOCKS) gr_stage_kern
   const int j = c.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
   const int k = c.lo[2] + blockIdx.z * blockDim.z + threadIdx.z;
   if (i >= c.hi[0] || j >= c.hi[1] || k >= c.hi[2]) return;
-  const long long sx = 1, sy = c.d[0], sz = (long long)c.d[0] * c.d[1];
-  const long long o = i + sy * j + sz * k;
-  const long long st[3] = {sx, sy, sz};
+  const uint32_t sy = (uint32_t)c.d[0], sz = sy * (uint32_t)c.d[1];
+  const uint32_t o = (uint32_t)i + sy * (uint32_t)j + sz * (uint32_t)k;
   const T x = gr_pos(c, 0, i), y = gr_pos(c, 1, j), z = gr_pos(c, 2, k);
   auto metric = [&]() { return metric_at(c, mt, i, j, k, x, y, z); };
   // the array pointers straight from the kernel parameters (a local array
-  // of them would take registers this kernel does not have)
+  // of them would take registers this kernel does not have); 32-bit element
+  // offsets (gr_check), so an address is one wide multiply-add, and the x
+  // neighbours are immediate offsets from the point's own address
   auto fetch = [&](auto qc, auto ac, int n) {
-    constexpr int q = decltype(qc)::value;
+    constexpr int q = decltype(qc)::value, ax = decltype(ac)::value;
     const T* p;
     if constexpr (q < 6) p = eh.p[q];
     else if constexpr (q < 13) p = u.p[q - 6];
     else p = sgt;
-    return __ldg(p + o + n * st[decltype(ac)::value]);
+    if constexpr (ax == 0) return __ldg(p + o + n);
+    else return __ldg(p + (uint32_t)(o + (uint32_t)n * (ax == 1 ? sy : sz)));
   };
   auto own = [&](int q) { return __ldg((q < 6 ? eh.p[q] : u.p[q - 6]) + o); };
   gr_stage_point<T, FIRST>(c, metric, x, y, z, o, fetch, own, out, du, un, aux, As, Bs, flags,
@@ -594,7 +625,7 @@ __global__ void __launch_bounds__(kGrTX * kGrTY, COFFEE_GR_TILE_MINB) gr_stage_t
       auto ownv = [&](int q) { return cs[q * kGrSP + own]; };
       const float x = gr_pos(c, 0, i), y = gr_pos(c, 1, j), z = gr_pos(c, 2, k);
       auto metric = [&]() { return metric_at(c, mt, i, j, k, x, y, z); };
-      gr_stage_point<float, FIRST>(c, metric, x, y, z, (long long)k * sz + ocol, fetch, ownv, out,
+      gr_stage_point<float, FIRST>(c, metric, x, y, z, (uint32_t)(k * sz + ocol), fetch, ownv, out,
                                    du, un, aux, As, Bs, flags, ehout);
 #pragma unroll
       for (int s2 = 0; s2 < 4; ++s2)
@@ -616,28 +647,57 @@ __global__ void __launch_bounds__(256) gr_ko_kernel(const __grid_constant__ GrCo
   const int j = c.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
   const int k = c.lo[2] + blockIdx.z * blockDim.z + threadIdx.z;
   if (i >= c.hi[0] || j >= c.hi[1] || k >= c.hi[2]) return;
-  const long long sy = c.d[0], sz = (long long)c.d[0] * c.d[1];
-  const long long o = i + sy * j + sz * k;
-  constexpr T K6[7] = {T(1), T(-6), T(15), T(-20), T(15), T(-6), T(1)};
-  T v[7];
+  const uint32_t sy = (uint32_t)c.d[0], sz = sy * (uint32_t)c.d[1];
+  const uint32_t o = (uint32_t)i + sy * (uint32_t)j + sz * (uint32_t)k;
+  // 6th difference of all three axes: the weights of a neighbour at distance
+  // 1, 2, 3 are 15, -6, 1 and the point's own -60
+  auto at = [&](const T* p, int ax, int n) {
+    if (ax == 0) return __ldg(p + o + n);
+    return __ldg(p + (uint32_t)(o + (uint32_t)n * (ax == 1 ? sy : sz)));
+  };
+  Pair<T> db[3];
 #pragma unroll
-  for (int a = 0; a < 7; ++a) {
-    const T* f = u.p[a];
-    T tx = T(0), ty = T(0), tz = T(0);
+  for (int a = 0; a < 3; ++a) {
+    const T *pd = u.p[a], *pb = u.p[3 + a];
+    Pair<T> s1 = both((T)0), s2 = s1, s3 = s1;
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
-      tx += K6[q] * __ldg(f + o + (q - 3));
-      ty += K6[q] * __ldg(f + o + (q - 3) * sy);
-      tz += K6[q] * __ldg(f + o + (q - 3) * sz);
+    for (int ax = 0; ax < 3; ++ax) {
+      auto sum = [&](int n) {
+        return padd(pk(at(pd, ax, -n), at(pb, ax, -n)), pk(at(pd, ax, n), at(pb, ax, n)));
+      };
+      s1 = padd(s1, sum(1));
+      s2 = padd(s2, sum(2));
+      s3 = padd(s3, sum(3));
     }
-    v[a] = __ldg(f + o) + c.ko_c * (tx + ty + tz);
+    const Pair<T> own = pk(__ldg(pd + o), __ldg(pb + o));
+    Pair<T> t = pfma(s2, both((T)-6), s3);
+    t = pfma(s1, both((T)15), t);
+    t = pfma(own, both((T)-60), t);
+    db[a] = pfma(t, both(c.ko_c), own);
+  }
+  T P;
+  {
+    const T* p = u.p[6];
+    T s1 = 0, s2 = 0, s3 = 0;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      s1 += at(p, ax, -1) + at(p, ax, 1);
+      s2 += at(p, ax, -2) + at(p, ax, 2);
+      s3 += at(p, ax, -3) + at(p, ax, 3);
+    }
+    const T own = __ldg(p + o);
+    P = sfma(sfma(own, (T)-60, sfma(s1, (T)15, sfma(s2, (T)-6, s3))), c.ko_c, own);
   }
   const Cks<T> m =
       metric_at(c, mt, i, j, k, gr_pos(c, 0, i), gr_pos(c, 1, j), gr_pos(c, 2, k));
-  gr_clamps(c, m, v);
+  gr_clamps(c, m, db);
 #pragma unroll
-  for (int a = 0; a < 7; ++a) out.p[a][o] = v[a];
-  if (ehout.p[0]) gr_eh_store(m, v, v + 3, ehout, o);
+  for (int a = 0; a < 3; ++a) {
+    out.p[a][o] = first(db[a]);
+    out.p[3 + a][o] = second(db[a]);
+  }
+  out.p[6][o] = P;
+  if (ehout.p[0]) gr_eh_store(m, db, ehout, o);
 }
 
 }  // namespace coffee

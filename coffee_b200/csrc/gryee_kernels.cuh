@@ -85,7 +85,7 @@ __device__ __forceinline__ void gyee_e(const GYeeArgs<T>& g, int i, int j, int k
   T dl[3];
   m.lower(iD, dl);
   // kernel_compute_E_gr_thread (field_solver_gr.cu:99-149)
-  g.Ed[A][o] = m.alpha * dl[A] + m.sg * (m.bu[b] * iB[c] - m.bu[c] * iB[b]);
+  g.Ed[A][o] = m.alpha * dl[A] + m.sg * (m.beta(b) * iB[c] - m.beta(c) * iB[b]);
 }
 
 template <int A, typename T>
@@ -104,7 +104,7 @@ __device__ __forceinline__ void gyee_h(const GYeeArgs<T>& g, int i, int j, int k
   T bl[3];
   m.lower(iB, bl);
   // kernel_compute_H_gr_thread (field_solver_gr.cu:152-225)
-  g.Hd[A][o] = m.alpha * bl[A] - m.sg * (m.bu[b] * iD[c] - m.bu[c] * iD[b]);
+  g.Hd[A][o] = m.alpha * bl[A] - m.sg * (m.beta(b) * iD[c] - m.beta(c) * iD[b]);
   g.Bd[A][o] = bl[A];
 }
 
