@@ -134,6 +134,12 @@ SIGNATURES = {
     "coffee_conv3d_backward_weight": (_i, [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp]),
     "coffee_conv3d_backward_weight_tc": (_i, [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp]),
     "coffee_bias_grad": (_i, [_vp, ctypes.c_longlong, _i, _vp, _vp]),
+    "coffee_leaky_bias_backward": (_i, [_vp, _vp, ctypes.c_longlong, _i, ctypes.c_float, _vp, _vp, _vp]),
+    "coffee_up2_leaky_bias_backward": (_i, [_vp, _i, _i, _i, _i, _i, _i, _i, _vp, ctypes.c_float, _vp, _vp,
+                                            _vp]),
+    "coffee_skip_pool2_leaky_bias_backward": (_i, [_vp, _i, _i, _vp, _i, _i, _i, _i, _i, _vp, ctypes.c_float,
+                                                   _vp, _vp, _vp]),
+    "coffee_up2_concat": (_i, [_vp, _i, _i, _i, _i, _i, _vp, _i, _vp, _vp]),
     "coffee_leaky_backward": (_i, [_vp, _vp, ctypes.c_longlong, ctypes.c_float, _vp, _vp, _vp]),
     "coffee_pool2_forward": (_i, [_vp, _i, _i, _i, _i, _i, _vp, _vp]),
     "coffee_pool2_backward_add": (_i, [_vp, _i, _i, _i, _i, _i, _vp, _vp]),

@@ -16,6 +16,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <initializer_list>
 
 #include "coffee_internal.h"
 #include "coffee_surrogate.h"
@@ -276,7 +277,9 @@ void launch_wgrad(const bf16* dy, const bf16* x, Grid4 g, int K, float* part, cu
 // blocks in order.
 constexpr int kBiasBlocks = 296;
 constexpr int kBiasMaxK = 64;
-__device__ float g_bias_part[kBiasBlocks * kBiasMaxK];
+// blocks of the fused passes (4 per SM: enough loads in flight)
+constexpr int kFusedBlocks = 592;
+__device__ float g_bias_part[kFusedBlocks * kBiasMaxK];
 
 __global__ void bias_grad_part_kernel(const float* __restrict__ dz, long long npts, int K,
                                       long long per) {
@@ -294,12 +297,162 @@ __global__ void bias_grad_part_kernel(const float* __restrict__ dz, long long np
   }
 }
 
-__global__ void bias_grad_sum_kernel(int K, int blocks, float* __restrict__ db) {
-  const int k = threadIdx.x;
-  if (k >= K) return;
+// Sums the blocks' partial sums: 256 threads, R = 256 / K rows of blocks per
+// channel in order, then the rows in order.  (One thread per channel took 13 us
+// for its chain of 296 loads.)
+__global__ void __launch_bounds__(256) bias_grad_sum_kernel(int K, int blocks,
+                                                            float* __restrict__ db) {
+  __shared__ float red[256];
+  const int R = 256 / K, k = threadIdx.x % K, r = threadIdx.x / K;
   float s = 0.f;
-  for (int b = 0; b < blocks; ++b) s += g_bias_part[b * kBiasMaxK + k];
+  if (r < R)
+    for (int b = r; b < blocks; b += R) s += g_bias_part[b * kBiasMaxK + k];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  if (r != 0) return;
+  for (int q = 1; q < R; ++q) s += red[q * K + k];
   db[k] = s;
+}
+
+// ---- fused elementwise passes of the backward pass ------------------------
+// These passes are bound by HBM, so each reads its inputs once, 16 or 32 bytes a
+// thread, writes only the BF16 gradient that the next convolutions read, and
+// keeps the bias gradient's partial sums on the way.  A thread handles 8
+// channels of one point; a block's threads cover 2048 / C points at a time with
+// thread t always on channels 8 (t % (C / 8)) .., so that its 8 bias sums stay
+// in registers.  C divides 2048 and is a multiple of 8.
+struct alignas(16) Vec4f { float v[4]; };
+struct alignas(16) Vec8b { bf16 v[8]; };
+
+__device__ __forceinline__ void load8(const float* __restrict__ p, float o[8]) {
+  const Vec4f a = *reinterpret_cast<const Vec4f*>(p), b = *reinterpret_cast<const Vec4f*>(p + 4);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    o[q] = a.v[q];
+    o[4 + q] = b.v[q];
+  }
+}
+
+// The derivative of the leaky ReLU at 8 channels of the activation a (whose sign
+// is that of its argument), the BF16 gradient and the bias sums.
+__device__ __forceinline__ void leaky8(const float d[8], const bf16* __restrict__ a,
+                                       float slope, bf16* __restrict__ dzb, float bias[8]) {
+  const Vec8b av = *reinterpret_cast<const Vec8b*>(a);
+  Vec8b out;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float v = d[q] * (__bfloat162float(av.v[q]) > 0.f ? 1.f : slope);
+    out.v[q] = __float2bfloat16_rn(v);
+    bias[q] += v;
+  }
+  *reinterpret_cast<Vec8b*>(dzb) = out;
+}
+
+// block sums of the threads' bias sums, in a fixed order
+__device__ __forceinline__ void bias_block_sum(const float bias[8], int C) {
+  __shared__ float red[256 * 9];
+  const int t = threadIdx.x, G = C / 8;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) red[t * 9 + q] = bias[q];
+  __syncthreads();
+  if (t < C) {
+    float s = 0.f;
+    for (int r = t / 8; r < 256; r += G) s += red[r * 9 + t % 8];
+    g_bias_part[blockIdx.x * kBiasMaxK + t] = s;
+  }
+}
+
+// dz = da leaky'(a): BF16 dz and the bias gradient's partial sums
+__global__ void __launch_bounds__(256) leaky_bias_kernel(const float* __restrict__ da,
+                                                         const bf16* __restrict__ a, long long n8,
+                                                         int C, float slope,
+                                                         bf16* __restrict__ dzb) {
+  float bias[8] = {};
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n8; i += gridDim.x * 256LL) {
+    float d[8];
+    load8(da + i * 8, d);
+    leaky8(d, a + i * 8, slope, dzb + i * 8, bias);
+  }
+  bias_block_sum(bias, C);
+}
+
+// The gradient of a 2x nearest upsampling (channels off .. off + C of dy's cy) at
+// the coarse point, through the leaky ReLU before it.
+__global__ void __launch_bounds__(256) up2_leaky_bias_kernel(const float* __restrict__ dy, Grid4 g,
+                                                             int C, int cy, int off,
+                                                             const bf16* __restrict__ a,
+                                                             float slope, bf16* __restrict__ dzb) {
+  const Grid4 f{g.n, g.d * 2, g.h * 2, g.w * 2};
+  const unsigned G = C / 8;
+  const long long n8 = g.npts() * G;
+  float bias[8] = {};
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n8; i += gridDim.x * 256LL) {
+    const int c = (int)(i % G) * 8;
+    int nn, z, yy, xx;
+    decompose(g, i / G, nn, z, yy, xx);
+    float s[8] = {};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const long long p = (((long long)nn * f.d + 2 * z + (q >> 2)) * f.h + 2 * yy + ((q >> 1) & 1)) *
+                              f.w + 2 * xx + (q & 1);
+      float v[8];
+      load8(dy + p * cy + off + c, v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s[e] += v[e];
+    }
+    leaky8(s, a + i * 8, slope, dzb + i * 8, bias);
+  }
+  bias_block_sum(bias, C);
+}
+
+// The gradient at the skip connection's source: channels off .. off + C of the
+// concatenation's gradient plus that of the 2x average pooling, through the
+// leaky ReLU.
+__global__ void __launch_bounds__(256) skip_pool_leaky_bias_kernel(
+    const float* __restrict__ dcat, int ccat, int off, const float* __restrict__ dp, Grid4 g,
+    int C, const bf16* __restrict__ a, float slope, bf16* __restrict__ dzb) {
+  const Grid4 h{g.n, g.d / 2, g.h / 2, g.w / 2};
+  const unsigned G = C / 8;
+  const long long n8 = g.npts() * G;
+  float bias[8] = {};
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n8; i += gridDim.x * 256LL) {
+    const int c = (int)(i % G) * 8;
+    const long long p = i / G;
+    int nn, z, yy, xx;
+    decompose(g, p, nn, z, yy, xx);
+    const long long pc = (((long long)nn * h.d + z / 2) * h.h + yy / 2) * h.w + xx / 2;
+    float d[8], e[8];
+    load8(dcat + p * ccat + off + c, d);
+    load8(dp + pc * C + c, e);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) d[q] += e[q] * 0.125f;
+    leaky8(d, a + i * 8, slope, dzb + i * 8, bias);
+  }
+  bias_block_sum(bias, C);
+}
+
+// The concatenation [up2(x), s]: C channels of the coarse x at twice the
+// resolution, then cs channels of s, 8 channels (16 bytes) a thread.
+__global__ void __launch_bounds__(256) up2_concat_kernel(const bf16* __restrict__ x, Grid4 g, int C,
+                                                         const bf16* __restrict__ s, int cs,
+                                                         bf16* __restrict__ y) {
+  const Grid4 f{g.n, g.d * 2, g.h * 2, g.w * 2};
+  const unsigned gc = C / 8, G = (C + cs) / 8;
+  const long long n8 = f.npts() * G;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n8; i += gridDim.x * 256LL) {
+    const unsigned q = (unsigned)(i % G);
+    const long long p = i / G;
+    Vec8b v;
+    if (q < gc) {
+      int nn, z, yy, xx;
+      decompose(f, p, nn, z, yy, xx);
+      const long long pc = (((long long)nn * g.d + z / 2) * g.h + yy / 2) * g.w + xx / 2;
+      v = *reinterpret_cast<const Vec8b*>(x + pc * C + 8 * q);
+    } else {
+      v = *reinterpret_cast<const Vec8b*>(s + p * cs + 8 * (q - gc));
+    }
+    *reinterpret_cast<Vec8b*>(y + i * 8) = v;
+  }
 }
 
 __global__ void leaky_bwd_kernel(const float* __restrict__ da, const float* __restrict__ z,
@@ -397,6 +550,62 @@ __global__ void channels_add_kernel(const float* __restrict__ dsrc, long long np
     dx[i] += dsrc[(i / c) * csrc + soff + i % c];
 }
 
+// FP32 -> BF16 with the bias gradient's partial sums (the linear last layer)
+__global__ void __launch_bounds__(256) to_bf16_bias_kernel(const float* __restrict__ dz,
+                                                           long long n8, int C,
+                                                           bf16* __restrict__ dzb) {
+  float bias[8] = {};
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n8; i += gridDim.x * 256LL) {
+    float d[8];
+    load8(dz + i * 8, d);
+    Vec8b o;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      o.v[q] = __float2bfloat16_rn(d[q]);
+      bias[q] += d[q];
+    }
+    *reinterpret_cast<Vec8b*>(dzb + i * 8) = o;
+  }
+  bias_block_sum(bias, C);
+}
+
+// The masked error 4 channels (16 bytes) a thread, c a multiple of 4; 1024
+// threads a block keep the 256 partial sums' interface with enough loads in
+// flight (0.34 ms with 256 threads and 4-byte loads at 8 x 64^3 x 16).
+__global__ void __launch_bounds__(1024) mse4_kernel(const float* __restrict__ out,
+                                                    const float* __restrict__ tgt,
+                                                    const float* __restrict__ mask,
+                                                    long long npts, int c, double inv,
+                                                    float* __restrict__ dout,
+                                                    double* __restrict__ partial) {
+  const unsigned G = c / 4;
+  const long long n4 = npts * G;
+  const float two = (float)(2.0 * inv);
+  double s = 0.0;
+  for (long long i = blockIdx.x * 1024LL + threadIdx.x; i < n4; i += gridDim.x * 1024LL) {
+    const float m = mask ? mask[i / G] : 1.f;
+    const Vec4f o = *reinterpret_cast<const Vec4f*>(out + 4 * i);
+    const Vec4f t = *reinterpret_cast<const Vec4f*>(tgt + 4 * i);
+    Vec4f d;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float e = o.v[q] - t.v[q];
+      d.v[q] = two * m * e;
+      s += (double)m * (double)e * (double)e;
+    }
+    *reinterpret_cast<Vec4f*>(dout + 4 * i) = d;
+  }
+  __shared__ double red[32];
+  for (int w = 16; w > 0; w >>= 1) s += __shfl_down_sync(0xffffffffu, s, w);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = red[threadIdx.x];
+    for (int w = 16; w > 0; w >>= 1) s += __shfl_down_sync(0xffffffffu, s, w);
+    if (threadIdx.x == 0) partial[blockIdx.x] = s * inv;
+  }
+}
+
 __global__ void mse_kernel(const float* __restrict__ out, const float* __restrict__ tgt,
                            const float* __restrict__ mask, long long npts, int c, double inv,
                            float* __restrict__ dout, double* __restrict__ partial) {
@@ -421,11 +630,12 @@ __global__ void mse_kernel(const float* __restrict__ out, const float* __restric
 
 __global__ void sum_partials_kernel(const double* __restrict__ partial, int n,
                                     double* __restrict__ out) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += partial[i];  // fixed order
-    *out = s;
-  }
+  // one warp: each lane its stretch, then the lanes, both in a fixed order
+  const int per = (n + 31) / 32, i0 = (int)threadIdx.x * per;
+  double s = 0.0;
+  for (int i = i0; i < min(n, i0 + per); ++i) s += partial[i];
+  for (int w = 16; w > 0; w >>= 1) s += __shfl_down_sync(0xffffffffu, s, w);
+  if (threadIdx.x == 0) *out = s;
 }
 
 __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g,
@@ -1200,9 +1410,17 @@ __global__ void wgrad_tc_reduce_kernel(const float* __restrict__ part, int K, in
   if (i >= n) return;
   const int k = (int)(i / (27 * C)), r = (int)(i % (27 * C)), tap = r / C, c = r % C;
   const int tpm = 128 / CBW, tg = tap / tpm, m = (tap % tpm) * CBW + c;
-  float s = 0.f;
-  for (int q = 0; q < nchunks; ++q) s += part[(((long long)q * ngroups + tg) * 128 + m) * K + k];
-  dw[i] = s;
+  // four sums of every fourth chunk keep four loads in flight
+  const float* p = part + ((long long)tg * 128 + m) * K + k;
+  const long long step = (long long)ngroups * 128 * K;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  int q = 0;
+  for (; q + 4 <= nchunks; q += 4) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e] += p[(q + e) * step];
+  }
+  for (; q < nchunks; ++q) s[0] += p[q * step];
+  dw[i] = (s[0] + s[1]) + (s[2] + s[3]);
 }
 
 // Most SMs the chunk count is sized for (the workspace bound).
@@ -1468,7 +1686,93 @@ extern "C" int coffee_bias_grad(const float* dz, long long npts, int k, float* d
   const int threads = k * std::max(1, 256 / k);
   bias_grad_part_kernel<<<(unsigned)blocks, (unsigned)threads, 0, st>>>(dz, npts, k, per);
   COFFEE_CUDA_TRY(cudaGetLastError());
-  bias_grad_sum_kernel<<<1, kBiasMaxK, 0, st>>>(k, blocks, db);
+  bias_grad_sum_kernel<<<1, 256, 0, st>>>(k, blocks, db);
+  COFFEE_CUDA_TRY(cudaGetLastError());
+  return COFFEE_OK;
+}
+
+namespace {
+// channels the fused passes take (a thread always meets the same 8), and
+// 16-byte alignment of every pointer
+bool fused_ok(int c, std::initializer_list<const void*> ps) {
+  if (c < 8 || c > kBiasMaxK || c % 8 != 0 || 2048 % c != 0) return false;
+  for (const void* p : ps)
+    if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return false;
+  return true;
+}
+unsigned fused_blocks(long long n8) {
+  return (unsigned)std::max<long long>(1, std::min<long long>(kFusedBlocks, (n8 + 255) / 256));
+}
+int bias_sum(int k, unsigned blocks, float* db, cudaStream_t st) {
+  COFFEE_CUDA_TRY(cudaGetLastError());
+  bias_grad_sum_kernel<<<1, 256, 0, st>>>(k, (int)blocks, db);
+  COFFEE_CUDA_TRY(cudaGetLastError());
+  return COFFEE_OK;
+}
+}  // namespace
+
+extern "C" int coffee_leaky_bias_backward(const float* da, const void* a, long long npts, int c,
+                                          float slope, void* dz_bf16, float* db, void* stream) {
+  clear_error();
+  if (!da || !dz_bf16 || !db || npts <= 0 || !fused_ok(c, {da, a, dz_bf16}))
+    return fail(COFFEE_E_INVALID, "coffee_leaky_bias_backward: bad argument");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const long long n8 = npts * (c / 8);
+  const unsigned nb = fused_blocks(n8);
+  if (a)
+    leaky_bias_kernel<<<nb, 256, 0, st>>>(da, static_cast<const bf16*>(a), n8, c, slope,
+                                          static_cast<bf16*>(dz_bf16));
+  else
+    to_bf16_bias_kernel<<<nb, 256, 0, st>>>(da, n8, c, static_cast<bf16*>(dz_bf16));
+  return bias_sum(c, nb, db, st);
+}
+
+extern "C" int coffee_up2_leaky_bias_backward(const float* dy, int n, int d, int h, int w, int c,
+                                              int cy, int off, const void* a, float slope,
+                                              void* dz_bf16, float* db, void* stream) {
+  clear_error();
+  if (!dy || !a || !dz_bf16 || !db || off < 0 || off + c > cy || cy % 4 != 0 || off % 4 != 0 ||
+      !fused_ok(c, {dy, a, dz_bf16}))
+    return fail(COFFEE_E_INVALID, "coffee_up2_leaky_bias_backward: bad argument");
+  const Grid4 g{n, d, h, w};
+  if (g.npts() <= 0) return fail(COFFEE_E_INVALID, "coffee_up2_leaky_bias_backward: bad argument");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const unsigned nb = fused_blocks(g.npts() * (c / 8));
+  up2_leaky_bias_kernel<<<nb, 256, 0, st>>>(dy, g, c, cy, off, static_cast<const bf16*>(a), slope,
+                                            static_cast<bf16*>(dz_bf16));
+  return bias_sum(c, nb, db, st);
+}
+
+extern "C" int coffee_skip_pool2_leaky_bias_backward(const float* dcat, int ccat, int off,
+                                                     const float* dp, int n, int d, int h, int w,
+                                                     int c, const void* a, float slope,
+                                                     void* dz_bf16, float* db, void* stream) {
+  clear_error();
+  if (!dcat || !dp || !a || !dz_bf16 || !db || off < 0 || off + c > ccat || ccat % 4 != 0 ||
+      off % 4 != 0 || d % 2 || h % 2 || w % 2 || !fused_ok(c, {dcat, dp, a, dz_bf16}))
+    return fail(COFFEE_E_INVALID, "coffee_skip_pool2_leaky_bias_backward: bad argument");
+  const Grid4 g{n, d, h, w};
+  if (g.npts() <= 0)
+    return fail(COFFEE_E_INVALID, "coffee_skip_pool2_leaky_bias_backward: bad argument");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const unsigned nb = fused_blocks(g.npts() * (c / 8));
+  skip_pool_leaky_bias_kernel<<<nb, 256, 0, st>>>(dcat, ccat, off, dp, g, c,
+                                                  static_cast<const bf16*>(a), slope,
+                                                  static_cast<bf16*>(dz_bf16));
+  return bias_sum(c, nb, db, st);
+}
+
+extern "C" int coffee_up2_concat(const void* x, int n, int d, int h, int w, int c, const void* s,
+                                 int cs, void* y, void* stream) {
+  clear_error();
+  if (!x || !s || !y || c < 8 || cs < 8 || c % 8 || cs % 8 ||
+      (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(s) |
+       reinterpret_cast<uintptr_t>(y)) % 16 != 0)
+    return fail(COFFEE_E_INVALID, "coffee_up2_concat: bad argument");
+  const Grid4 g{n, d, h, w};
+  if (g.npts() <= 0) return fail(COFFEE_E_INVALID, "coffee_up2_concat: bad argument");
+  up2_concat_kernel<<<blocks_for(g.npts() * (c + cs)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const bf16*>(x), g, c, static_cast<const bf16*>(s), cs, static_cast<bf16*>(y));
   COFFEE_CUDA_TRY(cudaGetLastError());
   return COFFEE_OK;
 }
@@ -1555,7 +1859,11 @@ extern "C" int coffee_mse(const float* out, const float* target, const float* ma
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // the partial sums live in loss[1 .. 256] (the caller provides 257 doubles)
   const unsigned nb = 256;
-  mse_kernel<<<nb, 256, 0, st>>>(out, target, mask, npts, c, 1.0 / count, dout, loss + 1);
+  if (c % 4 == 0 && (reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(target) |
+                     reinterpret_cast<uintptr_t>(dout)) % 16 == 0)
+    mse4_kernel<<<nb, 1024, 0, st>>>(out, target, mask, npts, c, 1.0 / count, dout, loss + 1);
+  else
+    mse_kernel<<<nb, 256, 0, st>>>(out, target, mask, npts, c, 1.0 / count, dout, loss + 1);
   sum_partials_kernel<<<1, 32, 0, st>>>(loss + 1, (int)nb, loss);
   COFFEE_CUDA_TRY(cudaGetLastError());
   return COFFEE_OK;

@@ -191,7 +191,9 @@ class UNet:
         torch = _torch()
         L = self.layers[i]
         shape = x.shape[:4] + (L.cout,)
-        z = torch.empty(shape, dtype=torch.float32, device=self.dev)
+        # an activated layer needs only its BF16 activation later (the leaky
+        # ReLU's derivative is a matter of its sign)
+        z = None if act else torch.empty(shape, dtype=torch.float32, device=self.dev)
         a = torch.empty(shape, dtype=torch.bfloat16, device=self.dev) if act else None
         fwd = conv_forward_tc if use_tc(L.cin, L.cout) else conv_forward
         fwd(x, L.wb, L.b, L.cout, act, z, a)
@@ -204,31 +206,26 @@ class UNet:
         lib = _lib.load()
         n, d, h, w, _ = x.shape
         s = {"x": x}
-        s["z1"], s["a1"] = self._conv(0, x, True)
-        s["z2"], s["a2"] = self._conv(1, s["a1"], True)
+        s["a1"] = self._conv(0, x, True)[1]
+        s["a2"] = self._conv(1, s["a1"], True)[1]
         p2 = torch.empty((n, d // 2, h // 2, w // 2, C1), dtype=torch.bfloat16, device=self.dev)
         check(lib.coffee_pool2_forward(_ptr(s["a2"]), n, d, h, w, C1, _ptr(p2), _stream()))
         s["p2"] = p2
-        s["z3"], s["a3"] = self._conv(2, p2, True)
-        s["z4"], s["a4"] = self._conv(3, s["a3"], True)
+        s["a3"] = self._conv(2, p2, True)[1]
+        s["a4"] = self._conv(3, s["a3"], True)[1]
         cat = torch.empty((n, d, h, w, C2 + C1), dtype=torch.bfloat16, device=self.dev)
-        check(lib.coffee_up2_forward(_ptr(s["a4"]), n, d // 2, h // 2, w // 2, C2, _ptr(cat),
-                                     C2 + C1, 0, _stream()))
-        check(lib.coffee_channels_copy(_ptr(s["a2"]), n * d * h * w, C1, _ptr(cat), C2 + C1, C2,
-                                       _stream()))
+        check(lib.coffee_up2_concat(_ptr(s["a4"]), n, d // 2, h // 2, w // 2, C2, _ptr(s["a2"]),
+                                    C1, _ptr(cat), _stream()))
         s["cat"] = cat
-        s["z5"], s["a5"] = self._conv(4, cat, True)
+        s["a5"] = self._conv(4, cat, True)[1]
         out, _ = self._conv(5, s["a5"], False)
         self._saved = s
         return out
 
-    def _layer_grads(self, i, dz, dzb, x_in):
-        """Bias and weight gradients of layer i from dz (FP32 and BF16) and its input."""
-        lib = _lib.load()
+    def _weight_grad(self, i, dzb, x_in):
+        """Weight gradient of layer i from its BF16 dz and its input."""
         torch = _torch()
         L = self.layers[i]
-        npts = dz.numel() // L.cout
-        check(lib.coffee_bias_grad(_ptr(dz), npts, L.cout, _ptr(L.gb), _stream()))
         need = workspace_bytes(L.cout, L.cin)
         if self._ws is None or self._ws.numel() < need:
             self._ws = torch.empty(need, dtype=torch.uint8, device=self.dev)
@@ -241,48 +238,44 @@ class UNet:
         lib = _lib.load()
         s = self._saved
         n, d, h, w, _ = dout.shape
-        full = n * d * h * w
 
-        def bf(t):
-            return to_bf16(t, torch.empty(t.shape, dtype=torch.bfloat16, device=self.dev))
+        def dz_like(a):
+            return torch.empty(a.shape, dtype=torch.bfloat16, device=self.dev)
 
-        def leaky_bwd(da, z):
-            dz = torch.empty_like(da)
-            dzb = torch.empty(da.shape, dtype=torch.bfloat16, device=self.dev)
-            check(lib.coffee_leaky_backward(_ptr(da), _ptr(z), da.numel(), SLOPE, _ptr(dz),
-                                            _ptr(dzb), _stream()))
-            return dz, dzb
+        def leaky(i, da, a):  # BF16 dz of layer i and its bias gradient
+            dzb = dz_like(da)
+            check(lib.coffee_leaky_bias_backward(_ptr(da), _ptr(a), da.numel() // da.shape[-1],
+                                                 da.shape[-1], SLOPE, _ptr(dzb),
+                                                 _ptr(self.layers[i].gb), _stream()))
+            return dzb
 
-        def dgrad(i, dzb, like):
+        def dgrad(i, dzb):
             L = self.layers[i]
-            dx = torch.empty(like.shape[:4] + (L.cin,), dtype=torch.float32, device=self.dev)
+            dx = torch.empty(dzb.shape[:4] + (L.cin,), dtype=torch.float32, device=self.dev)
             if use_tc(L.cout, L.cin):
                 return conv_forward_tc(dzb, L.wt, None, L.cin, False, dx, None)[0]
             return conv_backward_data(dzb, L.wt, L.cin, dx)
 
-        dzb6 = bf(dout)
-        self._layer_grads(5, dout, dzb6, s["a5"])
-        da5 = dgrad(5, dzb6, dout)
-        dz5, dzb5 = leaky_bwd(da5, s["z5"])
-        self._layer_grads(4, dz5, dzb5, s["cat"])
-        dcat = dgrad(4, dzb5, dout)
-        da4 = torch.empty((n, d // 2, h // 2, w // 2, C2), dtype=torch.float32, device=self.dev)
-        check(lib.coffee_up2_backward(_ptr(dcat), n, d // 2, h // 2, w // 2, C2, C2 + C1, 0,
-                                      _ptr(da4), _stream()))
-        da2 = torch.zeros((n, d, h, w, C1), dtype=torch.float32, device=self.dev)
-        check(lib.coffee_channels_add(_ptr(dcat), full, C2 + C1, C2, C1, _ptr(da2), _stream()))
-        dz4, dzb4 = leaky_bwd(da4, s["z4"])
-        self._layer_grads(3, dz4, dzb4, s["a3"])
-        da3 = dgrad(3, dzb4, da4)
-        dz3, dzb3 = leaky_bwd(da3, s["z3"])
-        self._layer_grads(2, dz3, dzb3, s["p2"])
-        dp2 = dgrad(2, dzb3, da4)
-        check(lib.coffee_pool2_backward_add(_ptr(dp2), n, d, h, w, C1, _ptr(da2), _stream()))
-        dz2, dzb2 = leaky_bwd(da2, s["z2"])
-        self._layer_grads(1, dz2, dzb2, s["a1"])
-        da1 = dgrad(1, dzb2, da2)
-        dz1, dzb1 = leaky_bwd(da1, s["z1"])
-        self._layer_grads(0, dz1, dzb1, s["x"])
+        dzb6 = leaky(5, dout, None)
+        self._weight_grad(5, dzb6, s["a5"])
+        dzb5 = leaky(4, dgrad(5, dzb6), s["a5"])
+        self._weight_grad(4, dzb5, s["cat"])
+        dcat = dgrad(4, dzb5)
+        dzb4 = dz_like(s["a4"])
+        check(lib.coffee_up2_leaky_bias_backward(_ptr(dcat), n, d // 2, h // 2, w // 2, C2, C2 + C1,
+                                                 0, _ptr(s["a4"]), SLOPE, _ptr(dzb4),
+                                                 _ptr(self.layers[3].gb), _stream()))
+        self._weight_grad(3, dzb4, s["a3"])
+        dzb3 = leaky(2, dgrad(3, dzb4), s["a3"])
+        self._weight_grad(2, dzb3, s["p2"])
+        dp2 = dgrad(2, dzb3)
+        dzb2 = dz_like(s["a2"])
+        check(lib.coffee_skip_pool2_leaky_bias_backward(_ptr(dcat), C2 + C1, C2, _ptr(dp2), n, d, h,
+                                                        w, C1, _ptr(s["a2"]), SLOPE, _ptr(dzb2),
+                                                        _ptr(self.layers[1].gb), _stream()))
+        self._weight_grad(1, dzb2, s["a1"])
+        dzb1 = leaky(0, dgrad(1, dzb2), s["a1"])
+        self._weight_grad(0, dzb1, s["x"])
 
     def step(self, lr):
         self.t += 1

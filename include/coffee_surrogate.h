@@ -88,6 +88,25 @@ COFFEE_API int coffee_conv3d_backward_weight_tc(const void* dy, const void* x, i
  * (deterministic); calls that could overlap on the GPU (other streams, other
  * host threads) must not share a device. */
 COFFEE_API int coffee_bias_grad(const float* dz, long long npts, int k, float* db, void* stream);
+/* The backward pass's elementwise passes, fused: dz = da * leaky'(a) (a: the BF16
+ * activation, whose sign is its argument's; null: dz = da) as BF16, and db[k] =
+ * the sum of dz over the points.  8 <= c <= 64, a power of two; pointers
+ * 16-byte aligned.  up2: da is the gradient of a 2x nearest upsampling, channels
+ * off .. off + c of dy (cy channels at twice the grid n, d, h, w).  skip_pool2:
+ * da is channels off .. off + c of dcat (ccat channels) plus the gradient of a 2x
+ * average pooling, dp at half the grid. */
+COFFEE_API int coffee_leaky_bias_backward(const float* da, const void* a, long long npts, int c,
+                                          float slope, void* dz_bf16, float* db, void* stream);
+COFFEE_API int coffee_up2_leaky_bias_backward(const float* dy, int n, int d, int h, int w, int c,
+                                              int cy, int off, const void* a, float slope,
+                                              void* dz_bf16, float* db, void* stream);
+COFFEE_API int coffee_skip_pool2_leaky_bias_backward(const float* dcat, int ccat, int off,
+                                                     const float* dp, int n, int d, int h, int w,
+                                                     int c, const void* a, float slope,
+                                                     void* dz_bf16, float* db, void* stream);
+/* y = [up2(x), s]: c channels of the coarse x (grid n, d, h, w), then cs of s. */
+COFFEE_API int coffee_up2_concat(const void* x, int n, int d, int h, int w, int c, const void* s,
+                                 int cs, void* y, void* stream);
 /* dz = da * leaky'(z) (FP32 and a BF16 copy). */
 COFFEE_API int coffee_leaky_backward(const float* da, const float* z, long long count, float slope,
                                      float* dz, void* dz_bf16, void* stream);

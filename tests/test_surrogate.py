@@ -362,3 +362,67 @@ def test_rotator_warm_start_wall_time():
     if not r["wall_to_settle_warm_s"] < r["wall_to_settle_cold_s"]:
         pytest.xfail(f"warm start slower than cold: {r['wall_to_settle_warm_s']:.2f} s against "
                      f"{r['wall_to_settle_cold_s']:.2f} s (gain {r['gain']:.2f})")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c,shape", [(8, (1, 2, 2, 2)), (16, (3, 2, 6, 10)), (32, (1, 4, 4, 34)),
+                                     (64, (2, 6, 2, 2)), (16, (2, 32, 32, 32))])
+def test_fused_backward_passes_match_torch(c, shape):
+    """The fused elementwise passes against plain FP64 torch on the same
+    operands: BF16 outputs bitwise where one FP32 product is rounded once, else
+    within a BF16 ulp (2^-8); bias sums within FP32 rounding of the sum of
+    absolute values (2^-23 sqrt(n) with a factor of 8)."""
+    import torch
+
+    from coffee_b200 import _lib
+    from coffee_b200 import surrogate as sg
+
+    lib = _lib.load()
+    n, d, h, w = shape
+    gen = torch.Generator(device="cuda").manual_seed(c + d)
+
+    def rnd(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    a = rnd(n, d, h, w, c).to(torch.bfloat16)
+    a[0, 0, 0, 0, 0] = 0.0
+    slope = torch.where(a.double() > 0, 1.0, float(np.float32(0.1)))
+    db = torch.empty(c, device="cuda")
+    dzb = torch.empty(n, d, h, w, c, dtype=torch.bfloat16, device="cuda")
+
+    def compare(dz, exact):
+        ref = dz.float().to(torch.bfloat16)
+        if exact:
+            assert torch.equal(dzb, ref)
+        else:
+            assert float((dzb.double() - dz).abs().max()) <= 2 ** -8 * float(dz.abs().max())
+        bound = 8 * 2 ** -23 * dz.abs().sum((0, 1, 2, 3)) + 1e-30
+        assert bool(((db.double() - dz.sum((0, 1, 2, 3))).abs() <= bound).all())
+
+    ptr, stream = sg._ptr, sg._stream()
+    da = rnd(n, d, h, w, c)
+    sg.check(lib.coffee_leaky_bias_backward(ptr(da), ptr(a), n * d * h * w, c, 0.1, ptr(dzb),
+                                            ptr(db), stream))
+    compare((da.double() * slope).float().double(), True)
+    sg.check(lib.coffee_leaky_bias_backward(ptr(da), None, n * d * h * w, c, 0.1, ptr(dzb), ptr(db),
+                                            stream))
+    compare(da.double(), True)
+    # channels 4 .. 4 + c of a gradient of 12 + c channels at twice the grid
+    dy = rnd(n, 2 * d, 2 * h, 2 * w, c + 12)
+    sg.check(lib.coffee_up2_leaky_bias_backward(ptr(dy), n, d, h, w, c, c + 12, 4, ptr(a), 0.1,
+                                                ptr(dzb), ptr(db), stream))
+    s = dy[..., 4:4 + c].double().reshape(n, d, 2, h, 2, w, 2, c).sum((2, 4, 6))
+    compare(s * slope, False)
+    dcat, dp = rnd(n, d, h, w, c + 8), rnd(n, d // 2, h // 2, w // 2, c)
+    sg.check(lib.coffee_skip_pool2_leaky_bias_backward(ptr(dcat), c + 8, 8, ptr(dp), n, d, h, w, c,
+                                                       ptr(a), 0.1, ptr(dzb), ptr(db), stream))
+    up = dp.double()
+    for ax in (1, 2, 3):
+        up = up.repeat_interleave(2, ax)
+    compare((dcat[..., 8:].double() + 0.125 * up) * slope, False)
+    x = rnd(n, d // 2, h // 2, w // 2, c).to(torch.bfloat16)
+    y = torch.empty(n, d, h, w, 2 * c, dtype=torch.bfloat16, device="cuda")
+    sg.check(lib.coffee_up2_concat(ptr(x), n, d // 2, h // 2, w // 2, c, ptr(a), c, ptr(y), stream))
+    for ax in (1, 2, 3):
+        x = x.repeat_interleave(2, ax)
+    assert torch.equal(y, torch.cat([x, a], -1))
