@@ -33,6 +33,7 @@ struct EzConst {
   GridGeom g;
   T delta[3], inv_delta[3], lower[3];
   T dt, ch2, tau, inv_tau;
+  int tau_mid;      // |tau| is near enough to 1 for the straight-line P / tau
   T ko_c;           // -KOeps * KO_const, KO_const = -1/64
   T gam_dt;         // damp_gamma / dt
   int use_edotb, divB_clean, clean_ep, check_egb;

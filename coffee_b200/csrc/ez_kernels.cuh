@@ -20,6 +20,7 @@
 // global address is one wide multiply-add of an offset onto an array base.
 #pragma once
 
+#include "ez_pair.cuh"
 #include "ez_physics.cuh"
 
 namespace coffee {
@@ -46,11 +47,87 @@ __device__ __forceinline__ T d1_4(T m2, T m1, T p1, T p2, T s) {
   return ((m2 - p2) + (T)8 * (p1 - m1)) * s;
 }
 
+// The same of both fields of a pair.  XA: diff1_4 of the reference
+// (finite_diff_simd.h:15-25) before its inv_delta factor, the division by 12
+// as q = t / 12 (RN), q + (t - 12 q) / 12 (xa::div12_fast; it gives +0 for t =
+// -0), its input noted in `g`.
+template <bool XA, typename T>
+__device__ __forceinline__ Pair<T> pd1_4(Pair<T> m2, Pair<T> m1, Pair<T> p1, Pair<T> p2,
+                                         const T inv12, Guard<T>& g) {
+  if constexpr (XA) {
+    const Pair<T> r12 = both((T)(1.0 / 12.0));
+    Pair<T> t = pfma(m1, both((T)-8), m2);
+    t = pfma(p1, both((T)8), t);
+    t = psub(t, p2);
+    g.small(t);
+    const Pair<T> q = pmul(t, r12);
+    return pfma(pfma(q, both((T)-12), t), r12, q);
+  } else {
+    return pmul(pfma(psub(p1, m1), both((T)8), psub(m2, p2)), both(inv12));
+  }
+}
+template <bool XA, typename T>
+__device__ __forceinline__ T sd1_4(T m2, T m1, T p1, T p2, const T inv12, Guard<T>& g) {
+  if constexpr (XA) {
+    const T r12 = (T)(1.0 / 12.0);
+    T t = sfma(m1, (T)-8, m2);
+    t = sfma(p1, (T)8, t);
+    t = xa::sub(t, p2);
+    g.small(t);
+    const T q = smul(t, r12);
+    return sfma(sfma(q, (T)-12, t), r12, q);
+  } else {
+    return d1_4(m2, m1, p1, p2, inv12);
+  }
+}
+
 // 6th-order, 2nd-difference KO operator along one axis (reference diff6_2,
 // finite_diff.h:25-30): f-3 - 6 f-2 + 15 f-1 - 20 f0 + 15 f+1 - 6 f+2 + f+3.
 template <typename T>
 __device__ __forceinline__ T d6_2(T m3, T m2, T m1, T c, T p1, T p2, T p3) {
   return ((m3 + p3) - (T)6 * (m2 + p2)) + ((T)15 * (m1 + p1) - (T)20 * c);
+}
+
+// The same of both fields of a pair; XA: the reference's order and fused terms
+// (xa::d6).
+template <bool XA, typename T>
+__device__ __forceinline__ Pair<T> pd6_2(Pair<T> m3, Pair<T> m2, Pair<T> m1, Pair<T> c, Pair<T> p1,
+                                         Pair<T> p2, Pair<T> p3) {
+  if constexpr (XA) {
+    Pair<T> t = pfma(m2, both((T)-6), m3);
+    t = pfma(m1, both((T)15), t);
+    t = pfma(c, both((T)-20), t);
+    t = pfma(p1, both((T)15), t);
+    t = pfma(p2, both((T)-6), t);
+    return padd(p3, t);
+  } else {
+    Pair<T> t = pfma(padd(m2, p2), both((T)-6), padd(m3, p3));
+    t = pfma(padd(m1, p1), both((T)15), t);
+    return pfma(c, both((T)-20), t);
+  }
+}
+
+// The CPU build's clamps (apply_clamps_xa) on v = (E, B, P) with the
+// straight-line quotients; a point outside their range is done again with the
+// IEEE operations.
+template <typename T>
+__device__ __forceinline__ void apply_clamps_mid(T v[7]) {
+  Guard<T> g;
+  const T N2 = xa::floor_tiny(xa::dot3(v[3], v[3], v[4], v[4], v[5], v[5]));
+  const T EB = xa::dot3(v[3], v[0], v[4], v[1], v[5], v[2]);
+  const T y = rcp_mid(N2);
+  const Pair<T> q01 = pdiv_mid(pk(xa::mul(EB, v[3]), xa::mul(EB, v[4])), both(-N2), both(y), g);
+  const Pair<T> q2 = pdiv_mid(both(xa::mul(EB, v[5])), both(-N2), both(y), g);
+  T e[3] = {xa::sub(v[0], first(q01)), xa::sub(v[1], second(q01)), xa::sub(v[2], first(q2))};
+  const T E2 = xa::dot3(e[0], e[0], e[1], e[1], e[2], e[2]);
+  g.below(N2, MidRange<T>::den_max);
+  g.below(E2, MidRange<T>::num_max);
+  if (g.bad() || E2 > N2) {
+    apply_clamps_xa(v[0], v[1], v[2], v[3], v[4], v[5]);
+  } else {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[a] = e[a];
+  }
 }
 
 // Write the 7 new values of point (i, j, k) (linear index o) to `out` at the
@@ -86,12 +163,6 @@ __device__ __forceinline__ void store_with_images(const GridGeom& g, const Colum
   }
 }
 
-// Everything a stage does at one point once its derivatives are known:
-// the current J, the new accumulators dU (from dold unless FIRST), the new
-// fields U + Bs dU, the clamps, the star boundary, the absorbing layer
-// (ST_LAST) and the stores of dU, J/divE/divB (ST_AUX), Un (ST_WRITE_UN) and
-// of U' with its guard images.  d{x,y,z}[f] are the inv_delta-scaled
-// 4th-order derivatives of field f at the point, u[f] its values.
 // Curl, divergence and gradient of the fields at one point, as the stage
 // needs them (all inv_delta-scaled 4th-order differences).
 template <typename T>
@@ -99,127 +170,273 @@ struct Derivs {
   T rotE[3], rotB[3], divE, divB, gradP[3];
 };
 
-// XA selects the CPU build's own arithmetic (ez_refarith.cuh) for the
-// current, the taper, the accumulators, the update and the clamps; the
-// derivatives then come in already combined in that arithmetic (Derivs).
-template <typename T, bool FIRST, bool BC, bool XA, bool DG>
-__device__ __forceinline__ void stage_point(const EzConst<T>& c, const T u[7],
-                                            const Derivs<T>& dv, const T dold[7],
-                                            const T As, const T Bs, const T tst,
-                                            const int flags, const ColumnCtx<T>& col,
-                                            const int k, const uint32_t o, const F7<T>& du,
-                                            const F7<T>& un, const F5<T>& aux,
-                                            const F7<T>& uout, const F6<T>& dg) {
-  const bool cpu = c.semantics == SEM_CPU_REF;
+// What a stage computes at one point before the boundaries: the new
+// accumulators and fields, the current and the divergences.
+template <typename T>
+struct StageValues {
+  T d[7], nu[7], J[3], divE, divB;
+};
+
+// One stage at a point in the CPU build's own arithmetic, operation for
+// operation (rk_step and clean_epar_check_eGTb, field_solver_EZ.cpp:143-259,
+// 552-634; ez_refarith.cuh), with the IEEE divisions and roots.  With DG the
+// clamps add to the energy-change diagnostics at point o.
+template <bool FIRST, bool DG, typename T>
+__device__ __forceinline__ void stage_values_ieee(const EzConst<T>& c, const T u[7],
+                                                  const Derivs<T>& dv, const T dold[7],
+                                                  const T As, const T Bs,
+                                                  const ColumnCtx<T>& col, const int k,
+                                                  const F6<T>& dg, const uint32_t o,
+                                                  StageValues<T>& r) {
   const T ex = u[0], ey = u[1], ez = u[2], bx = u[3], by = u[4], bz = u[5], P = u[6];
   const T rotBx = dv.rotB[0], rotBy = dv.rotB[1], rotBz = dv.rotB[2];
   const T rotEx = dv.rotE[0], rotEy = dv.rotE[1], rotEz = dv.rotE[2];
   const T divE = dv.divE;
   const T divB = dv.divB;
-  T d[7];
+  T* d = r.d;
   T Jx, Jy, Jz;
-  if constexpr (XA) {
-    // rk_step of the CPU build (field_solver_EZ.cpp:143-259) operation for
-    // operation
-    const T B2 = xa::floor_tiny(xa::dot3(bx, bx, by, by, bz, bz));
-    const T BrotB = xa::dot3(bx, rotBx, by, rotBy, bz, rotBz);
-    const T ErotE = xa::dot3(ex, rotEx, ey, rotEy, ez, rotEz);
-    const T cx = xa::fma(-by, ez, xa::mul(bz, ey));
-    const T cy = xa::fma(-bz, ex, xa::mul(bx, ez));
-    const T cz = xa::fma(-bx, ey, xa::mul(by, ex));
-    if (c.use_edotb) {
-      const T E2 = xa::dot3(ex, ex, ey, ey, ez, ez);
-      const T chi2 = xa::sub(B2, E2);
-      const T EdotB = xa::dot3(bx, ex, by, ey, bz, ez);
-      const T E02 = xa::fma(
-          xa::sub(xa::sqrt(xa::fma(xa::mul(EdotB, (T)4), EdotB, xa::mul(chi2, chi2))), chi2),
-          (T)0.5, B2);
-      const T Jp = xa::fma(EdotB, c.gam_dt, xa::sub(BrotB, ErotE));
-      Jx = xa::add(xa::div(xa::mul(divE, cx), E02), xa::div(xa::mul(bx, Jp), B2));
-      Jy = xa::add(xa::div(xa::mul(divE, cy), E02), xa::div(xa::mul(by, Jp), B2));
-      Jz = xa::add(xa::div(xa::mul(divE, cz), E02), xa::div(xa::mul(bz, Jp), B2));
-    } else {
-      const T Jp = xa::sub(BrotB, ErotE);
-      Jx = xa::div(xa::fma(bx, Jp, xa::mul(divE, cx)), B2);
-      Jy = xa::div(xa::fma(by, Jp, xa::mul(divE, cy)), B2);
-      Jz = xa::div(xa::fma(bz, Jp, xa::mul(divE, cz)), B2);
-    }
-    T Px = 0, Py = 0, Pz = 0;
-    if (c.divB_clean) {
-      Px = dv.gradP[0];
-      Py = dv.gradP[1];
-      Pz = dv.gradP[2];
-    }
-    const T s = p_taper_xa(c, col, k);
-    const T dt = c.dt;
-    // dU As (As = 0 on the first stage, where the old dU is not read)
-    T da[7];
-#pragma unroll
-    for (int f = 0; f < 7; ++f) {
-      if constexpr (FIRST) da[f] = (T)0;
-      else da[f] = xa::mul(dold[f], As);
-    }
-    d[0] = xa::fma(dt, xa::sub(rotBx, Jx), da[0]);
-    d[1] = xa::fma(dt, xa::sub(rotBy, Jy), da[1]);
-    d[2] = xa::fma(dt, xa::sub(rotBz, Jz), da[2]);
-    d[3] = xa::fma(-dt, xa::fma(Px, s, rotEx), da[3]);
-    d[4] = xa::fma(-dt, xa::fma(Py, s, rotEy), da[4]);
-    d[5] = xa::fma(-dt, xa::fma(Pz, s, rotEz), da[5]);
-    // dP As - P / tau with the product fused, minus dt (divB ch2)
-    if constexpr (FIRST)
-      d[6] = xa::fma(-dt, xa::mul(divB, c.ch2), -xa::div(P, c.tau));
-    else
-      d[6] = xa::fma(-dt, xa::mul(divB, c.ch2), xa::fma(dold[6], As, -xa::div(P, c.tau)));
+  const T B2 = xa::floor_tiny(xa::dot3(bx, bx, by, by, bz, bz));
+  const T BrotB = xa::dot3(bx, rotBx, by, rotBy, bz, rotBz);
+  const T ErotE = xa::dot3(ex, rotEx, ey, rotEy, ez, rotEz);
+  const T cx = xa::fma(-by, ez, xa::mul(bz, ey));
+  const T cy = xa::fma(-bz, ex, xa::mul(bx, ez));
+  const T cz = xa::fma(-bx, ey, xa::mul(by, ex));
+  if (c.use_edotb) {
+    const T E2 = xa::dot3(ex, ex, ey, ey, ez, ez);
+    const T chi2 = xa::sub(B2, E2);
+    const T EdotB = xa::dot3(bx, ex, by, ey, bz, ez);
+    const T E02 = xa::fma(
+        xa::sub(xa::sqrt(xa::fma(xa::mul(EdotB, (T)4), EdotB, xa::mul(chi2, chi2))), chi2),
+        (T)0.5, B2);
+    const T Jp = xa::fma(EdotB, c.gam_dt, xa::sub(BrotB, ErotE));
+    Jx = xa::add(xa::div(xa::mul(divE, cx), E02), xa::div(xa::mul(bx, Jp), B2));
+    Jy = xa::add(xa::div(xa::mul(divE, cy), E02), xa::div(xa::mul(by, Jp), B2));
+    Jz = xa::add(xa::div(xa::mul(divE, cz), E02), xa::div(xa::mul(bz, Jp), B2));
   } else {
-    T B2 = bx * bx + by * by + bz * bz;
-    if (B2 < Tiny<T>::v) B2 = Tiny<T>::v;
-    const T BrotB = bx * rotBx + by * rotBy + bz * rotBz;
-    const T ErotE = ex * rotEx + ey * rotEy + ez * rotEz;
-    const T cx = ey * bz - ez * by, cy = ez * bx - ex * bz, cz = ex * by - ey * bx;
-    if (c.use_edotb) {
-      // J with E.B damping (field_solver_EZ.cpp:170-186, .cu:72-91)
-      const T E2 = ex * ex + ey * ey + ez * ez;
-      const T chi2 = B2 - E2;
-      const T EdotB = ex * bx + ey * by + ez * bz;
-      const T E02 = (T)0.5 * (sqrt(chi2 * chi2 + (T)4 * EdotB * EdotB) - chi2) + B2;
-      const T Jp = BrotB - ErotE + EdotB * c.gam_dt;
-      const T a = fdiv(divE, E02), b = fdiv(Jp, B2);
-      Jx = a * cx + b * bx;
-      Jy = a * cy + b * by;
-      Jz = a * cz + b * bz;
-    } else {
-      const T Jp = BrotB - ErotE;
-      const T rB2 = fdiv((T)1, B2);
-      Jx = (divE * cx + Jp * bx) * rB2;
-      Jy = (divE * cy + Jp * by) * rB2;
-      Jz = (divE * cz + Jp * bz) * rB2;
-    }
-    T Px = 0, Py = 0, Pz = 0;
-    if (c.divB_clean) {
-      Px = dv.gradP[0];
-      Py = dv.gradP[1];
-      Pz = dv.gradP[2];
-      if (cpu) {
-        const T s = p_taper(c, col, k);
-        Px *= s;
-        Py *= s;
-        Pz *= s;
-      }
-    }
-    // new accumulators
-    const T dt = c.dt;
-    d[0] = (rotBx - Jx) * dt;
-    d[1] = (rotBy - Jy) * dt;
-    d[2] = (rotBz - Jz) * dt;
-    d[3] = -(rotEx + Px) * dt;
-    d[4] = -(rotEy + Py) * dt;
-    d[5] = -(rotEz + Pz) * dt;
-    d[6] = -P * c.inv_tau - divB * c.ch2 * dt;
-    if constexpr (!FIRST) {
+    const T Jp = xa::sub(BrotB, ErotE);
+    Jx = xa::div(xa::fma(bx, Jp, xa::mul(divE, cx)), B2);
+    Jy = xa::div(xa::fma(by, Jp, xa::mul(divE, cy)), B2);
+    Jz = xa::div(xa::fma(bz, Jp, xa::mul(divE, cz)), B2);
+  }
+  T Px = 0, Py = 0, Pz = 0;
+  if (c.divB_clean) {
+    Px = dv.gradP[0];
+    Py = dv.gradP[1];
+    Pz = dv.gradP[2];
+  }
+  const T s = p_taper_xa(c, col, k);
+  const T dt = c.dt;
+  // dU As (As = 0 on the first stage, where the old dU is not read)
+  T da[7];
 #pragma unroll
-      for (int f = 0; f < 7; ++f) d[f] = fma(dold[f], As, d[f]);
+  for (int f = 0; f < 7; ++f) {
+    if constexpr (FIRST) da[f] = (T)0;
+    else da[f] = xa::mul(dold[f], As);
+  }
+  d[0] = xa::fma(dt, xa::sub(rotBx, Jx), da[0]);
+  d[1] = xa::fma(dt, xa::sub(rotBy, Jy), da[1]);
+  d[2] = xa::fma(dt, xa::sub(rotBz, Jz), da[2]);
+  d[3] = xa::fma(-dt, xa::fma(Px, s, rotEx), da[3]);
+  d[4] = xa::fma(-dt, xa::fma(Py, s, rotEy), da[4]);
+  d[5] = xa::fma(-dt, xa::fma(Pz, s, rotEz), da[5]);
+  // dP As - P / tau with the product fused, minus dt (divB ch2)
+  if constexpr (FIRST)
+    d[6] = xa::fma(-dt, xa::mul(divB, c.ch2), -xa::div(P, c.tau));
+  else
+    d[6] = xa::fma(-dt, xa::mul(divB, c.ch2), xa::fma(dold[6], As, -xa::div(P, c.tau)));
+  // mul_add(dU, Bs, U), then clean_epar_check_eGTb
+  T* nu = r.nu;
+#pragma unroll
+  for (int f = 0; f < 7; ++f) nu[f] = xa::fma(d[f], Bs, u[f]);
+  if constexpr (DG)
+    apply_clamps_xa_dg<FIRST>(nu[0], nu[1], nu[2], nu[3], nu[4], nu[5], dg, o);
+  else
+    apply_clamps_xa(nu[0], nu[1], nu[2], nu[3], nu[4], nu[5]);
+  r.J[0] = Jx;
+  r.J[1] = Jy;
+  r.J[2] = Jz;
+  r.divE = divE;
+  r.divB = divB;
+}
+
+// The derivatives of one point from global memory with the IEEE division.
+template <typename T>
+__device__ __noinline__ Derivs<T> point_derivatives_ieee(const EzConst<T>& c,
+                                                         const F7<const T> uin, const uint32_t o) {
+  const uint32_t st[3] = {1u, (uint32_t)c.g.sy, (uint32_t)c.g.sz};
+  T g[7][3];
+  for (int f = 0; f < 7; ++f) {
+    const T* p = uin.p[f] + o;
+    for (int a = 0; a < 3; ++a) {
+      const long long t = st[a];
+      uint32_t unused = 0xFFFFFFFFu;
+      g[f][a] = xa::dq<true>(p[-2 * t], p[-t], p[t], p[2 * t], unused);
     }
   }
+  const T ix = c.inv_delta[0], iy = c.inv_delta[1], iz = c.inv_delta[2];
+  Derivs<T> dv;
+  auto curl_div = [&](int b, T* rot, T& dvg) {
+    rot[0] = xa::fma(-iz, g[b + 1][2], xa::mul(iy, g[b + 2][1]));
+    rot[1] = xa::fma(-ix, g[b + 2][0], xa::mul(iz, g[b][2]));
+    rot[2] = xa::fma(-iy, g[b][1], xa::mul(ix, g[b + 1][0]));
+    dvg = xa::fma(iz, g[b + 2][2], xa::fma(iy, g[b + 1][1], xa::mul(ix, g[b][0])));
+  };
+  curl_div(0, dv.rotE, dv.divE);
+  curl_div(3, dv.rotB, dv.divB);
+  dv.gradP[0] = xa::mul(ix, g[6][0]);
+  dv.gradP[1] = xa::mul(iy, g[6][1]);
+  dv.gradP[2] = xa::mul(iz, g[6][2]);
+  return dv;
+}
+
+// The same stage of one point from global memory, out of line: for the rare
+// points whose operands the straight-line arithmetic of stage_values_pair
+// does not cover (Guard).
+template <bool FIRST, typename T>
+__device__ __noinline__ StageValues<T> stage_point_ieee(const EzConst<T>& c, const F7<const T> uin,
+                                                        const F7<T> du, const ColumnCtx<T> col,
+                                                        const int k, const uint32_t o, const T As,
+                                                        const T Bs) {
+  T u[7], dold[7];
+  for (int f = 0; f < 7; ++f) {
+    u[f] = uin.p[f][o];
+    dold[f] = FIRST ? (T)0 : du.p[f][o];
+  }
+  const Derivs<T> dv = point_derivatives_ieee(c, uin, o);
+  StageValues<T> r;
+  F6<T> none;
+  stage_values_ieee<FIRST, false>(c, u, dv, dold, As, Bs, col, k, none, o, r);
+  return r;
+}
+
+// One stage at a point from its pairs: eb[a] = (E_a, B_a), rot and dvg the
+// pairs of their curls and divergences, dold the old accumulators of (E_a,
+// B_a) and of P.  XA: the CPU build's arithmetic, with straight-line
+// quotients and roots (ez_pair.cuh); `g` notes operands outside their range,
+// and the caller then uses stage_point_ieee.  Otherwise the regrouped
+// arithmetic: the same algorithm with shared divisions.
+template <bool FIRST, bool XA, typename T>
+__device__ __forceinline__ void stage_values_pair(const EzConst<T>& c, const Pair<T> eb[3],
+                                                  const T P, const Pair<T> rot[3],
+                                                  const Pair<T> dvg, const T gradP[3],
+                                                  const Pair<T> dold[3], const T doldP, const T As,
+                                                  const T Bs, const ColumnCtx<T>& col, const int k,
+                                                  Pair<T> d[3], T& dP, Pair<T> nu[3], T& nuP,
+                                                  T J[3], Guard<T>& g) {
+  const T divE = first(dvg), divB = second(dvg);
+  const T e[3] = {first(eb[0]), first(eb[1]), first(eb[2])};
+  const T b[3] = {second(eb[0]), second(eb[1]), second(eb[2])};
+  const Pair<T> sq = pdot3(eb, eb), br = pdot3(eb, rot);  // (E2, B2), (E.rotE, B.rotB)
+  const T B2 = xa::floor_tiny(second(sq));
+  const T dt = c.dt;
+  const T C[3] = {xa::fma(-b[1], e[2], xa::mul(b[2], e[1])),
+                  xa::fma(-b[2], e[0], xa::mul(b[0], e[2])),
+                  xa::fma(-b[0], e[1], xa::mul(b[1], e[0]))};
+  T Jp = xa::sub(second(br), first(br));
+  T Ptau;  // P / tau
+  T q[3];  // (E.B) B_a / B^2 of the clamps
+  if constexpr (XA) {
+    if (c.use_edotb) {
+      const T chi2 = xa::sub(B2, first(sq));
+      const T EdotB = xa::dot3(b[0], e[0], b[1], e[1], b[2], e[2]);
+      const T s2 = xa::fma(xa::mul(EdotB, (T)4), EdotB, xa::mul(chi2, chi2));
+      const T E02 = xa::fma(xa::sub(sqrt_floor(s2), chi2), (T)0.5, B2);
+      Jp = xa::fma(EdotB, c.gam_dt, Jp);
+      g.below(E02, MidRange<T>::den_max);
+      const Pair<T> nden = pk(-E02, -B2);
+      Pair<T> y = pk(rcp_seed(E02), rcp_seed(B2));
+      y = pfma(pfma(nden, y, both((T)1)), y, y);
+      const Pair<T> f = pk(divE, Jp);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const Pair<T> t = pdiv_mid(pmul(f, pk(C[a], b[a])), nden, y, g);
+        J[a] = xa::add(first(t), second(t));
+      }
+    } else {
+      g.below(B2, MidRange<T>::den_max);
+      const Pair<T> nden = both(-B2), y = both(rcp_mid(B2));
+      T n[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) n[a] = xa::fma(b[a], Jp, xa::mul(divE, C[a]));
+      const Pair<T> t01 = pdiv_mid(pk(n[0], n[1]), nden, y, g);
+      J[0] = first(t01);
+      J[1] = second(t01);
+      J[2] = first(pdiv_mid(both(n[2]), nden, y, g));
+    }
+  } else if (c.use_edotb) {
+    // J with E.B damping (field_solver_EZ.cpp:170-186, .cu:72-91)
+    const T chi2 = B2 - first(sq);
+    const T EdotB = e[0] * b[0] + e[1] * b[1] + e[2] * b[2];
+    const T E02 = (T)0.5 * (sqrt(chi2 * chi2 + (T)4 * EdotB * EdotB) - chi2) + B2;
+    const T x = fdiv(divE, E02), y = fdiv(Jp + EdotB * c.gam_dt, B2);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) J[a] = x * C[a] + y * b[a];
+  } else {
+    const T rB2 = fdiv((T)1, B2);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) J[a] = (divE * C[a] + Jp * b[a]) * rB2;
+  }
+  // the P gradient with its taper (CPU semantics), 0 without the cleaning
+  T s = 0;
+  if (c.divB_clean) {
+    if constexpr (XA) s = p_taper_mid(c, col, k, g);
+    else s = c.semantics == SEM_CPU_REF ? p_taper(c, col, k) : (T)1;
+  }
+  // new accumulators and fields
+  const Pair<T> pdt = pk(dt, -dt);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const Pair<T> da = FIRST ? both((T)0) : pmul(dold[a], both(As));
+    const Pair<T> w = pk(xa::sub(second(rot[a]), J[a]), xa::fma(gradP[a], s, first(rot[a])));
+    d[a] = pfma(pdt, w, da);
+    nu[a] = pfma(d[a], both(Bs), eb[a]);
+  }
+  // E.B = 0 and |E| <= |B|
+  T ne[3] = {first(nu[0]), first(nu[1]), first(nu[2])};
+  const T nb[3] = {second(nu[0]), second(nu[1]), second(nu[2])};
+  if constexpr (XA) {
+    const T N2 = xa::floor_tiny(xa::dot3(nb[0], nb[0], nb[1], nb[1], nb[2], nb[2]));
+    const T EB = xa::dot3(nb[0], ne[0], nb[1], ne[1], nb[2], ne[2]);
+    const T y = rcp_mid(N2);
+    const Pair<T> q01 =
+        pdiv_mid(pk(xa::mul(EB, nb[0]), xa::mul(EB, nb[1])), both(-N2), both(y), g);
+    const Pair<T> q2P = pdiv_mid(pk(xa::mul(EB, nb[2]), P), pk(-N2, -c.tau), pk(y, c.inv_tau), g);
+    q[0] = first(q01);
+    q[1] = second(q01);
+    q[2] = first(q2P);
+    Ptau = second(q2P);
+    g.below(N2, MidRange<T>::den_max);
+    g.below(xa::mul(P, P), MidRange<T>::num_max);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) ne[a] = xa::sub(ne[a], q[a]);
+    const T E2 = xa::dot3(ne[0], ne[0], ne[1], ne[1], ne[2], ne[2]);
+    g.below(E2, MidRange<T>::num_max);
+    if (E2 > N2) {
+      const T m = xa::sqrt(xa::div(N2, E2));
+#pragma unroll
+      for (int a = 0; a < 3; ++a) ne[a] = xa::mul(ne[a], m);
+    }
+  } else {
+    Ptau = P * c.inv_tau;
+    apply_clamps(c, ne[0], ne[1], ne[2], nb[0], nb[1], nb[2]);
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) nu[a] = pk(ne[a], nb[a]);
+  // dP As - P / tau with the product fused, minus dt (divB ch2)
+  dP = xa::fma(-dt, xa::mul(divB, c.ch2), FIRST ? -Ptau : xa::fma(doldP, As, -Ptau));
+  nuP = xa::fma(dP, Bs, P);
+}
+
+// The rest of a stage at one point: the start-of-step copy, the stores of the
+// accumulators and of J, div E and div B, the star boundary, the absorbing
+// layer and the store of the fields with their guard images.
+template <bool BC, typename T>
+__device__ __forceinline__ void stage_finish(const EzConst<T>& c, const T u[7], const T d[7],
+                                             T nu[7], const T J[3], const T divE, const T divB,
+                                             const T tst, const int flags,
+                                             const ColumnCtx<T>& col, const int k,
+                                             const uint32_t o, const F7<T>& du, const F7<T>& un,
+                                             const F5<T>& aux, const F7<T>& uout) {
   // the start-of-step copy is only read inside the absorbing layer
   T sig = (T)0;
   if constexpr (BC) sig = c.absorbing ? absorbing_sigma(c, col.i, col.j, k) : (T)0;
@@ -230,25 +447,11 @@ __device__ __forceinline__ void stage_point(const EzConst<T>& c, const T u[7],
 #pragma unroll
   for (int f = 0; f < 7; ++f) du.p[f][o] = d[f];
   if ((flags & ST_AUX) != 0) {
-    aux.p[0][o] = Jx;
-    aux.p[1][o] = Jy;
-    aux.p[2][o] = Jz;
+    aux.p[0][o] = J[0];
+    aux.p[1][o] = J[1];
+    aux.p[2][o] = J[2];
     aux.p[3][o] = divE;
     aux.p[4][o] = divB;
-  }
-  T nu[7];
-  if constexpr (XA) {
-    // mul_add(dU, Bs, U), then clean_epar_check_eGTb
-#pragma unroll
-    for (int f = 0; f < 7; ++f) nu[f] = xa::fma(d[f], Bs, u[f]);
-    if constexpr (DG)
-      apply_clamps_xa_dg<FIRST>(nu[0], nu[1], nu[2], nu[3], nu[4], nu[5], dg, o);
-    else
-      apply_clamps_xa(nu[0], nu[1], nu[2], nu[3], nu[4], nu[5]);
-  } else {
-#pragma unroll
-    for (int f = 0; f < 7; ++f) nu[f] = fma(d[f], Bs, u[f]);
-    apply_clamps(c, nu[0], nu[1], nu[2], nu[3], nu[4], nu[5]);
   }
   if constexpr (BC) star_boundary(c, col.i, col.j, k, tst, nu);
   if (BC && (flags & ST_LAST) != 0 && sig > (T)0) {
@@ -271,11 +474,11 @@ __device__ __forceinline__ void stage_point(const EzConst<T>& c, const T u[7],
 // in FP32), which needs an even row length d0: the copied row then starts at
 // the even column at or left of the tile's first column, `xoff` (0 or 1)
 // columns before it, and a row holds TX + 2H + 2 elements.
-template <typename T, int TX, int TY, int H, int V = 1>
+template <typename T, int TX, int TY, int H, int V = 1, int THREADS = TX * TY>
 struct TileLoader {
   static_assert(V == 1 || V == 2, "one element or an aligned pair per copy");
   static constexpr int SX = TX + 2 * H + (V == 2 ? 2 : 0);  // shared row stride (elements)
-  static constexpr int SY = TY + 2 * H, NT = TX * TY;
+  static constexpr int SY = TY + 2 * H, NT = THREADS;
   static constexpr int PER_ROW = SX / V;                    // copies per row
   static constexpr int NCOPY = PER_ROW * SY;
   static constexpr int NLOAD = (NCOPY + NT - 1) / NT;
@@ -316,6 +519,49 @@ struct TileLoader {
   }
 };
 
+// Per-thread copies of one (TX + 2H) x (TY + 2H) tile of one plane of the 7
+// fields into a ring slot, interleaved: element e of pair a (E_a, B_a) lies at a
+// PB + 2 e elements, of P at 3 PB + e, so that one 64-bit shared load (FP32)
+// reads both halves of a pair.  The copies are one element each: they need no
+// alignment of a row.
+template <typename T, int TX, int TY, int H>
+struct PairLoader {
+  static constexpr int SX = TX + 2 * H, SY = TY + 2 * H, NT = TX * TY;
+  static constexpr int NCOPY = SX * SY, NLOAD = (NCOPY + NT - 1) / NT;
+  static constexpr int ES = (int)sizeof(T);
+  static constexpr int PB = 2 * NCOPY * ES;      // bytes of a pair's plane
+  static constexpr int SB = 7 * NCOPY * ES;      // bytes of a ring slot
+  static constexpr uint32_t kNone = 0xFFFFFFFFu;
+  uint32_t pair0, p0;     // shared addresses of this thread's first element in slot 0
+  uint32_t eoff[NLOAD];   // element offsets within a global plane, or kNone
+
+  __device__ __forceinline__ PairLoader(const GridGeom& g, uint32_t sbase, int tid, int gx0,
+                                        int gy0) {
+    pair0 = sbase + (uint32_t)(2 * tid * ES);
+    p0 = sbase + (uint32_t)(3 * PB + tid * ES);
+#pragma unroll
+    for (int m = 0; m < NLOAD; ++m) {
+      const int e = tid + m * NT, r = e / SX, x = gx0 + e - r * SX, y = gy0 + r;
+      eoff[m] = e < NCOPY && x < g.dims[0] && y < g.dims[1]
+                    ? (uint32_t)y * (uint32_t)g.sy + (uint32_t)x
+                    : kNone;
+    }
+  }
+  __device__ __forceinline__ void copy(const F7<const T>& uin, uint32_t pe, uint32_t slot) const {
+    static_for<NLOAD>([&](auto mc) {
+      constexpr int m = decltype(mc)::value;
+      if (eoff[m] == kNone) return;
+      const uint32_t e = pe + eoff[m], d = pair0 + slot;
+      static_for<3>([&](auto ac) {
+        constexpr int a = decltype(ac)::value;
+        cp_async_off<ES, a * PB + 2 * m * NT * ES>(d, uin.p[a] + e);
+        cp_async_off<ES, a * PB + (2 * m * NT + 1) * ES>(d, uin.p[3 + a] + e);
+      });
+      cp_async_off<ES, m * NT * ES>(p0 + slot, uin.p[6] + e);
+    });
+  }
+};
+
 // ---------------------------------------------------------------------------
 // One LSRK stage (reference rk_step + clamps + star boundary + absorbing
 // layer + send_guard_cells, src/algorithms/field_solver_EZ.cpp:1024-1055,
@@ -326,84 +572,235 @@ struct TileLoader {
 //   U'  <- U + Bs dU
 //   U'  <- clamps, star boundary at tst, absorbing layer (ST_LAST)
 // reading U from `uin` and writing U' (with guard images) to `uout`.
-// Shared memory: a ring of 3 + PF + kRingSpare planes (k .. k+2, the
-// prefetch, the spare) of the 7 fields with a 2-point x/y halo, then
-// PF + 1 + kRingSpare planes of dU.  The z
-// neighbours of a thread's own column are kept in a register window of
-// planes k-2 .. k+2: each plane is read from shared memory once, as the
-// window's leading plane.
+//
+// This is the FP64 kernel (and the FP32 one of runs with both the boundary code and the
+// diagnostics).  The ring of 5 + PF + SPARE planes (k-2 .. k+2, the prefetch, a spare
+// that saves the second barrier) holds the whole stencil as pairs, read at
+// compile-time offsets; with the z neighbours in the ring instead of a register
+// window a thread's registers hold one point only, which in FP64 lets 12 warps of 168
+// registers share an SM.  FP64 stage at 256^3: 2610 us with a register window, 4 warps
+// a CTA and IEEE divisions, 1320 us here.  What bounds it is the latency between
+// dependent FP64 operations.  The old dU of a point is loaded at the top of its plane
+// and used after the derivatives.
 // ---------------------------------------------------------------------------
-// z-loop unroll of the stage kernel: 5 (the window length, no register
-// moves) or 1 (one plane per iteration, window shifted by moves), chosen
-// separately for the instances without and with the boundary code (BC):
-// the five copies of the out-of-line boundary calls make the BC instance
-// spill, and it runs faster plane by plane.
-#ifndef COFFEE_STAGE_ZUNROLL
-#define COFFEE_STAGE_ZUNROLL 5
-#endif
-#ifndef COFFEE_STAGE_ZUNROLL_BC
-#define COFFEE_STAGE_ZUNROLL_BC 1
-#endif
-template <bool BC>
-__host__ __device__ constexpr int stage_zunroll() {
-  return BC ? COFFEE_STAGE_ZUNROLL_BC : COFFEE_STAGE_ZUNROLL;
-}
-static_assert((stage_zunroll<false>() == 1 || stage_zunroll<false>() == 5) &&
-                  (stage_zunroll<true>() == 1 || stage_zunroll<true>() == 5),
-              "stage z unroll is 1 or 5");
-
-// Spare ring slots (0 or 1) of the stage and KO kernels.  With a spare slot
-// the copies of a new plane are issued right after the one barrier at the
-// top of an iteration, into the slot of the plane the previous iteration
-// finished with; without it they wait for a second barrier after the
-// iteration's arithmetic.  Measured at 512^3: the stage kernel is faster with
-// the spare slot, the KO kernel (two CTAs per SM) without.
-#ifndef COFFEE_STAGE_RING_SPARE
-#define COFFEE_STAGE_RING_SPARE 1
-#endif
-#ifndef COFFEE_KO_RING_SPARE
-#define COFFEE_KO_RING_SPARE 0
-#endif
-constexpr int kRingSpare = COFFEE_STAGE_RING_SPARE;
-constexpr int kKoRingSpare = COFFEE_KO_RING_SPARE;
-static_assert((kRingSpare == 0 || kRingSpare == 1) && (kKoRingSpare == 0 || kKoRingSpare == 1),
-              "0 or 1 spare ring slot");
-
-// Ring slots of the stage kernel.  Plane k lives in slot (k - lo[2]) % R of
-// the field ring and its dU in slot (k - lo[2]) % DR of the dU ring.  With
-// PF = 1 and the spare slot the field ring has 5 slots, the z unroll length:
-// every chunk then starts a multiple of 5 planes from lo[2] (the host picks
-// such chunks) and the field slot of every plane an unrolled iteration
-// touches is a compile-time constant.  (Rings grown to make the dU slots
-// constant too measured slower: shared memory taken from the L1 cache.)
-template <bool BC, int PF>
-__host__ __device__ constexpr int stage_ring() {
-  return 3 + PF + kRingSpare;
-}
-template <bool BC, int PF>
-__host__ __device__ constexpr int stage_dring() {
-  return PF + 1 + kRingSpare;
-}
-
-template <typename T, int TX, int TY, int PF, int V, bool BC>
-constexpr size_t stage_smem_bytes(bool first) {
-  return (size_t)stage_ring<BC, PF>() * 7 * TileLoader<T, TX, TY, 2, V>::FB +
-         (first ? 0 : (size_t)stage_dring<BC, PF>() * 7 * TX * TY * sizeof(T));
+template <typename T, int TX, int TY, int PF, int SPARE>
+constexpr size_t stage_smem_bytes() {
+  return (size_t)(5 + PF + SPARE) * PairLoader<T, TX, TY, 2>::SB;
 }
 
 // DG (with XA only): also accumulate the CPU build's energy-change
 // diagnostics of the clamps into dg.
-template <typename T, int TX, int TY, int PF, bool FIRST, bool BC, int V, bool XA, bool DG>
-__global__ void __launch_bounds__(TX * TY, min_blocks<T, TX * TY>())
+template <typename T, int TX, int TY, int PF, int SPARE, int MINB, bool FIRST, bool BC, bool XA,
+          bool DG>
+__global__ void __launch_bounds__(TX * TY, MINB)
     ez_stage_kernel(const __grid_constant__ EzConst<T> c, const F7<const T> uin,
                     const F7<T> uout, const F7<T> du, const F7<T> un, const F5<T> aux,
                     const F6<T> dg, const T As, const T Bs, const T tst, const int kchunk,
                     const int flags) {
   static_assert(XA || !DG, "the energy diagnostics need the reference arithmetic");
+  using L = PairLoader<T, TX, TY, 2>;
+  constexpr int R = 5 + PF + SPARE;  // ring slots
+  constexpr int ES = (int)sizeof(T), SX = L::SX, PB = L::PB, SB = L::SB;
+  constexpr int CEN = (2 * SX + 2) * 2 * ES;  // own pair, from the corner of its 5 x 5 patch
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const uint32_t sbase = smem_u32(smem_raw);
+
+  const GridGeom& g = c.g;
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
+  const int i = g.lo[0] + blockIdx.x * TX + tx;
+  const int j = g.lo[1] + blockIdx.y * TY + ty;
+  const int k0 = g.lo[2] + blockIdx.z * kchunk;
+  const int k1 = min(k0 + kchunk, g.hi[2]);
+  const bool active = (i < g.hi[0]) && (j < g.hi[1]);
+  // lanes of this warp that compute points: the fences between the field
+  // groups below are executed by these lanes only (a tile that overhangs
+  // the grid has idle lanes, which must not be named in the mask)
+  const unsigned amask = __ballot_sync(0xffffffffu, active);
+  const uint32_t sz = (uint32_t)g.sz;
+  const uint32_t own = (uint32_t)j * (uint32_t)g.sy + (uint32_t)i;
+  const ColumnCtx<T> col = make_column<XA>(c, i, j);
+  const L loader(g, sbase, tid, g.lo[0] + (int)blockIdx.x * TX - 2,
+                 g.lo[1] + (int)blockIdx.y * TY - 2);
+  const int kend = k1 + 2;  // planes [k0-2, k1+2) are read
+  auto issue = [&](int kp, uint32_t slot) {
+    if (kp < kend) loader.copy(uin, (uint32_t)kp * sz, slot);
+    cp_async_commit();
+  };
+  // plane k0 - 2 + q goes to slot q; the first wait needs planes up to k0 + 2
+#pragma unroll 1
+  for (int p = 0; p < 5 + PF; ++p) issue(k0 - 2 + p, (uint32_t)(p * SB));
+
+  const T six = c.inv_delta[0] / (T)12, siy = c.inv_delta[1] / (T)12,
+          siz = c.inv_delta[2] / (T)12;
+  const T ix = c.inv_delta[0], iy = c.inv_delta[1], iz = c.inv_delta[2];
+  const uint32_t pcorner = sbase + (uint32_t)((ty * SX + tx) * 2 * ES);
+  const uint32_t scorner = sbase + (uint32_t)(3 * PB + (ty * SX + tx) * ES);
+  uint32_t head = 0;  // slot of plane k - 2
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) {
+    cp_async_wait<PF>();  // planes up to k+2 have landed
+    __syncthreads();
+    auto slot = [&](int q) -> uint32_t {  // of plane k - 2 + q
+      const uint32_t s = head + (uint32_t)(q * SB);
+      return s >= (uint32_t)(R * SB) ? s - (uint32_t)(R * SB) : s;
+    };
+    if constexpr (SPARE == 1) issue(k + 3 + PF, slot(5 + PF));  // into the slot of plane k-3
+    if (active) {
+      const uint32_t o = (uint32_t)k * sz + own;
+      Pair<T> dold[3];
+      T doldP = 0;
+      if constexpr (!FIRST) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) dold[a] = pk(du.p[a][o], du.p[3 + a][o]);
+        doldP = du.p[6][o];
+      }
+      const uint32_t zs[5] = {slot(0), slot(1), slot(2), slot(3), slot(4)};
+      const uint32_t a0 = pcorner + zs[2], s0 = scorner + zs[2];
+      // The stencil is consumed component by component, then P; the
+      // warp-level fence between groups keeps the shared loads of the next
+      // group from being hoisted, which bounds the live registers.  d[a]: the
+      // derivatives along axis a of (E_x, B_x), ..., unscaled (the quotients of
+      // diff1_4) in the reference arithmetic, which scales and combines them
+      // as rk_step does (field_solver_EZ.cpp:143-150: the first product of a
+      // curl rounded, the second fused), inv_delta-scaled otherwise.
+      Guard<T> gd;
+      gd.large = !c.tau_mid;
+      auto derivatives = [&](auto ac, Pair<T> d[3]) {
+        constexpr int O = decltype(ac)::value * PB, P2 = 2 * ES;
+        d[0] = pd1_4<XA>(ldsp<T, O + CEN - 2 * P2>(a0), ldsp<T, O + CEN - P2>(a0),
+                         ldsp<T, O + CEN + P2>(a0), ldsp<T, O + CEN + 2 * P2>(a0), six, gd);
+        d[1] = pd1_4<XA>(ldsp<T, O + 2 * P2>(a0), ldsp<T, O + (SX + 2) * P2>(a0),
+                         ldsp<T, O + (3 * SX + 2) * P2>(a0), ldsp<T, O + (4 * SX + 2) * P2>(a0),
+                         siy, gd);
+        d[2] = pd1_4<XA>(ldsp<T, O + CEN>(pcorner + zs[0]), ldsp<T, O + CEN>(pcorner + zs[1]),
+                         ldsp<T, O + CEN>(pcorner + zs[3]), ldsp<T, O + CEN>(pcorner + zs[4]),
+                         siz, gd);
+      };
+      Pair<T> rot[3], dvg;
+      T gradP[3];
+      {
+        Pair<T> xd[3], yd[3], zd[3];
+        derivatives(std::integral_constant<int, 0>{}, xd);
+        __syncwarp(amask);
+        derivatives(std::integral_constant<int, 1>{}, yd);
+        __syncwarp(amask);
+        derivatives(std::integral_constant<int, 2>{}, zd);
+        if constexpr (XA) {
+          rot[0] = pfma(both(-iz), yd[2], pmul(both(iy), zd[1]));
+          rot[1] = pfma(both(-ix), zd[0], pmul(both(iz), xd[2]));
+          rot[2] = pfma(both(-iy), xd[1], pmul(both(ix), yd[0]));
+          dvg = pfma(both(iz), zd[2], pfma(both(iy), yd[1], pmul(both(ix), xd[0])));
+        } else {
+          rot[0] = psub(zd[1], yd[2]);
+          rot[1] = psub(xd[2], zd[0]);
+          rot[2] = psub(yd[0], xd[1]);
+          dvg = padd(padd(xd[0], yd[1]), zd[2]);
+        }
+      }
+      __syncwarp(amask);
+      constexpr int CE1 = CEN / 2;  // own P, from the corner of its patch
+      gradP[0] = sd1_4<XA>(lds<T, CE1 - 2 * ES>(s0), lds<T, CE1 - ES>(s0), lds<T, CE1 + ES>(s0),
+                           lds<T, CE1 + 2 * ES>(s0), six, gd);
+      gradP[1] = sd1_4<XA>(lds<T, 2 * ES>(s0), lds<T, (SX + 2) * ES>(s0),
+                           lds<T, (3 * SX + 2) * ES>(s0), lds<T, (4 * SX + 2) * ES>(s0), siy, gd);
+      gradP[2] = sd1_4<XA>(lds<T, CE1>(scorner + zs[0]), lds<T, CE1>(scorner + zs[1]),
+                           lds<T, CE1>(scorner + zs[3]), lds<T, CE1>(scorner + zs[4]), siz, gd);
+      if constexpr (XA) {
+        gradP[0] = xa::mul(ix, gradP[0]);
+        gradP[1] = xa::mul(iy, gradP[1]);
+        gradP[2] = xa::mul(iz, gradP[2]);
+      }
+      Pair<T> eb[3] = {ldsp<T, CEN>(a0), ldsp<T, PB + CEN>(a0), ldsp<T, 2 * PB + CEN>(a0)};
+      const T P = lds<T, CE1>(s0);
+      if constexpr (DG) {
+        const T u[7] = {first(eb[0]),  first(eb[1]),  first(eb[2]), second(eb[0]),
+                        second(eb[1]), second(eb[2]), P};
+        Derivs<T> dv;
+        T old[7];
+        StageValues<T> r;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          dv.rotE[a] = first(rot[a]);
+          dv.rotB[a] = second(rot[a]);
+          dv.gradP[a] = gradP[a];
+          old[a] = first(dold[a]);
+          old[3 + a] = second(dold[a]);
+        }
+        dv.divE = first(dvg);
+        dv.divB = second(dvg);
+        old[6] = doldP;
+        if (gd.bad()) dv = point_derivatives_ieee(c, uin, o);
+        stage_values_ieee<FIRST, true>(c, u, dv, old, As, Bs, col, k, dg, o, r);
+        stage_finish<BC>(c, u, r.d, r.nu, r.J, r.divE, r.divB, tst, flags, col, k, o, du, un, aux,
+                         uout);
+      } else {
+        Pair<T> dn[3], nu[3];
+        T dP, nuP, J[3];
+        stage_values_pair<FIRST, XA>(c, eb, P, rot, dvg, gradP, dold, doldP, As, Bs, col, k, dn,
+                                     dP, nu, nuP, J, gd);
+        T divE = first(dvg), divB = second(dvg);
+        if (XA && gd.bad()) {
+          const StageValues<T> r = stage_point_ieee<FIRST>(c, uin, du, col, k, o, As, Bs);
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            dn[a] = pk(r.d[a], r.d[3 + a]);
+            nu[a] = pk(r.nu[a], r.nu[3 + a]);
+            J[a] = r.J[a];
+          }
+          dP = r.d[6];
+          nuP = r.nu[6];
+          divE = r.divE;
+          divB = r.divB;
+        }
+        const T u[7] = {first(eb[0]),  first(eb[1]),  first(eb[2]), second(eb[0]),
+                        second(eb[1]), second(eb[2]), P};
+        const T d7[7] = {first(dn[0]),  first(dn[1]),  first(dn[2]), second(dn[0]),
+                         second(dn[1]), second(dn[2]), dP};
+        T n7[7] = {first(nu[0]),  first(nu[1]),  first(nu[2]), second(nu[0]),
+                   second(nu[1]), second(nu[2]), nuP};
+        stage_finish<BC>(c, u, d7, n7, J, divE, divB, tst, flags, col, k, o, du, un, aux, uout);
+      }
+    }
+    if constexpr (SPARE == 0) {
+      __syncthreads();
+      issue(k + 3 + PF, slot(5 + PF));  // into the slot of plane k-2
+    }
+    head = slot(1);
+  }
+  cp_async_wait<0>();
+}
+
+// ---------------------------------------------------------------------------
+// The same stage in FP32 with the z neighbours in a register window: planes k-2 ..
+// k+2 of a thread's column travel through 35 registers (the z loop unrolled by ZU = 5,
+// which renames instead of moving them; ZU = 1 with the boundary code, whose five
+// copies would spill), each plane read from the ring once, as the leading one, so a field costs 9
+// shared loads instead of 13; rows of even length are copied by aligned pairs.
+// With 128 registers 16 warps share an SM.  Bound by dependency latency and the
+// shared-memory queue (issue 52%, 613 instructions a point).  Stage at 512^3: 4526 us
+// with one field per instruction and IEEE divisions, 4313 us here; with the ring
+// kernel above instead (24 warps, but 13 shared loads per field and 4-byte copies)
+// 5.0 ms, with two rows per thread (8 warps, 251 registers) 6.4 ms.
+// ---------------------------------------------------------------------------
+template <int PF>
+__host__ __device__ constexpr int window_ring() {
+  return 4 + PF;  // planes k .. k+2, the prefetch, a spare slot
+}
+template <typename T, int TX, int TY, int PF, int V>
+constexpr size_t window_smem_bytes(bool first) {
+  return (size_t)window_ring<PF>() * 7 * TileLoader<T, TX, TY, 2, V>::FB +
+         (first ? 0 : (size_t)(PF + 2) * 7 * TX * TY * sizeof(T));
+}
+
+template <typename T, int TX, int TY, int PF, int ZU, bool FIRST, bool BC, int V, bool XA, bool DG>
+__global__ void __launch_bounds__(TX * TY, min_blocks<T, TX * TY>())
+    ez_stage_window_kernel(const __grid_constant__ EzConst<T> c, const F7<const T> uin,
+                    const F7<T> uout, const F7<T> du, const F7<T> un, const F5<T> aux, const F6<T> dg,
+                    const T As, const T Bs, const T tst, const int kchunk,
+                    const int flags) {
   using L = TileLoader<T, TX, TY, 2, V>;
-  constexpr int R = stage_ring<BC, PF>();    // field ring slots
-  constexpr int DR = stage_dring<BC, PF>();  // dU ring slots
-  constexpr int ZU = stage_zunroll<BC>();
+  constexpr int R = window_ring<PF>();    // field ring slots
+  constexpr int DR = PF + 2;              // dU ring slots
 
   constexpr int ES = (int)sizeof(T);
   constexpr int SX = L::SX, FB = L::FB, SB = 7 * FB;
@@ -471,17 +868,21 @@ __global__ void __launch_bounds__(TX * TY, min_blocks<T, TX * TY>())
           siz = c.inv_delta[2] / (T)12;
   const T ix = c.inv_delta[0], iy = c.inv_delta[1], iz = c.inv_delta[2];
   const uint32_t corner = sbase + (uint32_t)((ty * SX + tx + loader.xoff) * ES);
-  // Register window: in window phase S, w[(S + q) % 5][f] = field f at
-  // (i, j, k - 2 + q).  Planes k-2 .. k+1 are carried from the previous
-  // plane and k+2 is read from the ring into the slot of the dead plane k-3,
-  // so advancing the window moves no registers when the z loop is unrolled
-  // by the window length (ZU = 5).
-  T w[5][7];
+  // Register window: in window phase S, w[(S + q) % 5][a] = (E_a, B_a) and
+  // wp[(S + q) % 5] = P at (i, j, k - 2 + q).  Planes k-2 .. k+1 are carried
+  // from the previous plane and k+2 is read from the ring into the slot of the
+  // dead plane k-3, so advancing the window moves no registers when the z loop
+  // is unrolled by the window length (ZU = 5).
+  Pair<T> w[5][3];
+  T wp[5];
   if (active) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t e = (uint32_t)(k0 - 2 + q) * sz + own;
 #pragma unroll
-      for (int f = 0; f < 7; ++f) w[q][f] = uin.p[f][(uint32_t)(k0 - 2 + q) * sz + own];
+      for (int a = 0; a < 3; ++a) w[q][a] = pk(uin.p[a][e], uin.p[3 + a][e]);
+      wp[q] = uin.p[6][e];
+    }
   }
 
   auto plane = [&](auto sc, const int k) {
@@ -492,112 +893,147 @@ __global__ void __launch_bounds__(TX * TY, min_blocks<T, TX * TY>())
     using P2 = std::integral_constant<int, 2>;
     using PN = std::integral_constant<int, 3 + PF>;   // the plane issued now
     using PD = std::integral_constant<int, 1 + PF>;   // and its dU plane
-    if constexpr (kRingSpare == 1)  // into the slot of plane k-1
-      issue(k + 3 + PF, fslot(sc, PN{}, k), dslot(sc, PD{}, k));
+    issue(  // into the slot of plane k-1
+        k + 3 + PF, fslot(sc, PN{}, k), dslot(sc, PD{}, k));
     if (active && k < k1) {
       const uint32_t a0 = corner + fslot(sc, Z{}, k);
       const uint32_t ap2 = corner + fslot(sc, P2{}, k);
-      // The stencil is consumed field group by field group (B, then E, then
-      // P); the warp-level fence between groups keeps the shared loads of the
-      // next group from being hoisted, which bounds the live registers.
-      T u[7], dold[7];
-      Derivs<T> dv;
-      // dxyz[a]: the derivative of field f along axis a, inv_delta-scaled;
-      // in the reference arithmetic (XA) the unscaled quotient of diff1_4,
-      // which curl_div scales and combines as the CPU build does.  EX
-      // selects the exact division for the rare quotients the fast one
-      // flags through the key minimum `kmin` (xa::div12_fast).
-      uint32_t kmin = 0xFFFFFFFFu;
-      auto d1 = [&](auto fc, auto ex, T* dxyz) {
-        constexpr int f = decltype(fc)::value;
-        constexpr bool EX = decltype(ex)::value;
-        constexpr int o = f * FB;
-        if constexpr (XA) {
-          dxyz[0] = xa::dq<EX>(lds<T, o + CEN - 2 * ES>(a0), lds<T, o + CEN - ES>(a0),
-                               lds<T, o + CEN + ES>(a0), lds<T, o + CEN + 2 * ES>(a0), kmin);
-          dxyz[1] = xa::dq<EX>(lds<T, o + 2 * ES>(a0), lds<T, o + (SX + 2) * ES>(a0),
-                               lds<T, o + (3 * SX + 2) * ES>(a0),
-                               lds<T, o + (4 * SX + 2) * ES>(a0), kmin);
-        } else {
-          dxyz[0] = d1_4(lds<T, o + CEN - 2 * ES>(a0), lds<T, o + CEN - ES>(a0),
-                         lds<T, o + CEN + ES>(a0), lds<T, o + CEN + 2 * ES>(a0), six);
-          dxyz[1] = d1_4(lds<T, o + 2 * ES>(a0), lds<T, o + (SX + 2) * ES>(a0),
-                         lds<T, o + (3 * SX + 2) * ES>(a0), lds<T, o + (4 * SX + 2) * ES>(a0), siy);
-        }
-        w[(S + 4) % 5][f] = lds<T, o + CEN>(ap2);
-        u[f] = w[(S + 2) % 5][f];
-        if constexpr (XA)
-          dxyz[2] = xa::dq<EX>(w[S % 5][f], w[(S + 1) % 5][f], w[(S + 3) % 5][f],
-                               w[(S + 4) % 5][f], kmin);
-        else
-          dxyz[2] = d1_4(w[S % 5][f], w[(S + 1) % 5][f], w[(S + 3) % 5][f], w[(S + 4) % 5][f],
-                         siz);
+      constexpr int W0 = S % 5, W1 = (S + 1) % 5, W2 = (S + 2) % 5, W3 = (S + 3) % 5,
+                    W4 = (S + 4) % 5;
+      // The stencil is consumed component by component, then P; the
+      // warp-level fence between groups keeps the shared loads of the next
+      // group from being hoisted, which bounds the live registers.  d[a]: the
+      // derivatives along axis a of (E_x, B_x), ..., unscaled (the quotients of
+      // diff1_4) in the reference arithmetic, which scales and combines them
+      // as rk_step does (field_solver_EZ.cpp:143-150: the first product of a
+      // curl rounded, the second fused), inv_delta-scaled otherwise.
+      Guard<T> g;
+      g.large = !c.tau_mid;
+      auto derivatives = [&](auto ac, Pair<T> d[3]) {
+        constexpr int a = decltype(ac)::value;
+        auto at = [&](auto oc) {
+          constexpr int off = decltype(oc)::value;
+          return pk(lds<T, a * FB + off>(a0), lds<T, (3 + a) * FB + off>(a0));
+        };
+        using std::integral_constant;
+        d[0] = pd1_4<XA>(at(integral_constant<int, CEN - 2 * ES>{}),
+                         at(integral_constant<int, CEN - ES>{}),
+                         at(integral_constant<int, CEN + ES>{}),
+                         at(integral_constant<int, CEN + 2 * ES>{}), six, g);
+        d[1] = pd1_4<XA>(at(integral_constant<int, 2 * ES>{}),
+                         at(integral_constant<int, (SX + 2) * ES>{}),
+                         at(integral_constant<int, (3 * SX + 2) * ES>{}),
+                         at(integral_constant<int, (4 * SX + 2) * ES>{}), siy, g);
+        w[W4][a] = pk(lds<T, a * FB + CEN>(ap2), lds<T, (3 + a) * FB + CEN>(ap2));
+        d[2] = pd1_4<XA>(w[W0][a], w[W1][a], w[W3][a], w[W4][a], siz, g);
       };
-      // curl and divergence of one vector field from its derivatives; in the
-      // reference arithmetic the curl's first product is rounded and its
-      // second fused (rk_step, field_solver_EZ.cpp:143-150)
-      auto curl_div = [&](const T* xd, const T* yd, const T* zd, T* rot, T& dvg) {
-        if constexpr (XA) {
-          rot[0] = xa::fma(-iz, yd[2], xa::mul(iy, zd[1]));
-          rot[1] = xa::fma(-ix, zd[0], xa::mul(iz, xd[2]));
-          rot[2] = xa::fma(-iy, xd[1], xa::mul(ix, yd[0]));
-          dvg = xa::fma(iz, zd[2], xa::fma(iy, yd[1], xa::mul(ix, xd[0])));
-        } else {
-          rot[0] = zd[1] - yd[2];
-          rot[1] = xd[2] - zd[0];
-          rot[2] = yd[0] - xd[1];
-          dvg = xd[0] + yd[1] + zd[2];
-        }
-      };
-      auto derivatives = [&](auto ex) {
-        {
-          T bxd[3], byd[3], bzd[3];
-          d1(std::integral_constant<int, 3>{}, ex, bxd);
-          d1(std::integral_constant<int, 4>{}, ex, byd);
-          d1(std::integral_constant<int, 5>{}, ex, bzd);
-          curl_div(bxd, byd, bzd, dv.rotB, dv.divB);
-        }
+      Pair<T> rot[3], dvg;
+      T gradP[3];
+      {
+        Pair<T> xd[3], yd[3], zd[3];
+        derivatives(std::integral_constant<int, 0>{}, xd);
         __syncwarp(amask);
-        {
-          T exd[3], eyd[3], ezd[3];
-          d1(std::integral_constant<int, 0>{}, ex, exd);
-          d1(std::integral_constant<int, 1>{}, ex, eyd);
-          d1(std::integral_constant<int, 2>{}, ex, ezd);
-          curl_div(exd, eyd, ezd, dv.rotE, dv.divE);
-        }
+        derivatives(std::integral_constant<int, 1>{}, yd);
         __syncwarp(amask);
-        d1(std::integral_constant<int, 6>{}, ex, dv.gradP);
-      };
-      derivatives(std::false_type{});
-      // a quotient in the subnormal range (|t| < 2^-124, t != 0): the whole
-      // warp recomputes its derivatives with the exact division (the same
-      // operands are still in shared memory and the window)
-      if constexpr (XA)
-        if (__any_sync(amask, kmin < xa::kTinyKey)) derivatives(std::true_type{});
-      if constexpr (XA) {
-        dv.gradP[0] = xa::mul(ix, dv.gradP[0]);
-        dv.gradP[1] = xa::mul(iy, dv.gradP[1]);
-        dv.gradP[2] = xa::mul(iz, dv.gradP[2]);
+        derivatives(std::integral_constant<int, 2>{}, zd);
+        if constexpr (XA) {
+          rot[0] = pfma(both(-iz), yd[2], pmul(both(iy), zd[1]));
+          rot[1] = pfma(both(-ix), zd[0], pmul(both(iz), xd[2]));
+          rot[2] = pfma(both(-iy), xd[1], pmul(both(ix), yd[0]));
+          dvg = pfma(both(iz), zd[2], pfma(both(iy), yd[1], pmul(both(ix), xd[0])));
+        } else {
+          rot[0] = psub(zd[1], yd[2]);
+          rot[1] = psub(xd[2], zd[0]);
+          rot[2] = psub(yd[0], xd[1]);
+          dvg = padd(padd(xd[0], yd[1]), zd[2]);
+        }
       }
+      __syncwarp(amask);
+      {
+        constexpr int o6 = 6 * FB;
+        gradP[0] = sd1_4<XA>(lds<T, o6 + CEN - 2 * ES>(a0), lds<T, o6 + CEN - ES>(a0),
+                             lds<T, o6 + CEN + ES>(a0), lds<T, o6 + CEN + 2 * ES>(a0), six, g);
+        gradP[1] = sd1_4<XA>(lds<T, o6 + 2 * ES>(a0), lds<T, o6 + (SX + 2) * ES>(a0),
+                             lds<T, o6 + (3 * SX + 2) * ES>(a0),
+                             lds<T, o6 + (4 * SX + 2) * ES>(a0), siy, g);
+        wp[W4] = lds<T, o6 + CEN>(ap2);
+        gradP[2] = sd1_4<XA>(wp[W0], wp[W1], wp[W3], wp[W4], siz, g);
+        if constexpr (XA) {
+          gradP[0] = xa::mul(ix, gradP[0]);
+          gradP[1] = xa::mul(iy, gradP[1]);
+          gradP[2] = xa::mul(iz, gradP[2]);
+        }
+      }
+      Pair<T> dold[3];
+      T doldP = 0;
       if constexpr (!FIRST) {
         const uint32_t ad = dme + dslot(sc, Z{}, k);
-        static_for<7>([&](auto fc) {
-          constexpr int f = decltype(fc)::value;
-          dold[f] = lds<T, f * DFB>(ad);
+        static_for<3>([&](auto ac) {
+          constexpr int a = decltype(ac)::value;
+          dold[a] = pk(lds<T, a * DFB>(ad), lds<T, (3 + a) * DFB>(ad));
         });
+        doldP = lds<T, 6 * DFB>(ad);
       }
-      stage_point<T, FIRST, BC, XA, DG>(c, u, dv, dold, As, Bs, tst, flags, col, k,
-                                        (uint32_t)k * sz + own, du, un, aux, uout, dg);
+      const uint32_t o = (uint32_t)k * sz + own;
+      const Pair<T>* eb = w[W2];
+      const T u[7] = {first(eb[0]),  first(eb[1]),  first(eb[2]), second(eb[0]),
+                      second(eb[1]), second(eb[2]), wp[W2]};
+      if constexpr (DG) {
+        Derivs<T> dv;
+        T old[7];
+        StageValues<T> r;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          dv.rotE[a] = first(rot[a]);
+          dv.rotB[a] = second(rot[a]);
+          dv.gradP[a] = gradP[a];
+          old[a] = first(dold[a]);
+          old[3 + a] = second(dold[a]);
+        }
+        dv.divE = first(dvg);
+        dv.divB = second(dvg);
+        old[6] = doldP;
+        if (g.bad()) dv = point_derivatives_ieee(c, uin, o);
+        stage_values_ieee<FIRST, true>(c, u, dv, old, As, Bs, col, k, dg, o, r);
+        stage_finish<BC>(c, u, r.d, r.nu, r.J, r.divE, r.divB, tst, flags, col, k, o, du, un, aux,
+                         uout);
+      } else {
+        Pair<T> dn[3], nu[3];
+        T dP, nuP, J[3];
+        stage_values_pair<FIRST, XA>(c, eb, u[6], rot, dvg, gradP, dold, doldP, As, Bs, col, k, dn,
+                                     dP, nu, nuP, J, g);
+        T d7[7], n7[7], divE = first(dvg), divB = second(dvg);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          d7[a] = first(dn[a]);
+          d7[3 + a] = second(dn[a]);
+          n7[a] = first(nu[a]);
+          n7[3 + a] = second(nu[a]);
+        }
+        d7[6] = dP;
+        n7[6] = nuP;
+        if (XA && g.bad()) {
+          const StageValues<T> r = stage_point_ieee<FIRST>(c, uin, du, col, k, o, As, Bs);
+#pragma unroll
+          for (int f = 0; f < 7; ++f) {
+            d7[f] = r.d[f];
+            n7[f] = r.nu[f];
+          }
+#pragma unroll
+          for (int a = 0; a < 3; ++a) J[a] = r.J[a];
+          divE = r.divE;
+          divB = r.divB;
+        }
+        stage_finish<BC>(c, u, d7, n7, J, divE, divB, tst, flags, col, k, o, du, un, aux, uout);
+      }
       if constexpr (ZU == 1) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < 4; ++q) {
 #pragma unroll
-          for (int f = 0; f < 7; ++f) w[q][f] = w[q + 1][f];
+          for (int a = 0; a < 3; ++a) w[q][a] = w[q + 1][a];
+          wp[q] = wp[q + 1];
+        }
       }
-    }
-    if constexpr (kRingSpare == 0) {
-      __syncthreads();
-      issue(k + 3 + PF, fslot(sc, PN{}, k), dslot(sc, PD{}, k));  // into the slot of plane k
     }
   };
   if constexpr (ZU == 5) {
@@ -629,6 +1065,16 @@ __global__ void __launch_bounds__(TX * TY, min_blocks<T, TX * TY>())
 // planes k-3..k+3 per thread; shared memory keeps plane k (x/y neighbours)
 // and the arriving planes k+1..k+3+PF.
 // ---------------------------------------------------------------------------
+// Spare ring slots (0 or 1) of the KO kernel.  With a spare slot the copies of
+// a new plane are issued right after the one barrier at the top of an
+// iteration; without it they wait for a second barrier after the iteration's
+// arithmetic.  Measured at 512^3: faster without (two CTAs per SM).
+#ifndef COFFEE_KO_RING_SPARE
+#define COFFEE_KO_RING_SPARE 0
+#endif
+constexpr int kKoRingSpare = COFFEE_KO_RING_SPARE;
+static_assert(kKoRingSpare == 0 || kKoRingSpare == 1, "0 or 1 spare ring slot");
+
 // z-loop unroll of the KO kernel: 7 (the window length, no register moves)
 // or 1 (one plane per iteration, window shifted by moves), per instance
 // (with and without the boundary code); both are faster unrolled.
@@ -702,16 +1148,20 @@ __global__ void __launch_bounds__(TX * TY, min_blocks<T, TX * TY>())
 #pragma unroll 1
   for (int p = 0; p < 4 + PF; ++p) issue(k0 + p, (uint32_t)(((k0 + p - lo2) % R) * SB));
 
-  // Register window: in window phase S, w[(S + q) % 7][f] = field f at
-  // (i, j, k - 3 + q); planes k-3 .. k+2 are carried, k+3 is read from the
-  // ring into the slot of the dead plane k-4 (no register moves when the z
-  // loop is unrolled by the window length, ZU = 7).
-  T w[7][7];
+  // Register window: in window phase S, w[(S + q) % 7][a] = (E_a, B_a) and
+  // wp[(S + q) % 7] = P at (i, j, k - 3 + q); planes k-3 .. k+2 are carried,
+  // k+3 is read from the ring into the slot of the dead plane k-4 (no register
+  // moves when the z loop is unrolled by the window length, ZU = 7).
+  Pair<T> w[7][3];
+  T wp[7];
   if (active) {
 #pragma unroll
-    for (int f = 0; f < 7; ++f)
+    for (int q = 0; q < 6; ++q) {
+      const uint32_t e = (uint32_t)(k0 - 3 + q) * sz + own;
 #pragma unroll
-      for (int q = 0; q < 6; ++q) w[q][f] = uin.p[f][(uint32_t)(k0 - 3 + q) * sz + own];
+      for (int a = 0; a < 3; ++a) w[q][a] = pk(uin.p[a][e], uin.p[3 + a][e]);
+      wp[q] = uin.p[6][e];
+    }
   }
   const bool ko_p = (c.semantics != SEM_CPU_REF);
   const uint32_t corner = sbase + (uint32_t)((ty * SX + tx + loader.xoff) * ES);
@@ -724,59 +1174,75 @@ __global__ void __launch_bounds__(TX * TY, min_blocks<T, TX * TY>())
     if (active && k < k1) {
       const uint32_t a0 = corner + fslot(sc, std::integral_constant<int, 0>{}, k);
       const uint32_t a3 = corner + fslot(sc, std::integral_constant<int, 3>{}, k);
-      T nu[7];
-      static_for<7>([&](auto fc) {
-        constexpr int f = decltype(fc)::value;
-        constexpr int o = f * FB;
-        w[(S + 6) % 7][f] = lds<T, o + CEN>(a3);
-        const T cv = w[(S + 3) % 7][f];
-        if (f < 6 || ko_p) {
-          auto d6 = [](T m3, T m2, T m1, T c0, T p1, T p2, T p3) {
-            if constexpr (XA) return xa::d6(m3, m2, m1, c0, p1, p2, p3);
-            else return d6_2(m3, m2, m1, c0, p1, p2, p3);
-          };
-          const T kx = d6(lds<T, o + CEN - 3 * ES>(a0), lds<T, o + CEN - 2 * ES>(a0),
-                          lds<T, o + CEN - ES>(a0), cv, lds<T, o + CEN + ES>(a0),
-                          lds<T, o + CEN + 2 * ES>(a0), lds<T, o + CEN + 3 * ES>(a0));
-          const T ky = d6(lds<T, o + 3 * ES>(a0), lds<T, o + (SX + 3) * ES>(a0),
-                          lds<T, o + (2 * SX + 3) * ES>(a0), cv,
-                          lds<T, o + (4 * SX + 3) * ES>(a0), lds<T, o + (5 * SX + 3) * ES>(a0),
-                          lds<T, o + (6 * SX + 3) * ES>(a0));
-          const T kz = d6(w[S % 7][f], w[(S + 1) % 7][f], w[(S + 2) % 7][f], cv,
-                          w[(S + 4) % 7][f], w[(S + 5) % 7][f], w[(S + 6) % 7][f]);
-          // the reference arithmetic sums the axes x, y, z left to right and
-          // fuses f + KO (-KOeps KO_const) (field_solver_EZ.cpp:350-420)
-          if constexpr (XA) nu[f] = xa::fma(c.ko_c, xa::add(xa::add(kx, ky), kz), cv);
-          else nu[f] = fma(kx + ky + kz, c.ko_c, cv);
-        } else {
-          nu[f] = cv;
-        }
+      constexpr int C3 = (S + 3) % 7;  // the window slot of plane k
+      Pair<T> nu[3];
+      T nuP = wp[C3];
+      static_for<3>([&](auto ac) {
+        constexpr int a = decltype(ac)::value;
+        using std::integral_constant;
+        auto at = [&](auto oc) {
+          constexpr int off = decltype(oc)::value;
+          return pk(lds<T, a * FB + off>(a0), lds<T, (3 + a) * FB + off>(a0));
+        };
+        w[(S + 6) % 7][a] = pk(lds<T, a * FB + CEN>(a3), lds<T, (3 + a) * FB + CEN>(a3));
+        const Pair<T> cv = w[C3][a];
+        const Pair<T> kx = pd6_2<XA>(at(integral_constant<int, CEN - 3 * ES>{}),
+                                     at(integral_constant<int, CEN - 2 * ES>{}),
+                                     at(integral_constant<int, CEN - ES>{}), cv,
+                                     at(integral_constant<int, CEN + ES>{}),
+                                     at(integral_constant<int, CEN + 2 * ES>{}),
+                                     at(integral_constant<int, CEN + 3 * ES>{}));
+        const Pair<T> ky = pd6_2<XA>(at(integral_constant<int, 3 * ES>{}),
+                                     at(integral_constant<int, (SX + 3) * ES>{}),
+                                     at(integral_constant<int, (2 * SX + 3) * ES>{}), cv,
+                                     at(integral_constant<int, (4 * SX + 3) * ES>{}),
+                                     at(integral_constant<int, (5 * SX + 3) * ES>{}),
+                                     at(integral_constant<int, (6 * SX + 3) * ES>{}));
+        const Pair<T> kz = pd6_2<XA>(w[S % 7][a], w[(S + 1) % 7][a], w[(S + 2) % 7][a], cv,
+                                     w[(S + 4) % 7][a], w[(S + 5) % 7][a], w[(S + 6) % 7][a]);
+        // the reference arithmetic sums the axes x, y, z left to right and
+        // fuses f + KO (-KOeps KO_const) (field_solver_EZ.cpp:350-420)
+        nu[a] = pfma(both(c.ko_c), padd(padd(kx, ky), kz), cv);
       });
+      wp[(S + 6) % 7] = lds<T, 6 * FB + CEN>(a3);
+      if (ko_p) {
+        constexpr int o6 = 6 * FB;
+        const T kx = d6_2(lds<T, o6 + CEN - 3 * ES>(a0), lds<T, o6 + CEN - 2 * ES>(a0),
+                          lds<T, o6 + CEN - ES>(a0), nuP, lds<T, o6 + CEN + ES>(a0),
+                          lds<T, o6 + CEN + 2 * ES>(a0), lds<T, o6 + CEN + 3 * ES>(a0));
+        const T ky = d6_2(lds<T, o6 + 3 * ES>(a0), lds<T, o6 + (SX + 3) * ES>(a0),
+                          lds<T, o6 + (2 * SX + 3) * ES>(a0), nuP,
+                          lds<T, o6 + (4 * SX + 3) * ES>(a0), lds<T, o6 + (5 * SX + 3) * ES>(a0),
+                          lds<T, o6 + (6 * SX + 3) * ES>(a0));
+        const T kz = d6_2(wp[S % 7], wp[(S + 1) % 7], wp[(S + 2) % 7], nuP, wp[(S + 4) % 7],
+                          wp[(S + 5) % 7], wp[(S + 6) % 7]);
+        nuP = sfma(kx + ky + kz, c.ko_c, nuP);
+      }
       const uint32_t o = (uint32_t)k * sz + own;
+      T n7[7] = {first(nu[0]),  first(nu[1]),  first(nu[2]), second(nu[0]),
+                 second(nu[1]), second(nu[2]), nuP};
       if constexpr (DG) {
         // dU_KO = (|B|^2 + |E|^2) after the pass minus before it, and
         // dU_KO_cum += it (field_solver_EZ.cpp:398-455)
-        constexpr int C3 = (S + 3) % 7;  // the window slot of plane k
-        const T u0 = xa::add(xa::dot3(w[C3][3], w[C3][3], w[C3][4], w[C3][4], w[C3][5], w[C3][5]),
-                             xa::dot3(w[C3][0], w[C3][0], w[C3][1], w[C3][1], w[C3][2], w[C3][2]));
-        const T u1 = xa::add(xa::dot3(nu[3], nu[3], nu[4], nu[4], nu[5], nu[5]),
-                             xa::dot3(nu[0], nu[0], nu[1], nu[1], nu[2], nu[2]));
-        const T dko = xa::sub(u1, u0);
+        const Pair<T> s0 = pdot3(w[C3], w[C3]), s1 = pdot3(nu, nu);
+        const T dko = xa::sub(xa::add(second(s1), first(s1)), xa::add(second(s0), first(s0)));
         dg.p[5][o] = xa::add(dko, dg.p[5][o]);
         dg.p[2][o] = dko;
-        apply_clamps_xa_dg<false>(nu[0], nu[1], nu[2], nu[3], nu[4], nu[5], dg, o);
+        apply_clamps_xa_dg<false>(n7[0], n7[1], n7[2], n7[3], n7[4], n7[5], dg, o);
       } else if constexpr (XA) {
-        apply_clamps_xa(nu[0], nu[1], nu[2], nu[3], nu[4], nu[5]);
+        apply_clamps_mid(n7);
       } else {
-        apply_clamps(c, nu[0], nu[1], nu[2], nu[3], nu[4], nu[5]);
+        apply_clamps(c, n7[0], n7[1], n7[2], n7[3], n7[4], n7[5]);
       }
-      if constexpr (BC) star_boundary(c, i, j, k, tko, nu);
-      store_with_images(g, col, uout, k, o, nu);
+      if constexpr (BC) star_boundary(c, i, j, k, tko, n7);
+      store_with_images(g, col, uout, k, o, n7);
       if constexpr (ZU == 1) {
 #pragma unroll
-        for (int q = 0; q < 6; ++q)
+        for (int q = 0; q < 6; ++q) {
 #pragma unroll
-          for (int f = 0; f < 7; ++f) w[q][f] = w[q + 1][f];
+          for (int a = 0; a < 3; ++a) w[q][a] = w[q + 1][a];
+          wp[q] = wp[q + 1];
+        }
       }
     }
     if constexpr (kKoRingSpare == 0) {
@@ -802,6 +1268,162 @@ __global__ void __launch_bounds__(TX * TY, min_blocks<T, TX * TY>())
     for (int k = k0; k < k1; ++k) plane(std::integral_constant<int, 0>{}, k);
   }
   cp_async_wait<0>();
+}
+
+// ---------------------------------------------------------------------------
+// The stage and the KO pass with one point per thread, straight from global memory.
+// A small grid fills the GPU with neither tiles nor planes (at 32^3 the streaming
+// kernels run 14 CTAs, each waiting for one plane after the other), and up to some
+// 200^3 points the stencil's 13 planes of 7 fields stay in L2 and L1, so that loads
+// without tiles, barriers or a window cost less than they save: 80 registers, 24
+// warps per SM, neighbours in z within a block (32 x 4 x 2 threads).  The arithmetic
+// is the streaming kernels' (bit for bit in the reference arithmetic).  Stage of one
+// point per thread against the streaming one, us: 32^3 13 / 19, 128^3 87 / 94, 192^3
+// 258 / 283, 256^3 591 / 570, 512^3 5128 / 4313; with the star 192^3 298 / 426, 384^3
+// 2264 / 2370.  What bounds it is the latency of the loads (FP32) and, from 256^3 on,
+// L2 misses.
+// ---------------------------------------------------------------------------
+#ifndef COFFEE_DIRECT_Y
+#define COFFEE_DIRECT_Y 4
+#endif
+#ifndef COFFEE_DIRECT_Z
+#define COFFEE_DIRECT_Z 2
+#endif
+#ifndef COFFEE_DIRECT_MINB
+#define COFFEE_DIRECT_MINB 3
+#endif
+constexpr int kDirectX = 32, kDirectY = COFFEE_DIRECT_Y;
+template <typename T>
+__host__ __device__ constexpr int direct_z() {
+  return sizeof(T) == 4 ? COFFEE_DIRECT_Z : 1;
+}
+
+template <typename T, bool FIRST, bool BC, bool XA>
+__global__ void __launch_bounds__(kDirectX * kDirectY * direct_z<T>(),
+                                  sizeof(T) == 4 ? COFFEE_DIRECT_MINB : 2)
+    ez_stage_direct_kernel(const __grid_constant__ EzConst<T> c, const F7<const T> uin,
+                           const F7<T> uout, const F7<T> du, const F7<T> un, const F5<T> aux,
+                           const T As, const T Bs, const T tst, const int flags, const int j0,
+                           const int k0) {
+  const GridGeom& g = c.g;
+  const int i = g.lo[0] + blockIdx.x * kDirectX + threadIdx.x;
+  const int j = j0 + blockIdx.y * kDirectY + threadIdx.y;
+  const int k = k0 + blockIdx.z * direct_z<T>() + threadIdx.z;
+  if (i >= g.hi[0] || j >= g.hi[1] || k >= g.hi[2]) return;
+  const uint32_t sy = (uint32_t)g.sy, sz = (uint32_t)g.sz;
+  const uint32_t o = (uint32_t)k * sz + (uint32_t)j * sy + (uint32_t)i;
+  const ColumnCtx<T> col = make_column<XA>(c, i, j);
+  Pair<T> dold[3];
+  T doldP = 0;
+  if constexpr (!FIRST) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) dold[a] = pk(du.p[a][o], du.p[3 + a][o]);
+    doldP = du.p[6][o];
+  }
+  const T ix = c.inv_delta[0], iy = c.inv_delta[1], iz = c.inv_delta[2];
+  const uint32_t st[3] = {1u, sy, sz};
+  Guard<T> gd;
+  gd.large = !c.tau_mid;
+  Pair<T> d[3][3];  // d[a][x]: component a along axis x
+  T dp[3];
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    const T f12 = c.inv_delta[x] / (T)12;
+    const uint32_t q[4] = {o - 2 * st[x], o - st[x], o + st[x], o + 2 * st[x]};
+    T p[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) p[n] = __ldg(uin.p[6] + q[n]);
+    dp[x] = sd1_4<XA>(p[0], p[1], p[2], p[3], f12, gd);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      Pair<T> v[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) v[n] = pk(__ldg(uin.p[a] + q[n]), __ldg(uin.p[3 + a] + q[n]));
+      d[a][x] = pd1_4<XA>(v[0], v[1], v[2], v[3], f12, gd);
+    }
+  }
+  Pair<T> rot[3], dvg;
+  if constexpr (XA) {
+    rot[0] = pfma(both(-iz), d[1][2], pmul(both(iy), d[2][1]));
+    rot[1] = pfma(both(-ix), d[2][0], pmul(both(iz), d[0][2]));
+    rot[2] = pfma(both(-iy), d[0][1], pmul(both(ix), d[1][0]));
+    dvg = pfma(both(iz), d[2][2], pfma(both(iy), d[1][1], pmul(both(ix), d[0][0])));
+    dp[0] = xa::mul(ix, dp[0]);
+    dp[1] = xa::mul(iy, dp[1]);
+    dp[2] = xa::mul(iz, dp[2]);
+  } else {
+    rot[0] = psub(d[2][1], d[1][2]);
+    rot[1] = psub(d[0][2], d[2][0]);
+    rot[2] = psub(d[1][0], d[0][1]);
+    dvg = padd(padd(d[0][0], d[1][1]), d[2][2]);
+  }
+  Pair<T> eb[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) eb[a] = pk(__ldg(uin.p[a] + o), __ldg(uin.p[3 + a] + o));
+  const T P = __ldg(uin.p[6] + o);
+  StageValues<T> r;
+  {
+    Pair<T> dn[3], nu[3];
+    stage_values_pair<FIRST, XA>(c, eb, P, rot, dvg, dp, dold, doldP, As, Bs, col, k, dn, r.d[6],
+                                 nu, r.nu[6], r.J, gd);
+    r.divE = first(dvg);
+    r.divB = second(dvg);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      r.d[a] = first(dn[a]);
+      r.d[3 + a] = second(dn[a]);
+      r.nu[a] = first(nu[a]);
+      r.nu[3 + a] = second(nu[a]);
+    }
+  }
+  if (XA && gd.bad()) r = stage_point_ieee<FIRST>(c, uin, du, col, k, o, As, Bs);
+  const T u[7] = {first(eb[0]),  first(eb[1]),  first(eb[2]), second(eb[0]),
+                  second(eb[1]), second(eb[2]), P};
+  stage_finish<BC>(c, u, r.d, r.nu, r.J, r.divE, r.divB, tst, flags, col, k, o, du, un, aux, uout);
+}
+
+template <typename T, bool BC, bool XA>
+__global__ void __launch_bounds__(kDirectX * kDirectY * direct_z<T>(),
+                                  sizeof(T) == 4 ? COFFEE_DIRECT_MINB : 2)
+    ez_ko_direct_kernel(const __grid_constant__ EzConst<T> c, const F7<const T> uin,
+                        const F7<T> uout, const T tko, const int j0, const int k0) {
+  const GridGeom& g = c.g;
+  const int i = g.lo[0] + blockIdx.x * kDirectX + threadIdx.x;
+  const int j = j0 + blockIdx.y * kDirectY + threadIdx.y;
+  const int k = k0 + blockIdx.z * direct_z<T>() + threadIdx.z;
+  if (i >= g.hi[0] || j >= g.hi[1] || k >= g.hi[2]) return;
+  const uint32_t st[3] = {1u, (uint32_t)g.sy, (uint32_t)g.sz};
+  const uint32_t o = (uint32_t)k * st[2] + (uint32_t)j * st[1] + (uint32_t)i;
+  const ColumnCtx<T> col = make_column<XA>(c, i, j);
+  T n7[7];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    auto at = [&](uint32_t q) { return pk(__ldg(uin.p[a] + q), __ldg(uin.p[3 + a] + q)); };
+    const Pair<T> cv = at(o);
+    Pair<T> s[3];
+#pragma unroll
+    for (int x = 0; x < 3; ++x)
+      s[x] = pd6_2<XA>(at(o - 3 * st[x]), at(o - 2 * st[x]), at(o - st[x]), cv, at(o + st[x]),
+                       at(o + 2 * st[x]), at(o + 3 * st[x]));
+    const Pair<T> v = pfma(both(c.ko_c), padd(padd(s[0], s[1]), s[2]), cv);
+    n7[a] = first(v);
+    n7[3 + a] = second(v);
+  }
+  n7[6] = __ldg(uin.p[6] + o);
+  if (c.semantics != SEM_CPU_REF) {
+    const T* p = uin.p[6];
+    T s[3];
+#pragma unroll
+    for (int x = 0; x < 3; ++x)
+      s[x] = d6_2(__ldg(p + (o - 3 * st[x])), __ldg(p + (o - 2 * st[x])), __ldg(p + (o - st[x])),
+                  n7[6], __ldg(p + (o + st[x])), __ldg(p + (o + 2 * st[x])),
+                  __ldg(p + (o + 3 * st[x])));
+    n7[6] = sfma(s[0] + s[1] + s[2], c.ko_c, n7[6]);
+  }
+  if constexpr (XA) apply_clamps_mid(n7);
+  else apply_clamps(c, n7[0], n7[1], n7[2], n7[3], n7[4], n7[5]);
+  if constexpr (BC) star_boundary(c, i, j, k, tko, n7);
+  store_with_images(g, col, uout, k, o, n7);
 }
 
 }  // namespace coffee

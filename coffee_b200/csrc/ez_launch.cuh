@@ -34,10 +34,16 @@ template <typename T> struct Shape;
 // FP32 tile shapes; the defaults are the tuned values, the macros exist so
 // that a build can be made with other shapes to measure them.
 #ifndef COFFEE_F32_STY
-#define COFFEE_F32_STY 16
+#define COFFEE_F32_STY 12
 #endif
 #ifndef COFFEE_F32_SPF
 #define COFFEE_F32_SPF 1
+#endif
+#ifndef COFFEE_F32_SPARE
+#define COFFEE_F32_SPARE 0
+#endif
+#ifndef COFFEE_F32_SMINB
+#define COFFEE_F32_SMINB 2
 #endif
 #ifndef COFFEE_F32_KTY
 #define COFFEE_F32_KTY 8
@@ -46,19 +52,16 @@ template <typename T> struct Shape;
 #define COFFEE_F32_KPF 1
 #endif
 template <> struct Shape<float> {
-  static constexpr int STX = 32, STY = COFFEE_F32_STY, SPF = COFFEE_F32_SPF;  // stage tile, prefetch
+  // stage tile, planes of prefetch, spare ring slots, resident CTAs per SM
+  static constexpr int STX = 32, STY = COFFEE_F32_STY, SPF = COFFEE_F32_SPF;
+  static constexpr int SSPARE = COFFEE_F32_SPARE, SMINB = COFFEE_F32_SMINB;
   static constexpr int KTX = 32, KTY = COFFEE_F32_KTY, KPF = COFFEE_F32_KPF;  // KO tile, prefetch
 };
 template <> struct Shape<double> {
-  static constexpr int STX = 32, STY = 4, SPF = 1;
+  static constexpr int STX = 32, STY = 12, SPF = 1, SSPARE = 0, SMINB = 1;
   static constexpr int KTX = 32, KTY = 4, KPF = 1;
 };
 
-template <typename T, int V, bool BC>
-size_t stage_smem(bool first) {
-  using S = Shape<T>;
-  return stage_smem_bytes<T, S::STX, S::STY, S::SPF, V, BC>(first);
-}
 template <typename T, int V, bool BC>
 size_t ko_smem() {
   using S = Shape<T>;
@@ -115,7 +118,7 @@ void build_const(const coffee_env* env, int semantics, EzConst<T>* c) {
   c->dt = (T)p.dt;
   c->ch2 = (T)p.ch2;
   c->tau = (T)p.tau;
-  c->inv_tau = (T)(1.0 / (double)c->tau);
+  c->inv_tau = (T)1 / c->tau;  // correctly rounded: the quotients P / tau need it
   // -KOeps * KO_const with KO_const = -1/64 (FFE_DISSIPATION_ORDER 6)
   c->ko_c = -(T)p.KOeps * (T)(-1.0 / 64.0);
   c->gam_dt = (T)p.damp_gamma / (T)p.dt;
@@ -125,6 +128,8 @@ void build_const(const coffee_env* env, int semantics, EzConst<T>* c) {
   c->check_egb = p.check_egb;
   c->semantics = semantics;
   c->taper_lanes = (sizeof(T) == 4) ? 16 : 8;  // AVX-512 width of the reference CPU build
+  // quotients by tau stay in the range of the straight-line division
+  c->tau_mid = std::fabs((double)c->tau) > 1e-6 && std::fabs((double)c->tau) < 1e6;
   c->problem = p.problem;
   bool abs_any = p.shift_ghost > 0;
   for (int a = 0; a < 3; ++a) {
@@ -181,12 +186,34 @@ inline bool flat_needs_bc(const coffee_params& p, int semantics) {
   return false;
 }
 
+// Points up to which the one-point-per-thread kernels are the faster ones (us, one
+// point per thread / streaming): FP32 stage 192^3 258 / 283, 256^3 591 / 570; FP32 KO
+// 128^3 76 / 76, 192^3 226 / 202; regrouped arithmetic, stage and KO 96^3 38 + 37 / 43
+// + 35, 128^3 85 + 87 / 79 + 76; FP64 stage 160^3 360 / 372, 256^3 1418 / 1320, KO
+// 256^3 978 / 1044.  With the boundary code the stage in the reference arithmetic is
+// faster at every size (192^3 298 / 421, 384^3 2264 / 2370, 512^3 5807 / 5732: the only
+// one), its KO pass up to 384^3 (1762 / 1790; 512^3 4538 / 3793), the regrouped ones
+// below 256^3 (192^3 300 + 271 / 334 + 317, 256^3 681 + 619 / 586 + 521).
+struct DirectPoints {
+  long long stage, ko;
+};
+template <typename T>
+constexpr DirectPoints direct_points(bool bc, bool xa) {
+  if (sizeof(T) == 8) return {8000000, 20000000};
+  if (bc && xa) return {1LL << 31, 57000000};
+  if (bc) return {10000000, 10000000};
+  if (xa) return {12000000, 2200000};
+  return {1200000, 1200000};
+}
+
 // Launch geometry of the flat kernels for one grid.
 struct FlatLaunch {
   bool bc;   // star / absorbing-layer code compiled in
   bool vec;  // planes copied as aligned element pairs (even row length d0)
   bool xa;   // the CPU build's own arithmetic (CPU semantics, ez_refarith.cuh)
   bool dg;   // and its energy-change diagnostics (xa only)
+  // one point per thread (not with the diagnostics)
+  bool direct_stage, direct_ko;
   int kchunk_stage, kchunk_ko;
   dim3 grid_stage, grid_ko;
 };
@@ -194,44 +221,102 @@ struct FlatLaunch {
 template <typename T, bool BC, int V, bool XA, bool DG = false>
 struct FlatKernels {
   using S = Shape<T>;
-  static constexpr auto first = ez_stage_kernel<T, S::STX, S::STY, S::SPF, true, BC, V, XA, DG>;
-  static constexpr auto rest = ez_stage_kernel<T, S::STX, S::STY, S::SPF, false, BC, V, XA, DG>;
-  static constexpr auto ko = ez_ko_kernel<T, S::KTX, S::KTY, S::KPF, BC, V, XA, DG>;
+  // the stage kernel: the register window in FP32 without the boundary code and
+  // the diagnostics, else the plane ring
+  static constexpr bool kFloat = std::is_same<T, float>::value;
+  static constexpr bool kDirectOnly = kFloat && BC && XA && !DG;  // the stage kernel
+  static constexpr bool kWindow = kFloat && !(BC && XA);
+  static constexpr int kTileX = 32, kTileY = kWindow ? 16 : S::STY;  // points of a stage CTA
+  static constexpr int kZU = BC ? 1 : 5;                 // z unroll of the window kernel
+  static constexpr int kChunkMult = kWindow ? kZU : 1;   // z chunks are multiples of it
+  template <bool FIRST>
+  static constexpr auto stage_fn() {
+    if constexpr (kWindow)
+      return ez_stage_window_kernel<T, kTileX, kTileY, S::SPF, kZU, FIRST, BC, V, XA, DG>;
+    else
+      return ez_stage_kernel<T, S::STX, S::STY, S::SPF, S::SSPARE, S::SMINB, FIRST, BC, XA, DG>;
+  }
+  static constexpr size_t stage_bytes(bool first) {
+    if constexpr (kWindow) return window_smem_bytes<T, kTileX, kTileY, S::SPF, V>(first);
+    else return stage_smem_bytes<T, S::STX, S::STY, S::SPF, S::SSPARE>();
+  }
+  static constexpr auto ko_fn() {
+    return ez_ko_kernel<T, S::KTX, S::KTY, S::KPF, BC, V, XA, DG>;
+  }
+
 
   static cudaError_t set_attributes() {
-    cudaError_t e = cudaFuncSetAttribute(first, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)stage_smem<T, V, BC>(true));
+    cudaError_t e = cudaSuccess;
+    if constexpr (!kDirectOnly) {
+      e = cudaFuncSetAttribute(stage_fn<true>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)stage_bytes(true));
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(stage_fn<false>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)stage_bytes(false));
+    }
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)stage_smem<T, V, BC>(false));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(ko_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)ko_smem<T, V, BC>());
     return e;
   }
   static cudaError_t occupancy(int* stage, int* kop) {
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(stage, rest, S::STX * S::STY,
-                                                                  stage_smem<T, V, BC>(false));
+    cudaError_t e = cudaSuccess;
+    if constexpr (!kDirectOnly)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(stage, stage_fn<false>(), kTileX * kTileY,
+                                                        stage_bytes(false));
     if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(kop, ko, S::KTX * S::KTY,
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(kop, ko_fn(), S::KTX * S::KTY,
                                                         ko_smem<T, V, BC>());
     return e;
+  }
+  // launches of the one-point-per-thread kernels: fn(grid, first row, first plane),
+  // more than one where an axis has more blocks than a grid dimension takes
+  template <class Fn>
+  static void direct_launches(const GridGeom& g, Fn&& fn) {
+    constexpr int kMax = 65535, bz = direct_z<T>();
+    const int n0 = g.hi[0] - g.lo[0];
+    for (int k = g.lo[2]; k < g.hi[2]; k += kMax * bz)
+      for (int j = g.lo[1]; j < g.hi[1]; j += kMax * kDirectY) {
+        const int n1 = std::min(g.hi[1] - j, kMax * kDirectY), n2 = std::min(g.hi[2] - k, kMax * bz);
+        fn(dim3((n0 + kDirectX - 1) / kDirectX, (n1 + kDirectY - 1) / kDirectY, (n2 + bz - 1) / bz),
+           j, k);
+      }
   }
   static void stage(bool is_first, const FlatLaunch& L, cudaStream_t st, const EzConst<T>& c,
                     const F7<const T>& src, const F7<T>& dst, const F7<T>& du, const F7<T>& un,
                     const F5<T>& aux, const F6<T>& dg, T As, T Bs, T tst, int flags) {
-    const dim3 bs(S::STX, S::STY);
-    if (is_first)
-      first<<<L.grid_stage, bs, stage_smem<T, V, BC>(true), st>>>(
-          c, src, dst, du, un, aux, dg, As, Bs, tst, L.kchunk_stage, flags);
-    else
-      rest<<<L.grid_stage, bs, stage_smem<T, V, BC>(false), st>>>(
-          c, src, dst, du, un, aux, dg, As, Bs, tst, L.kchunk_stage, flags);
+    auto launch = [&](auto fc) {
+      constexpr bool FIRST = decltype(fc)::value;
+      if constexpr (!DG) {
+        if (kDirectOnly || L.direct_stage) {
+          direct_launches(c.g, [&](dim3 grid, int j0, int k0) {
+            ez_stage_direct_kernel<T, FIRST, BC, XA>
+                <<<grid, dim3(kDirectX, kDirectY, direct_z<T>()), 0, st>>>(
+                    c, src, dst, du, un, aux, As, Bs, tst, flags, j0, k0);
+          });
+          return;
+        }
+      }
+      if constexpr (!kDirectOnly)
+        stage_fn<FIRST>()<<<L.grid_stage, dim3(kTileX, kTileY), stage_bytes(FIRST), st>>>(
+            c, src, dst, du, un, aux, dg, As, Bs, tst, L.kchunk_stage, flags);
+    };
+    if (is_first) launch(std::true_type{});
+    else launch(std::false_type{});
   }
   static void ko_pass(const FlatLaunch& L, cudaStream_t st, const EzConst<T>& c,
                       const F7<const T>& src, const F7<T>& dst, const F6<T>& dg, T tko) {
-    ko<<<L.grid_ko, dim3(S::KTX, S::KTY), ko_smem<T, V, BC>(), st>>>(c, src, dst, dg, tko,
-                                                                     L.kchunk_ko);
+    if constexpr (!DG) {
+      if (L.direct_ko) {
+        direct_launches(c.g, [&](dim3 grid, int j0, int k0) {
+          ez_ko_direct_kernel<T, BC, XA><<<grid, dim3(kDirectX, kDirectY, direct_z<T>()), 0, st>>>(
+              c, src, dst, tko, j0, k0);
+        });
+        return;
+      }
+    }
+    ko_fn()<<<L.grid_ko, dim3(S::KTX, S::KTY), ko_smem<T, V, BC>(), st>>>(c, src, dst, dg, tko,
+                                                                         L.kchunk_ko);
   }
 };
 
@@ -293,9 +378,13 @@ inline int flat_plan(const coffee_env* env, int semantics, FlatLaunch* L,
   if (npts >= (1LL << 31))
     return fail(COFFEE_E_CONFIG, "%lld points per array: the flat solver takes fewer than 2^31",
                 npts);
-  int per_sm_stage = 1, per_sm_ko = 1;
+  int per_sm_stage = 1, per_sm_ko = 1, tile_y = 1, stage_mult = 1;
   cudaError_t occ = cudaSuccess;
-  with_flat_kernels<T>(*L, [&](auto K) { occ = decltype(K)::occupancy(&per_sm_stage, &per_sm_ko); });
+  with_flat_kernels<T>(*L, [&](auto K) {
+    occ = decltype(K)::occupancy(&per_sm_stage, &per_sm_ko);
+    tile_y = decltype(K)::kTileY;
+    stage_mult = decltype(K)::kChunkMult;
+  });
   COFFEE_CUDA_TRY(occ);
   if (per_sm_stage < 1 || per_sm_ko < 1)
     return fail(COFFEE_E_CUDA, "stage/KO kernels cannot be resident (occupancy 0)");
@@ -303,20 +392,22 @@ inline int flat_plan(const coffee_env* env, int semantics, FlatLaunch* L,
   const coffee_params& p = env->p;
   int box[3];
   for (int a = 0; a < 3; ++a) box[a] = p.N[a] + 2 * p.shift_ghost;
-  const int sx = (box[0] + S::STX - 1) / S::STX, sy = (box[1] + S::STY - 1) / S::STY;
+  const int sx = (box[0] + S::STX - 1) / S::STX, sy = (box[1] + tile_y - 1) / tile_y;
   // a kernel whose ring length equals its z unroll needs chunks of a
   // multiple of it (its ring slots are then compile-time constants)
   auto chunk_mult = [](int unroll, int ring) { return unroll == ring ? unroll : 1; };
   L->kchunk_stage = pick_kchunk(
-      box[2], sx * sy, sms * per_sm_stage, 4,
-      L->bc ? chunk_mult(stage_zunroll<true>(), stage_ring<true, S::SPF>())
-            : chunk_mult(stage_zunroll<false>(), stage_ring<false, S::SPF>()));
+      box[2], sx * sy, sms * per_sm_stage, 4, stage_mult);
   L->grid_stage = dim3(sx, sy, (box[2] + L->kchunk_stage - 1) / L->kchunk_stage);
   const int kx = (box[0] + S::KTX - 1) / S::KTX, ky = (box[1] + S::KTY - 1) / S::KTY;
   L->kchunk_ko = pick_kchunk(box[2], kx * ky, sms * per_sm_ko, 6,
                              L->bc ? chunk_mult(ko_zunroll<true>(), ko_ring<true, S::KPF>())
                                    : chunk_mult(ko_zunroll<false>(), ko_ring<false, S::KPF>()));
   L->grid_ko = dim3(kx, ky, (box[2] + L->kchunk_ko - 1) / L->kchunk_ko);
+  const long long pts = (long long)box[0] * box[1] * box[2];
+  const DirectPoints dp = direct_points<T>(L->bc, L->xa);
+  L->direct_stage = !L->dg && pts <= dp.stage;
+  L->direct_ko = !L->dg && pts <= dp.ko;
   return COFFEE_OK;
 }
 

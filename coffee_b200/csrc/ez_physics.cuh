@@ -5,6 +5,7 @@
 #pragma once
 
 #include "ez_common.cuh"
+#include "ez_pair.cuh"
 #include "ez_refarith.cuh"
 
 namespace coffee {
@@ -423,6 +424,17 @@ __device__ __forceinline__ T p_taper_xa(const EzConst<T>& c, const ColumnCtx<T>&
   const T z = xa::lane_pos(c.delta[2], c.lower[2], k - c.g.guard[2], col.taper_dz);
   const T r = xa::sqrt(xa::dot3(col.taper_x, col.taper_x, col.taper_y, col.taper_y, z, z));
   return xa::taper_of_r(r);
+}
+
+// The same with the straight-line root and reciprocal of ez_pair.cuh.
+template <typename T>
+__device__ __forceinline__ T p_taper_mid(const EzConst<T>& c, const ColumnCtx<T>& col, int k,
+                                         Guard<T>& g) {
+  const T z = xa::lane_pos(c.delta[2], c.lower[2], k - c.g.guard[2], col.taper_dz);
+  const T r2 = xa::dot3(col.taper_x, col.taper_x, col.taper_y, col.taper_y, z, z);
+  g.above(r2, (T)1e-18);
+  g.below(r2, MidRange<T>::num_max);
+  return xa::taper_of_r<true>(sqrt_mid(r2));
 }
 
 template <bool XA, typename T>

@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include "ez_common.cuh"
+#include "ez_pair.cuh"
 
 namespace coffee {
 namespace xa {
@@ -132,6 +133,11 @@ __device__ __forceinline__ float vcl_expf(float x0) {
   return z;
 }
 
+// MID: without the branches of the IEEE division.  1 - 2 / (e + 1) is 1 for
+// every x >= 10 (the quotient is below 2^-27), so the exponential's argument
+// may stop at 2 * 16 and its divisor stays in the middle of the range, where
+// 2 RN(1/(e + 1)) is the rounded quotient.
+template <bool MID>
 __device__ __forceinline__ float vcl_tanhf(float x0) {
   const float x = fabsf(x0);
   float y;
@@ -142,8 +148,10 @@ __device__ __forceinline__ float vcl_tanhf(float x0) {
     p = __fmaf_rn(__fmaf_rn(2.06390887954E-2f, x2, -5.37397155531E-2f), x4, p);
     y = __fmaf_rn(p, __fmul_rn(x, x2), x);
   } else {
-    const float e = vcl_expf(__fadd_rn(x, x));
-    y = __fsub_rn(1.0f, __fdiv_rn(2.0f, __fadd_rn(e, 1.0f)));
+    const float xe = MID ? fminf(x, 16.0f) : x;
+    const float e = __fadd_rn(vcl_expf(__fadd_rn(xe, xe)), 1.0f);
+    const float q = MID ? __fmul_rn(2.0f, rcp_mid(e)) : __fdiv_rn(2.0f, e);
+    y = __fsub_rn(1.0f, q);
   }
   if (x > 44.4f) y = 1.0f;
   return copysignf(y, x0);
@@ -153,9 +161,11 @@ __device__ __forceinline__ float vcl_tanhf(float x0) {
 // 222-230), s = (1 - tanh((r - 3) / 0.5)) / 2, the division by 0.5 being a
 // multiplication by 2 (exact).  FP64: CUDA's tanh (the reference's double
 // build uses its library's double tanh; the two agree to rounding).
+template <bool MID = false>
 __device__ __forceinline__ float taper_of_r(float r) {
-  return __fmul_rn(__fsub_rn(1.0f, vcl_tanhf(__fmul_rn(__fadd_rn(r, -3.0f), 2.0f))), 0.5f);
+  return __fmul_rn(__fsub_rn(1.0f, vcl_tanhf<MID>(__fmul_rn(__fadd_rn(r, -3.0f), 2.0f))), 0.5f);
 }
+template <bool MID = false>
 __device__ __forceinline__ double taper_of_r(double r) {
   return __dmul_rn(__dsub_rn(1.0, ::tanh(__dmul_rn(__dadd_rn(r, -3.0), 2.0))), 0.5);
 }

@@ -225,3 +225,83 @@ def test_fp64_with_the_float_builds_taper_lanes():
     env.close()
     for f in range(7):
         assert rel_l2(out[f], d["out_f64_l16"][f]) < 1e-12, f
+
+
+def _ragged_case(n, tiny=False, star=False, dtype=np.float32):
+    """A periodic box of any size with smooth waves on B = x-hat (or a star with
+    an absorbing layer); with `tiny`, E and P fall from 1 to below the smallest
+    normal number across the box, zeros included."""
+    if star:
+        p = problems.pulsar_params(N=n[0], half_size=8.0, radius=2.1, pml=5)
+        d = p.size[0] / p.N[0]
+        p.N, p.size = list(n), [d * m for m in n]
+        p.p1, p.p3 = 0.6, 0.8
+    else:
+        p = problems.alfven_params(8)
+        p.N = list(n)
+        p.size = [m / 32 for m in n]
+        p.dt = 0.4 / 32
+    g = p.guard
+    x = [(np.arange(p.N[a] + 2 * g[a]) - g[a]) / p.N[a] * 2 * np.pi for a in range(3)]
+    Z, Y, X = np.meshgrid(x[2], x[1], x[0], indexing="ij")
+    if star:
+        f = problems.pulsar_fields(p, np.float64)
+        f[0:3] = [0.1 * f[3 + (c + 1) % 3] * np.sin(X + c) for c in range(3)]
+    else:
+        f = [0.2 * np.sin(X + Y + c) * np.cos(Z - c) for c in range(3)]
+        f += [(1.0 if c == 0 else 0.0) + 0.3 * np.cos(X - Z + 2 * c) * np.sin(Y + c)
+              for c in range(3)]
+        f.append(0.05 * np.sin(X + Z))
+    if tiny:
+        fall = 10.0 ** (-46.0 * (0.5 - 0.5 * np.cos(Z)))
+        f = [a if 3 <= c < 6 else a * fall for c, a in enumerate(f)]
+    return p, [a.astype(dtype) for a in f]
+
+
+# FP32 boxes: KO streams above 2.2 million points (the fifth) and the stage above 12
+# million (the last)
+@pytest.mark.parametrize("n,tiny", [((6, 7, 8), False), ((33, 6, 9), False), ((33, 6, 9), True),
+                                    ((31, 40, 20), True), ((161, 129, 107), False),
+                                    ((161, 129, 107), True), ((229, 231, 228), True),
+                                    ((230, 229, 229), False)])
+def test_flat_boxes_of_any_size_bit_for_bit(n, tiny):
+    """FP32 boxes with ragged edges in every direction, on both sides of the
+    one-point-per-thread limits and with rows of even and odd length, equal the
+    restatement bit for bit, also where quotients and derivatives leave the
+    range of the straight-line division."""
+    p, f = _ragged_case(n, tiny)
+    ref, _ = oracle.run_port(p, f, 2, semantics=0, taper_lanes=16)
+    out, _ = run_flat(p, f, 2)
+    for c in range(7):
+        assert count_differing(out[c], ref[c]) == 0, NAMES[c]
+
+
+@pytest.mark.parametrize("n", [(33, 20, 9), (129, 97, 103)])
+@pytest.mark.parametrize("semantics,arithmetic", [("cpu", "fast"), ("gpu", "reference")])
+def test_flat_boxes_of_any_size_regrouped(n, semantics, arithmetic):
+    """The regrouped arithmetic on the same grids: within FP32 rounding of the
+    FP64 restatement (2e-6 relative L2: some tens of roundings over ten stages)."""
+    p, f = _ragged_case(n)
+    ref, _ = oracle.run_port(p, [a.astype(np.float64) for a in f], 2,
+                             semantics=0 if semantics == "cpu" else 1, taper_lanes=16)
+    out, _ = run_flat(p, f, 2, semantics=semantics, arithmetic=arithmetic)
+    for c in range(7):
+        assert rel_l2(out[c], ref[c]) < 2e-6, NAMES[c]
+
+
+@pytest.mark.parametrize("n,star", [((33, 20, 9), False), ((201, 207, 203), False),
+                                    ((40, 42, 41), True), ((72, 70, 69), True)])
+def test_flat_fp64_and_star_of_any_size(n, star):
+    """FP64 (both kernels) within 1e-12 of the restatement, and the star with its
+    absorbing layer in FP32 within the float build's own bar (2e-5)."""
+    p, f = _ragged_case(n, star=star, dtype=np.float64)
+    ref, _ = oracle.run_port(p, f, 2, semantics=0, taper_lanes=8)
+    out, _ = run_flat(p, f, 2)
+    for c in range(7):
+        assert rel_l2(out[c], ref[c]) < 1e-12, NAMES[c]
+    if star:
+        f = [a.astype(np.float32) for a in f]
+        ref, _ = oracle.run_port(p, f, 2, semantics=0, taper_lanes=16)
+        out, _ = run_flat(p, f, 2)
+        for c in range(7):
+            assert rel_l2(out[c], ref[c]) < 2e-5, NAMES[c]
