@@ -70,6 +70,7 @@ void fill_sph_const(const coffee_env* env, const void* tab, SphConst<T>* c) {
   c->dt = (T)p.dt;
   c->ch2 = (T)p.ch2;
   c->tau = (T)p.tau;
+  c->inv_tau = (T)1 / c->tau;
   c->gam_dt = (T)((T)p.damp_gamma / (T)p.dt);
   c->ko_c = (T)(p.KOeps / 64.0);
   c->calc_current = p.calc_current;
@@ -130,6 +131,7 @@ void fill_cyl_const(const coffee_env* env, CylConst<T>* c) {
   c->dt = (T)p.dt;
   c->ch2 = (T)p.ch2;
   c->tau = (T)p.tau;
+  c->inv_tau = (T)1 / c->tau;
   c->ko_c = (T)(p.KOeps / 64.0);
   c->clean_ep = p.clean_ep;
   c->check_egb = p.check_egb;

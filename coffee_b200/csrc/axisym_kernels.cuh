@@ -15,6 +15,7 @@
 
 #include "coffee_b200.h"
 #include "ez_common.cuh"
+#include "ez_pair.cuh"
 
 namespace coffee {
 
@@ -22,18 +23,19 @@ enum AxiFlags { AX_LAST = 1, AX_AUX = 2, AX_WRITE_UN = 4 };
 
 // CTAs of 256 threads kept resident per SM (bounds the registers per thread;
 // the kernels are latency-bound on their stencil loads, so more warps help,
-// until spilling costs more).  Measured on 2048 x 1024 / 1024 x 2048 grids:
-// the log-spherical kernels are fastest with 8 (32 registers), the
-// cylindrical stage with 6 (40), the cylindrical KO with 4 (64); the
-// batched log-spherical kernels (64 runs) with 4.
+// until spilling costs more).  Measured, us for four steps: log-spherical 2048 x
+// 1024 with 8 (32 registers) / 6 / 5 / 4: 2038 / 2060 / 2162 / 2193; eight
+// batched runs (whose parameters come from shared memory) with 4 (64) / 5 / 6:
+// 5053 / 4868 / 4924; cylindrical 1024 x 2048, stage with 6 (40) / 5 / 4 / 3: 2083 /
+// 1905 / 1798 / 2000, KO with 4 (64).
 #ifndef COFFEE_SPH_MIN_BLOCKS
 #define COFFEE_SPH_MIN_BLOCKS 8
 #endif
 #ifndef COFFEE_SPH_BATCH_MIN_BLOCKS
-#define COFFEE_SPH_BATCH_MIN_BLOCKS 4
+#define COFFEE_SPH_BATCH_MIN_BLOCKS 5
 #endif
 #ifndef COFFEE_CYL_STAGE_MIN_BLOCKS
-#define COFFEE_CYL_STAGE_MIN_BLOCKS 6
+#define COFFEE_CYL_STAGE_MIN_BLOCKS 4
 #endif
 #ifndef COFFEE_CYL_KO_MIN_BLOCKS
 #define COFFEE_CYL_KO_MIN_BLOCKS 4
@@ -62,7 +64,7 @@ struct SphConst {
   int axis_lo, axis_hi;    // theta = 0 / theta = pi rows, -1 if not on the grid
   int g0, g1;              // guards: x_i = x0 + dx * (i - g0), y_j = y0 + dy * (j - g1)
   T dx, dy, inv_dx, inv_dy, x0, y0;
-  T dt, ch2, tau, gam_dt, ko_c;
+  T dt, ch2, tau, inv_tau, gam_dt, ko_c;
   int calc_current, edotb, divB_clean, clean_ep, check_egb, ko_geometry;
   T radius, b0, omega;
   T tp_start, tp_end, dw0, nT, thp1, thp2;
@@ -82,12 +84,58 @@ struct CylConst {
   int axis_col;  // the R = 0 column, -1 if not on the grid
   int g0, g1;    // guards: R_i = R0 + dR * (i - g0), z_j = z0 + dz * (j - g1)
   T dR, dz, inv_dR, inv_dz, R0, z0;
-  T dt, ch2, tau, ko_c;
+  T dt, ch2, tau, inv_tau, ko_c;
   int clean_ep, check_egb;
   T radius, b0, omega;
   T tp_start, tp_end, dw0, th1, th2;  // wpert window in theta (precomputed)
   int absorbing;
   T xh, xl, yh, yl, pmlscale, sigpml;
+};
+
+// The four weights of diff1_4 (src/algorithms/finite_diff.h:14-19) and the seven of
+// the 6th difference.
+template <typename T>
+__device__ __forceinline__ constexpr T diff4(int k) {
+  return T(k == 0 ? 1 : k == 1 ? -8 : k == 2 ? 8 : -1);
+}
+template <typename T>
+__device__ __forceinline__ constexpr T diff6(int k) {
+  return T(k == 0 || k == 6 ? 1 : k == 1 || k == 5 ? -6 : k == 3 ? -20 : 15);
+}
+
+// Stencil values around one point of (E_a, B_a) pairs or single fields, at offset k
+// along x (immediate offsets from the point's address) or y (one 32-bit element
+// offset per row; an array of these 2D grids has far fewer than 2^31 points).
+// NC as for ldf.
+template <bool NC, typename T>
+struct Stencil2D {
+  const F7<T>& u;
+  uint32_t o, d0;
+  __device__ __forceinline__ T x(int f, int k) const { return ldf<NC>(u.p[f] + o + k); }
+  __device__ __forceinline__ T y(int f, int k) const {
+    return ldf<NC>(u.p[f] + (uint32_t)(o + (uint32_t)k * d0));
+  }
+  __device__ __forceinline__ Pair<T> px(int a, int k) const { return pk(x(a, k), x(3 + a, k)); }
+  __device__ __forceinline__ Pair<T> py(int a, int k) const { return pk(y(a, k), y(3 + a, k)); }
+  // sum of w[k] times the pair a at the four points of diff1_4
+  __device__ __forceinline__ Pair<T> dx(int a, const T w[4]) const {
+    Pair<T> t = pmul(px(a, -2), both(w[0]));
+    t = pfma(px(a, -1), both(w[1]), t);
+    t = pfma(px(a, 1), both(w[2]), t);
+    return pfma(px(a, 2), both(w[3]), t);
+  }
+  __device__ __forceinline__ Pair<T> dy(int a, const T w[4]) const {
+    Pair<T> t = pmul(py(a, -2), both(w[0]));
+    t = pfma(py(a, -1), both(w[1]), t);
+    t = pfma(py(a, 1), both(w[2]), t);
+    return pfma(py(a, 2), both(w[3]), t);
+  }
+  __device__ __forceinline__ T dx1(int f) const {
+    return sfma(T(8), x(f, 1) - x(f, -1), x(f, -2) - x(f, 2));
+  }
+  __device__ __forceinline__ T dy1(int f) const {
+    return sfma(T(8), y(f, 1) - y(f, -1), y(f, -2) - y(f, 2));
+  }
 };
 
 template <typename T>
@@ -207,8 +255,9 @@ __device__ __noinline__ V7<T> sph_absorb(const SphConst<T>& c, V7<T> v, V7<T> n,
 // launch of its own, one thread per column, the boundary cost 20 us after
 // each 80 us stage at 2048 x 1024 (one chain of dependent accesses).
 template <typename T>
-__device__ __forceinline__ void sph_store(const SphConst<T>& c, const int j, const long long o,
+__device__ __forceinline__ void sph_store(const SphConst<T>& c, const int j, const uint32_t o32,
                                           const V7<T>& w, const F7<T>& out) {
+  const long long o = o32;
   // rows above theta = 0 and below theta = pi (far from an axis not on the grid)
   const int up = c.axis_lo >= 0 ? j - c.axis_lo : 1 << 20;
   const int down = c.axis_hi >= 0 ? c.axis_hi - j : 1 << 20;
@@ -259,115 +308,105 @@ __device__ __forceinline__ void sph_stage_point(const SphConst<T>& c, const int 
                                                 const F7<T>& du, const F7<T>& un,
                                                 const F5<T>& aux, const T As, const T Bs,
                                                 const T tst, const int flags) {
-  const long long d0 = c.d0;
-  const long long o = i + j * d0;
-  T r[5], sn[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    r[k] = __ldg(c.rt + i - 2 + k);
-    sn[k] = __ldg(c.st + j - 2 + k);
-  }
-  const T rc = r[2], sc = sn[2];
+  const uint32_t d0 = (uint32_t)c.d0;
+  const uint32_t o = (uint32_t)i + (uint32_t)j * d0;
+  const Stencil2D<NC, T> st{u, o, d0};
+  const T rc = __ldg(c.rt + i), sc = __ldg(c.st + j), asc = fabs(sc);
   const T g11 = rc * rc;
   const T g33 = (rc * sc) * (rc * sc);
-  T gms = rc * rc * rc * fabs(sc);
+  T gms = rc * rc * rc * asc;
   if (gms < Tiny<T>::v) gms = Tiny<T>::v;
   const T igms = T(1) / gms;
 
-  const T* Ex = u.p[0];
-  const T* Ey = u.p[1];
-  const T* Ez = u.p[2];
-  const T* Bx = u.p[3];
-  const T* By = u.p[4];
-  const T* Bz = u.p[5];
-  const T* P = u.p[6];
-  auto X = [&](const T* f, int k) { return ldf<NC>(f + o + (k - 2)); };
-  auto Y = [&](const T* f, int k) { return ldf<NC>(f + o + (k - 2) * d0); };
-
-  // lowered fields at the stencil points: El_x = r^2 E_x, El_y = r^2 E_y,
-  // El_z = (r sin th)^2 E_z (metric_sph.h:90-122)
-  auto g33x = [&](int k) { return (r[k] * sc) * (r[k] * sc); };
-  auto g33y = [&](int k) { return (rc * sn[k]) * (rc * sn[k]); };
-  const T idx12 = c.inv_dx, idy12 = c.inv_dy;
-  auto dX = [&](auto fn) { return d1_4w(fn(0), fn(1), fn(3), fn(4)) * idx12; };
-  auto dY = [&](auto fn) { return d1_4w(fn(0), fn(1), fn(3), fn(4)) * idy12; };
-
-  const T rotBx = dY([&](int k) { return g33y(k) * Y(Bz, k); }) * igms;
-  const T rotEx = dY([&](int k) { return g33y(k) * Y(Ez, k); }) * igms;
-  const T rotBy = -dX([&](int k) { return g33x(k) * X(Bz, k); }) * igms;
-  const T rotEy = -dX([&](int k) { return g33x(k) * X(Ez, k); }) * igms;
-  const T rotBz = (dX([&](int k) { return r[k] * r[k] * X(By, k); }) -
-                   dY([&](int k) { return g11 * Y(Bx, k); })) * igms;
-  const T rotEz = (dX([&](int k) { return r[k] * r[k] * X(Ey, k); }) -
-                   dY([&](int k) { return g11 * Y(Ex, k); })) * igms;
-  // div4_sph (field_solver_EZ_spherical.cu:99-124): sqrt(gamma) = r^3 |sin th|
-  const T asc = fabs(sc);
-  auto sgx = [&](int k) { return r[k] * r[k] * r[k] * asc; };
-  auto sgy = [&](int k) { return rc * rc * rc * fabs(sn[k]); };
-  const T divE = (dX([&](int k) { return X(Ex, k) * sgx(k); }) +
-                  dY([&](int k) { return Y(Ey, k) * sgy(k); })) * igms;
-  const T divB = (dX([&](int k) { return X(Bx, k) * sgx(k); }) +
-                  dY([&](int k) { return Y(By, k) * sgy(k); })) * igms;
-
-  T v[7];
+  // the weights of diff1_4 times those of the lowered fields (El_x = r^2 E_x,
+  // El_y = r^2 E_y, El_z = (r sin th)^2 E_z, metric_sph.h:90-122) or of div4_sph
+  // (sqrt(gamma) = r^3 |sin th|, field_solver_EZ_spherical.cu:99-124) at the
+  // stencil points, over sqrt(gamma): formed once for the E and B of a pair
+  const T hx = c.inv_dx * T(1.0 / 12.0), hy = c.inv_dy * T(1.0 / 12.0);
+  T x11[4], x33[4], xs[4], y11[4], y33[4], ys[4];
 #pragma unroll
-  for (int a = 0; a < 7; ++a) v[a] = ldf<NC>(u.p[a] + o);
-  const T el[3] = {g11 * v[0], g11 * v[1], g33 * v[2]};
-  const T bl[3] = {g11 * v[3], g11 * v[4], g33 * v[5]};
-  T B2 = v[3] * bl[0] + v[4] * bl[1] + v[5] * bl[2];
-  if (B2 < Tiny<T>::v) B2 = Tiny<T>::v;
+  for (int k = 0; k < 4; ++k) {
+    const int n = k < 2 ? k - 2 : k - 1;
+    const T r = __ldg(c.rt + i + n), sn = __ldg(c.st + j + n);
+    const T wx = diff4<T>(k) * (hx * igms), wy = diff4<T>(k) * (hy * igms);
+    x11[k] = r * r * wx;
+    x33[k] = (r * sc) * (r * sc) * wx;
+    xs[k] = r * r * r * asc * wx;
+    y11[k] = g11 * wy;
+    y33[k] = (rc * sn) * (rc * sn) * wy;
+    ys[k] = rc * rc * rc * fabs(sn) * wy;
+  }
+  // (rot E, rot B) and (div E, div B)
+  const Pair<T> rot0 = st.dy(2, y33);
+  const Pair<T> rot1 = pmul(st.dx(2, x33), both(T(-1)));
+  const Pair<T> rot2 = psub(st.dx(1, x11), st.dy(0, y11));
+  const Pair<T> rot[3] = {rot0, rot1, rot2};
+  const Pair<T> dvg = padd(st.dx(0, xs), st.dy(1, ys));
+  const T divE = first(dvg), divB = second(dvg);
+
+  Pair<T> eb[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) eb[a] = st.px(a, 0);
+  const T P = st.x(6, 0);
   T J[3] = {T(0), T(0), T(0)};
   if (c.calc_current) {
-    T Jp = (bl[0] * rotBx + bl[1] * rotBy + bl[2] * rotBz) -
-           (el[0] * rotEx + el[1] * rotEy + el[2] * rotEz);
-    const T cx = el[1] * bl[2] - el[2] * bl[1];
-    const T cy = el[2] * bl[0] - el[0] * bl[2];
-    const T cz = el[0] * bl[1] - el[1] * bl[0];
+    const Pair<T> low[3] = {pmul(eb[0], both(g11)), pmul(eb[1], both(g11)), pmul(eb[2], both(g33))};
+    const Pair<T> sq = pdot3(eb, low), lr = pdot3(low, rot);  // (E2, B2), (E.rotE, B.rotB)
+    T B2 = second(sq);
+    if (B2 < Tiny<T>::v) B2 = Tiny<T>::v;
+    T Jp = second(lr) - first(lr);
+    const T el[3] = {first(low[0]), first(low[1]), first(low[2])};
+    const T bl[3] = {second(low[0]), second(low[1]), second(low[2])};
+    const T C[3] = {el[1] * bl[2] - el[2] * bl[1], el[2] * bl[0] - el[0] * bl[2],
+                    el[0] * bl[1] - el[1] * bl[0]};
     if (c.edotb) {
-      const T E2 = v[0] * el[0] + v[1] * el[1] + v[2] * el[2];
-      const T chi2 = B2 - E2;
-      const T EdotB = v[0] * bl[0] + v[1] * bl[1] + v[2] * bl[2];
+      const T chi2 = B2 - first(sq);
+      const T EdotB = first(eb[0]) * bl[0] + first(eb[1]) * bl[1] + first(eb[2]) * bl[2];
       const T E02 = T(0.5) * (sqrt(chi2 * chi2 + T(4) * EdotB * EdotB) - chi2);
       Jp += c.gam_dt * EdotB;
       const T a = fdiv(divE * igms, E02 + B2);
       const T q = fdiv(Jp, B2);
-      J[0] = a * cx + q * v[3];
-      J[1] = a * cy + q * v[4];
-      J[2] = a * cz + q * v[5];
+#pragma unroll
+      for (int n = 0; n < 3; ++n) J[n] = a * C[n] + q * second(eb[n]);
     } else {
       const T iB2 = fdiv(T(1), B2);
-      J[0] = (divE * cx * igms + Jp * v[3]) * iB2;
-      J[1] = (divE * cy * igms + Jp * v[4]) * iB2;
-      J[2] = (divE * cz * igms + Jp * v[5]) * iB2;
+#pragma unroll
+      for (int n = 0; n < 3; ++n) J[n] = (divE * C[n] * igms + Jp * second(eb[n])) * iB2;
     }
   }
-  T Px = T(0), Py = T(0);
+  T gP[3] = {T(0), T(0), T(0)};
   if (c.divB_clean) {
-    Px = fdiv(dX([&](int k) { return X(P, k); }), g11);
-    Py = fdiv(dY([&](int k) { return Y(P, k); }), g11);
+    const T ig = fdiv(T(1), g11);
+    gP[0] = st.dx1(6) * (hx * ig);
+    gP[1] = st.dy1(6) * (hy * ig);
     // Pz = dfdz(P) / gamma_33 with dfdz = 0; the reference's 0/0 on the
     // theta = 0 row only reaches dB_z of that row, which the axis
     // boundary overwrites.
   }
   const T dt = c.dt;
-  T rhs[7];
-  rhs[0] = dt * (rotBx - J[0]);
-  rhs[1] = dt * (rotBy - J[1]);
-  rhs[2] = dt * (rotBz - J[2]);
-  rhs[3] = -dt * (rotEx + Px);
-  rhs[4] = -dt * (rotEy + Py);
-  rhs[5] = -dt * rotEz;
-  rhs[6] = -dt * c.ch2 * divB - v[6] / c.tau;
-
   if (flags & AX_WRITE_UN) {
 #pragma unroll
-    for (int a = 0; a < 6; ++a) un.p[a][o] = v[a];
+    for (int a = 0; a < 3; ++a) {
+      un.p[a][o] = first(eb[a]);
+      un.p[3 + a][o] = second(eb[a]);
+    }
   }
+  T v[7];
 #pragma unroll
-  for (int a = 0; a < 7; ++a) {
-    const T d = FIRST ? rhs[a] : As * du.p[a][o] + rhs[a];
-    du.p[a][o] = d;
-    v[a] += Bs * d;
+  for (int a = 0; a < 3; ++a) {
+    Pair<T> d = pmul(pk(second(rot[a]) - J[a], first(rot[a]) + gP[a]), pk(dt, -dt));
+    if constexpr (!FIRST) d = pfma(pk(du.p[a][o], du.p[3 + a][o]), both(As), d);
+    du.p[a][o] = first(d);
+    du.p[3 + a][o] = second(d);
+    const Pair<T> n = pfma(d, both(Bs), eb[a]);
+    v[a] = first(n);
+    v[3 + a] = second(n);
+  }
+  {
+    T d = -dt * c.ch2 * divB - P * c.inv_tau;
+    if constexpr (!FIRST) d = sfma(du.p[6][o], As, d);
+    du.p[6][o] = d;
+    v[6] = sfma(d, Bs, P);
   }
   if (flags & AX_AUX) {
     aux.p[0][o] = J[0];
@@ -418,37 +457,51 @@ __global__ void __launch_bounds__(256, kSphMinBlocks) sph_stage_kernel(const __g
 template <typename T, bool NC = true>
 __device__ __forceinline__ void sph_ko_point(const SphConst<T>& c, const int i, const int j,
                                              const F7<T>& u, const F7<T>& out, const T tend) {
-  const long long d0 = c.d0;
-  const long long o = i + j * d0;
-  constexpr T K6[7] = {T(1), T(-6), T(15), T(-20), T(15), T(-6), T(1)};
-  T wx[7], wy[7];
+  const uint32_t d0 = (uint32_t)c.d0;
+  const uint32_t o = (uint32_t)i + (uint32_t)j * d0;
+  const Stencil2D<NC, T> st{u, o, d0};
   const T rc = __ldg(c.rt + i), sc = __ldg(c.st + j);
-  T gms = rc * rc * rc * fabs(sc);
-  if (gms < Tiny<T>::v) gms = Tiny<T>::v;
-  if (c.ko_geometry) {  // sqrt(gamma) at the stencil points
+  T wx[7], wy[7], scale = c.ko_c;
+  if (c.ko_geometry) {  // sqrt(gamma) at the stencil points over that of the point
+    T gms = rc * rc * rc * fabs(sc);
+    if (gms < Tiny<T>::v) gms = Tiny<T>::v;
+    scale = c.ko_c / gms;
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
       const T rk = __ldg(c.rt + i - 3 + k);
-      wx[k] = K6[k] * (rk * rk * rk * fabs(sc));
-      wy[k] = K6[k] * (rc * rc * rc * fabs(__ldg(c.st + j - 3 + k)));
+      wx[k] = diff6<T>(k) * (rk * rk * rk * fabs(sc));
+      wy[k] = diff6<T>(k) * (rc * rc * rc * fabs(__ldg(c.st + j - 3 + k)));
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < 7; ++k) wx[k] = wy[k] = K6[k];
+    for (int k = 0; k < 7; ++k) wx[k] = wy[k] = diff6<T>(k);
   }
+  const T wc = wx[3] + wy[3];
   T v[7];
 #pragma unroll
-  for (int a = 0; a < 7; ++a) {
-    const T* f = u.p[a];
-    T tx = T(0), ty = T(0);
+  for (int a = 0; a < 3; ++a) {
+    const Pair<T> own = st.px(a, 0);
+    Pair<T> t = pmul(own, both(wc));
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
-      tx += wx[k] * ldf<NC>(f + o + (k - 3));
-      ty += wy[k] * ldf<NC>(f + o + (k - 3) * d0);
+      if (k == 3) continue;
+      t = pfma(st.px(a, k - 3), both(wx[k]), t);
+      t = pfma(st.py(a, k - 3), both(wy[k]), t);
     }
-    T t = tx + ty;
-    if (c.ko_geometry) t = t / gms;
-    v[a] = ldf<NC>(f + o) + c.ko_c * t;
+    const Pair<T> n = pfma(t, both(scale), own);
+    v[a] = first(n);
+    v[3 + a] = second(n);
+  }
+  {
+    const T own = st.x(6, 0);
+    T t = own * wc;
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      if (k == 3) continue;
+      t = sfma(st.x(6, k - 3), wx[k], t);
+      t = sfma(st.y(6, k - 3), wy[k], t);
+    }
+    v[6] = sfma(t, scale, own);
   }
   sph_clamps(c, v, rc * rc, (rc * sc) * (rc * sc));
   V7<T> w;
@@ -955,56 +1008,67 @@ __global__ void __launch_bounds__(256, kCylStageMinBlocks) cyl_stage_kernel(cons
   const int i = c.lo0 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = c.lo1 + blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= c.hi0 || j >= c.hi1) return;
-  const long long d0 = c.d0;
-  const long long o = i + j * d0;
+  const uint32_t d0 = (uint32_t)c.d0;
+  const uint32_t o = (uint32_t)i + (uint32_t)j * d0;
+  const Stencil2D<true, T> st{u, o, d0};
   T R = c.R0 + c.dR * (T)(i - c.g0);
   if (fabs(R) < Tiny<T>::v) R = Tiny<T>::v;
-  auto X = [&](const T* f, int k) { return __ldg(f + o + (k - 2)); };
-  auto Y = [&](const T* f, int k) { return __ldg(f + o + (k - 2) * d0); };
-  auto dR = [&](const T* f) { return d1_4w(X(f, 0), X(f, 1), X(f, 3), X(f, 4)) * c.inv_dR; };
-  auto dz = [&](const T* f) { return d1_4w(Y(f, 0), Y(f, 1), Y(f, 3), Y(f, 4)) * c.inv_dz; };
-  // dfRdRR (:110-113): (R f)_R / R, 2 f_R on the axis
+  // the weights of diff1_4 along R and z and of dfRdRR (:110-113): (R f)_R / R, 2 f_R
+  // on the axis
   const bool on_axis = fabs(R) < c.dR * T(0.25);
-  auto dRR = [&](const T* f) {
-    if (on_axis) return T(2) * dR(f);
-    const T h = c.dR;
-    return d1_4w(X(f, 0) * (R - T(2) * h), X(f, 1) * (R - h), X(f, 3) * (R + h),
-                 X(f, 4) * (R + T(2) * h)) * c.inv_dR / R;
-  };
-  const T *ER = u.p[0], *Ez = u.p[1], *Ef = u.p[2], *BR = u.p[3], *Bz = u.p[4], *Bf = u.p[5];
-  const T rotBR = -dz(Bf), rotBz = dRR(Bf), rotBf = dz(BR) - dR(Bz);
-  const T rotER = -dz(Ef), rotEz = dRR(Ef), rotEf = dz(ER) - dR(Ez);
-  const T divE = dRR(ER) + dz(Ez);
-  const T divB = dRR(BR) + dz(Bz);
-  T v[7];
+  const T hR = c.inv_dR * T(1.0 / 12.0), hz = c.inv_dz * T(1.0 / 12.0), iR = T(1) / R;
+  T wR[4], wz[4], wRR[4];
 #pragma unroll
-  for (int a = 0; a < 7; ++a) v[a] = __ldg(u.p[a] + o);
-  T B2 = v[3] * v[3] + v[4] * v[4] + v[5] * v[5];
+  for (int k = 0; k < 4; ++k) {
+    const int n = k < 2 ? k - 2 : k - 1;
+    wR[k] = diff4<T>(k) * hR;
+    wz[k] = diff4<T>(k) * hz;
+    wRR[k] = on_axis ? T(2) * wR[k] : wR[k] * ((R + T(n) * c.dR) * iR);
+  }
+  // (rot E, rot B) along R, z, phi and (div E, div B)
+  const Pair<T> rot[3] = {pmul(st.dy(2, wz), both(T(-1))), st.dx(2, wRR),
+                          psub(st.dy(0, wz), st.dx(1, wR))};
+  const Pair<T> dvg = padd(st.dx(0, wRR), st.dy(1, wz));
+  const T divE = first(dvg), divB = second(dvg);
+  Pair<T> eb[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) eb[a] = st.px(a, 0);
+  const T P = st.x(6, 0);
+  const T E[3] = {first(eb[0]), first(eb[1]), first(eb[2])};
+  const T B[3] = {second(eb[0]), second(eb[1]), second(eb[2])};
+  T B2 = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
   if (B2 < Tiny<T>::v) B2 = Tiny<T>::v;
-  const T Jp = (v[3] * rotBR + v[4] * rotBz + v[5] * rotBf) -
-               (v[0] * rotER + v[1] * rotEz + v[2] * rotEf);
+  const Pair<T> lr = pdot3(eb, rot);
+  const T Jp = second(lr) - first(lr);
   const T iB2 = fdiv(T(1), B2);
-  const T JR = (divE * (v[2] * v[4] - v[1] * v[5]) + Jp * v[3]) * iB2;
-  const T Jf = (divE * (v[1] * v[3] - v[0] * v[4]) + Jp * v[5]) * iB2;
-  const T Jz = (divE * (v[0] * v[5] - v[2] * v[3]) + Jp * v[4]) * iB2;
+  const T J[3] = {(divE * (E[2] * B[1] - E[1] * B[2]) + Jp * B[0]) * iB2,
+                  (divE * (E[0] * B[2] - E[2] * B[0]) + Jp * B[1]) * iB2,
+                  (divE * (E[1] * B[0] - E[0] * B[1]) + Jp * B[2]) * iB2};
+  const T gP[3] = {st.dx1(6) * hR, st.dy1(6) * hz, T(0)};
   const T dt = c.dt;
-  T rhs[7];
-  rhs[0] = dt * (rotBR - JR);
-  rhs[1] = dt * (rotBz - Jz);
-  rhs[2] = dt * (rotBf - Jf);
-  rhs[3] = -dt * (rotER + dR(u.p[6]));
-  rhs[4] = -dt * (rotEz + dz(u.p[6]));
-  rhs[5] = -dt * rotEf;
-  rhs[6] = -dt * c.ch2 * divB - v[6] / c.tau;
   if (flags & AX_WRITE_UN) {
 #pragma unroll
-    for (int a = 0; a < 6; ++a) un.p[a][o] = v[a];
+    for (int a = 0; a < 3; ++a) {
+      un.p[a][o] = E[a];
+      un.p[3 + a][o] = B[a];
+    }
   }
+  T v[7];
 #pragma unroll
-  for (int a = 0; a < 7; ++a) {
-    const T d = FIRST ? rhs[a] : As * du.p[a][o] + rhs[a];
-    du.p[a][o] = d;
-    v[a] += Bs * d;
+  for (int a = 0; a < 3; ++a) {
+    Pair<T> d = pmul(pk(second(rot[a]) - J[a], first(rot[a]) + gP[a]), pk(dt, -dt));
+    if constexpr (!FIRST) d = pfma(pk(du.p[a][o], du.p[3 + a][o]), both(As), d);
+    du.p[a][o] = first(d);
+    du.p[3 + a][o] = second(d);
+    const Pair<T> n = pfma(d, both(Bs), eb[a]);
+    v[a] = first(n);
+    v[3 + a] = second(n);
+  }
+  {
+    T d = -dt * c.ch2 * divB - P * c.inv_tau;
+    if constexpr (!FIRST) d = sfma(du.p[6][o], As, d);
+    du.p[6][o] = d;
+    v[6] = sfma(d, Bs, P);
   }
   cyl_clamps(c, v);
   cyl_finish(c, i, j, o, v, out, un, tst, (flags & AX_LAST) != 0);
@@ -1020,20 +1084,33 @@ __global__ void __launch_bounds__(256, kCylKoMinBlocks) cyl_ko_kernel(const __gr
   const int i = c.lo0 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = c.lo1 + blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= c.hi0 || j >= c.hi1) return;
-  const long long d0 = c.d0;
-  const long long o = i + j * d0;
-  constexpr T K6[7] = {T(1), T(-6), T(15), T(-20), T(15), T(-6), T(1)};
+  const uint32_t d0 = (uint32_t)c.d0;
+  const uint32_t o = (uint32_t)i + (uint32_t)j * d0;
+  const Stencil2D<true, T> st{u, o, d0};
+  // the 6th differences of both axes: neighbours at distance 1, 2, 3 weigh 15, -6, 1
+  // and the point -40
   T v[7];
 #pragma unroll
-  for (int a = 0; a < 7; ++a) {
-    const T* f = u.p[a];
-    T tx = T(0), ty = T(0);
+  for (int a = 0; a < 3; ++a) {
+    Pair<T> t[4];
 #pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      tx += K6[k] * __ldg(f + o + (k - 3));
-      ty += K6[k] * __ldg(f + o + (k - 3) * d0);
-    }
-    v[a] = __ldg(f + o) + c.ko_c * (tx + ty);
+    for (int n = 1; n < 4; ++n)
+      t[n] = padd(padd(st.px(a, -n), st.px(a, n)), padd(st.py(a, -n), st.py(a, n)));
+    const Pair<T> own = st.px(a, 0);
+    Pair<T> s = pfma(t[2], both(T(-6)), t[3]);
+    s = pfma(own, both(T(-40)), pfma(t[1], both(T(15)), s));
+    const Pair<T> n = pfma(s, both(c.ko_c), own);
+    v[a] = first(n);
+    v[3 + a] = second(n);
+  }
+  {
+    T t[4];
+#pragma unroll
+    for (int n = 1; n < 4; ++n)
+      t[n] = (st.x(6, -n) + st.x(6, n)) + (st.y(6, -n) + st.y(6, n));
+    const T own = st.x(6, 0);
+    const T s = sfma(own, T(-40), sfma(t[1], T(15), sfma(t[2], T(-6), t[3])));
+    v[6] = sfma(s, c.ko_c, own);
   }
   cyl_clamps(c, v);
   cyl_finish(c, i, j, o, v, out, un, tend, false);
