@@ -526,7 +526,7 @@ def run_ours(args):
                               if n_side >= 512 else "smaller case (profiling)"),
                        "parallelism": f"replicas x{ws}"},
             "hbm_gbs": hbm_gbs,
-            "roofline": {"kernel": "ez_stage_kernel (LSRK stages 2-5)", "bound": "hbm",
+            "roofline": {"kernel": "ez_stage_window_kernel (LSRK stages 2-5)", "bound": "hbm",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "traffic": (traffic_pp * cells if traffic_pp else None),
