@@ -313,12 +313,15 @@ __device__ __noinline__ V7<T> gr_absorb(const GrConst<T>& c, V7<T> v, V7<T> n, T
 // field_solver_gr_EZ.cu:188-420, then the clamps and, in the last stage,
 // the absorbing layers: order of :876-893).  u: D, B, P of the current
 // buffer; eh: E, H of the same buffer.
-// Minimum resident 256-thread CTAs per SM of the stage kernel: the kernel is
-// bound by the latency of its stencil loads, and 6 CTAs (40 registers, a
-// little spilling) hide it best (1.31 -> 1.19 ms per launch at 256^3; 7 or 8
-// CTAs spill too much).
+// Minimum resident 256-thread CTAs per SM of the stage and KO kernels: bound by the
+// latency of their stencil loads, they want warps until spilling costs more.  256^3
+// Wald run, one step, with (stage, KO) CTAs of (7, 6) / (6, 4) / (5, 5) / (4, 4): 6118
+// / 5555 / 5337 / 5335 us.
 #ifndef COFFEE_GR_STAGE_MIN_BLOCKS
-#define COFFEE_GR_STAGE_MIN_BLOCKS 6
+#define COFFEE_GR_STAGE_MIN_BLOCKS 5
+#endif
+#ifndef COFFEE_GR_KO_MIN_BLOCKS
+#define COFFEE_GR_KO_MIN_BLOCKS 5
 #endif
 // The stage at one point, given its stencil values through fetch(q, ax,
 // n): array q (0-2 E, 3-5 H, 6-8 D, 9-11 B, 12 P, 13 sqrt(gamma)) at offset
@@ -639,7 +642,7 @@ __global__ void __launch_bounds__(kGrTX * kGrTY, COFFEE_GR_TILE_MINB) gr_stage_t
 // Kreiss-Oliger pass (kernel_KO_step1_gr / _step2_gr, :523-608, with the
 // 3D 6th difference of finite_diff.h:84-92), then the clamps (:895-900).
 template <typename T>
-__global__ void __launch_bounds__(256) gr_ko_kernel(const __grid_constant__ GrConst<T> c,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? COFFEE_GR_KO_MIN_BLOCKS : 2) gr_ko_kernel(const __grid_constant__ GrConst<T> c,
                                                     const F7<T> u, const F7<T> out,
                                                     const T* __restrict__ mt,
                                                     const F7<T> ehout) {
