@@ -23,13 +23,17 @@ enum AxiFlags { AX_LAST = 1, AX_AUX = 2, AX_WRITE_UN = 4 };
 
 // CTAs of 256 threads kept resident per SM (bounds the registers per thread;
 // the kernels are latency-bound on their stencil loads, so more warps help,
-// until spilling costs more).  Measured, us for four steps: log-spherical 2048 x
-// 1024 with 8 (32 registers) / 6 / 5 / 4: 2038 / 2060 / 2162 / 2193; eight
-// batched runs (whose parameters come from shared memory) with 4 (64) / 5 / 6:
-// 5053 / 4868 / 4924; cylindrical 1024 x 2048, stage with 6 (40) / 5 / 4 / 3: 2083 /
+// until spilling costs more).  Measured, us a step: log-spherical 2048 x 1024 with 8
+// (32 registers) / 6 / 5 / 4: 554 / 496 / 506 / 522, 512 x 256 67 / 66 / 63 / 55; FP64
+// with 8 / 6 / 5 / 4 / 3: 1748 / 1203 / 987 / 893 / 984.  Batched runs (whose parameters
+// come from shared memory), us for four steps of eight, with 4 (64) / 5 / 6: 5053 / 4868
+// / 4924.  Cylindrical 1024 x 2048, us for four steps, stage with 6 (40) / 5 / 4 / 3: 2083 /
 // 1905 / 1798 / 2000, KO with 4 (64).
 #ifndef COFFEE_SPH_MIN_BLOCKS
-#define COFFEE_SPH_MIN_BLOCKS 8
+#define COFFEE_SPH_MIN_BLOCKS 6
+#endif
+#ifndef COFFEE_SPH_MIN_BLOCKS_F64
+#define COFFEE_SPH_MIN_BLOCKS_F64 4
 #endif
 #ifndef COFFEE_SPH_BATCH_MIN_BLOCKS
 #define COFFEE_SPH_BATCH_MIN_BLOCKS 5
@@ -40,7 +44,8 @@ enum AxiFlags { AX_LAST = 1, AX_AUX = 2, AX_WRITE_UN = 4 };
 #ifndef COFFEE_CYL_KO_MIN_BLOCKS
 #define COFFEE_CYL_KO_MIN_BLOCKS 4
 #endif
-constexpr int kSphMinBlocks = COFFEE_SPH_MIN_BLOCKS;
+template <typename T>
+constexpr int kSphMinBlocks = sizeof(T) == 4 ? COFFEE_SPH_MIN_BLOCKS : COFFEE_SPH_MIN_BLOCKS_F64;
 constexpr int kSphBatchMinBlocks = COFFEE_SPH_BATCH_MIN_BLOCKS;
 constexpr int kCylStageMinBlocks = COFFEE_CYL_STAGE_MIN_BLOCKS;
 constexpr int kCylKoMinBlocks = COFFEE_CYL_KO_MIN_BLOCKS;
@@ -117,7 +122,7 @@ struct Stencil2D {
   }
   __device__ __forceinline__ Pair<T> px(int a, int k) const { return pk(x(a, k), x(3 + a, k)); }
   __device__ __forceinline__ Pair<T> py(int a, int k) const { return pk(y(a, k), y(3 + a, k)); }
-  // sum of w[k] times the pair a at the four points of diff1_4
+  // sum of w[k] times the pair a at the four points of diff1_4, or with its own weights
   __device__ __forceinline__ Pair<T> dx(int a, const T w[4]) const {
     Pair<T> t = pmul(px(a, -2), both(w[0]));
     t = pfma(px(a, -1), both(w[1]), t);
@@ -129,6 +134,12 @@ struct Stencil2D {
     t = pfma(py(a, -1), both(w[1]), t);
     t = pfma(py(a, 1), both(w[2]), t);
     return pfma(py(a, 2), both(w[3]), t);
+  }
+  __device__ __forceinline__ Pair<T> dx(int a) const {
+    return pfma(psub(px(a, 1), px(a, -1)), both(T(8)), psub(px(a, -2), px(a, 2)));
+  }
+  __device__ __forceinline__ Pair<T> dy(int a) const {
+    return pfma(psub(py(a, 1), py(a, -1)), both(T(8)), psub(py(a, -2), py(a, 2)));
   }
   __device__ __forceinline__ T dx1(int f) const {
     return sfma(T(8), x(f, 1) - x(f, -1), x(f, -2) - x(f, 2));
@@ -318,30 +329,36 @@ __device__ __forceinline__ void sph_stage_point(const SphConst<T>& c, const int 
   if (gms < Tiny<T>::v) gms = Tiny<T>::v;
   const T igms = T(1) / gms;
 
-  // the weights of diff1_4 times those of the lowered fields (El_x = r^2 E_x,
-  // El_y = r^2 E_y, El_z = (r sin th)^2 E_z, metric_sph.h:90-122) or of div4_sph
-  // (sqrt(gamma) = r^3 |sin th|, field_solver_EZ_spherical.cu:99-124) at the
-  // stencil points, over sqrt(gamma): formed once for the E and B of a pair
-  const T hx = c.inv_dx * T(1.0 / 12.0), hy = c.inv_dy * T(1.0 / 12.0);
-  T x11[4], x33[4], xs[4], y11[4], y33[4], ys[4];
+  // The lowered fields (El_x = r^2 E_x, El_y = r^2 E_y, El_z = (r sin th)^2 E_z,
+  // metric_sph.h:90-122) and sqrt(gamma) = r^3 |sin th| of div4_sph
+  // (field_solver_EZ_spherical.cu:99-124) are products of a power of r and one of
+  // sin th: a derivative along r is summed with the weights of diff1_4 times the
+  // power of r, one along theta with those times the power of sin th, both formed
+  // once for the E and B of a pair.  What the four points share scales the finished
+  // sum, and what both derivatives of a curl or divergence share scales their sum:
+  // these sums cancel, and a factor multiplied into a weight or into one of two
+  // derivatives rounds it to a value that no longer matches the others, at a point the
+  // same one in every stage (B_theta and P of a run 5% farther from 64 bits).
+  T r2[4], r3[4], s1[4], s2[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int n = k < 2 ? k - 2 : k - 1;
     const T r = __ldg(c.rt + i + n), sn = __ldg(c.st + j + n);
-    const T wx = diff4<T>(k) * (hx * igms), wy = diff4<T>(k) * (hy * igms);
-    x11[k] = r * r * wx;
-    x33[k] = (r * sc) * (r * sc) * wx;
-    xs[k] = r * r * r * asc * wx;
-    y11[k] = g11 * wy;
-    y33[k] = (rc * sn) * (rc * sn) * wy;
-    ys[k] = rc * rc * rc * fabs(sn) * wy;
+    r2[k] = diff4<T>(k) * (r * r);
+    r3[k] = diff4<T>(k) * (r * r * r);
+    s1[k] = diff4<T>(k) * fabs(sn);
+    s2[k] = diff4<T>(k) * (sn * sn);
   }
   // (rot E, rot B) and (div E, div B)
-  const Pair<T> rot0 = st.dy(2, y33);
-  const Pair<T> rot1 = pmul(st.dx(2, x33), both(T(-1)));
-  const Pair<T> rot2 = psub(st.dx(1, x11), st.dy(0, y11));
-  const Pair<T> rot[3] = {rot0, rot1, rot2};
-  const Pair<T> dvg = padd(st.dx(0, xs), st.dy(1, ys));
+  Pair<T> rot[3] = {pmul(st.dy(2, s2), both(c.inv_dy * g11)),
+                    pmul(st.dx(2, r2), both(-c.inv_dx * (sc * sc))),
+                    pfma(st.dx(1, r2), both(c.inv_dx), pmul(st.dy(0), both(-c.inv_dy * g11)))};
+  Pair<T> dvg = pfma(st.dx(0, r3), both(c.inv_dx * asc),
+                     pmul(st.dy(1, s1), both(c.inv_dy * (g11 * rc))));
+  const T igms12 = igms * T(1.0 / 12.0);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) rot[a] = pmul(rot[a], both(igms12));
+  dvg = pmul(dvg, both(igms12));
   const T divE = first(dvg), divB = second(dvg);
 
   Pair<T> eb[3];
@@ -376,9 +393,8 @@ __device__ __forceinline__ void sph_stage_point(const SphConst<T>& c, const int 
   }
   T gP[3] = {T(0), T(0), T(0)};
   if (c.divB_clean) {
-    const T ig = fdiv(T(1), g11);
-    gP[0] = st.dx1(6) * (hx * ig);
-    gP[1] = st.dy1(6) * (hy * ig);
+    gP[0] = fdiv(st.dx1(6) * (c.inv_dx * T(1.0 / 12.0)), g11);
+    gP[1] = fdiv(st.dy1(6) * (c.inv_dy * T(1.0 / 12.0)), g11);
     // Pz = dfdz(P) / gamma_33 with dfdz = 0; the reference's 0/0 on the
     // theta = 0 row only reaches dB_z of that row, which the axis
     // boundary overwrites.
@@ -436,7 +452,7 @@ __device__ __forceinline__ void sph_stage_point(const SphConst<T>& c, const int 
 }
 
 template <typename T, bool FIRST>
-__global__ void __launch_bounds__(256, kSphMinBlocks) sph_stage_kernel(const __grid_constant__ SphConst<T> c,
+__global__ void __launch_bounds__(256, kSphMinBlocks<T>) sph_stage_kernel(const __grid_constant__ SphConst<T> c,
                                                         const F7<T> u, const F7<T> out,
                                                         const F7<T> du, const F7<T> un,
                                                         const F5<T> aux, const T As,
@@ -476,32 +492,29 @@ __device__ __forceinline__ void sph_ko_point(const SphConst<T>& c, const int i, 
 #pragma unroll
     for (int k = 0; k < 7; ++k) wx[k] = wy[k] = diff6<T>(k);
   }
-  const T wc = wx[3] + wy[3];
+  // one chain per axis from one end to the other, where the running sum stays
+  // below 10 fields (a sum that starts with the point's own -40 rounds at that size)
   T v[7];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const Pair<T> own = st.px(a, 0);
-    Pair<T> t = pmul(own, both(wc));
+    Pair<T> tx = pmul(st.px(a, -3), both(wx[0])), ty = pmul(st.py(a, -3), both(wy[0]));
 #pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      if (k == 3) continue;
-      t = pfma(st.px(a, k - 3), both(wx[k]), t);
-      t = pfma(st.py(a, k - 3), both(wy[k]), t);
+    for (int k = 1; k < 7; ++k) {
+      tx = pfma(st.px(a, k - 3), both(wx[k]), tx);
+      ty = pfma(st.py(a, k - 3), both(wy[k]), ty);
     }
-    const Pair<T> n = pfma(t, both(scale), own);
+    const Pair<T> n = pfma(padd(tx, ty), both(scale), st.px(a, 0));
     v[a] = first(n);
     v[3 + a] = second(n);
   }
   {
-    const T own = st.x(6, 0);
-    T t = own * wc;
+    T tx = st.x(6, -3) * wx[0], ty = st.y(6, -3) * wy[0];
 #pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      if (k == 3) continue;
-      t = sfma(st.x(6, k - 3), wx[k], t);
-      t = sfma(st.y(6, k - 3), wy[k], t);
+    for (int k = 1; k < 7; ++k) {
+      tx = sfma(st.x(6, k - 3), wx[k], tx);
+      ty = sfma(st.y(6, k - 3), wy[k], ty);
     }
-    v[6] = sfma(t, scale, own);
+    v[6] = sfma(tx + ty, scale, st.x(6, 0));
   }
   sph_clamps(c, v, rc * rc, (rc * sc) * (rc * sc));
   V7<T> w;
@@ -513,7 +526,7 @@ __device__ __forceinline__ void sph_ko_point(const SphConst<T>& c, const int i, 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256, kSphMinBlocks) sph_ko_kernel(const __grid_constant__ SphConst<T> c,
+__global__ void __launch_bounds__(256, kSphMinBlocks<T>) sph_ko_kernel(const __grid_constant__ SphConst<T> c,
                                                      const F7<T> u, const F7<T> out,
                                                      const T tend) {
   const int i = c.lo0 + blockIdx.x * blockDim.x + threadIdx.x;

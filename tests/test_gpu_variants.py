@@ -342,3 +342,40 @@ def test_logsph_axis_rows(nr, nth, shift, theta):
         # FP64 roundings by at most 1e4 on these grids
         scale = np.abs(ref[f]).max() + 1e-30
         np.testing.assert_allclose(out[f][0], ref[f], rtol=0, atol=1e-11 * scale)
+
+
+def _rounding(cls, p, fields, evolve, nsteps):
+    """Distance of an FP32 run from the FP64 restatement over that of the FP32
+    restatement (plain operations, no fused multiply-adds), per field."""
+    f = [np.asarray(a, dtype=np.float32) for a in fields]
+    U = np.stack([a.reshape(a.shape[-2:]) if evolve is not gr_oracle.gr_evolve else a for a in f])
+    ref, plain = evolve(p, U.astype(np.float64), nsteps), evolve(p, U, nsteps)
+    out, _ = _run_ours(cls, p, [a.reshape((1,) * (3 - a.ndim) + a.shape) for a in f], nsteps)
+    return [rel_l2(out[c].reshape(ref[c].shape), ref[c]) / rel_l2(plain[c], ref[c])
+            for c in range(7)]
+
+
+def _waves(p, rng, ndim=2):
+    """Seven random sums of three plane waves on p's grid."""
+    n = [np.arange(p.N[a] + 2 * p.guard[a]) / p.N[a] for a in reversed(range(ndim))]
+    x = np.meshgrid(*n, indexing="ij")[::-1]
+    return [sum(rng.uniform(0.3, 1) * np.sin(2 * np.pi * sum(rng.integers(1, 4) * q for q in x) +
+                                             rng.uniform(0, 6.3)) for _ in range(3))
+            for _ in range(7)]
+
+
+def test_logsph_rounding():
+    """The sums of the log-spherical stage and KO pass round no more than they
+    have to.  Four seeds, mean: B_theta 0.979, P 0.812; with the metric and
+    1 / sqrt(gamma) rounded into the difference weights 1.029 and 0.829."""
+    r = []
+    for seed in range(4):
+        p = problems.sph_pulsar_params(nr=300, nth=170)
+        f = problems.sph_pulsar_fields(p, np.float64)
+        w = _waves(p, np.random.default_rng(seed))
+        scale = np.abs(f[3]) + np.abs(f[4])
+        r.append(_rounding(FieldSolverEZSpherical, p,
+                           [(a + 0.03 * scale * b)[0] for a, b in zip(f, w)], axo.sph_evolve, 4))
+    r = np.mean(r, 0)
+    print(r)
+    assert r[4] < 1.0 and r[6] < 0.82
