@@ -27,8 +27,8 @@ enum AxiFlags { AX_LAST = 1, AX_AUX = 2, AX_WRITE_UN = 4 };
 // (32 registers) / 6 / 5 / 4: 554 / 496 / 506 / 522, 512 x 256 67 / 66 / 63 / 55; FP64
 // with 8 / 6 / 5 / 4 / 3: 1748 / 1203 / 987 / 893 / 984.  Batched runs (whose parameters
 // come from shared memory), us for four steps of eight, with 4 (64) / 5 / 6: 5053 / 4868
-// / 4924.  Cylindrical 1024 x 2048, us for four steps, stage with 6 (40) / 5 / 4 / 3: 2083 /
-// 1905 / 1798 / 2000, KO with 4 (64).
+// / 4924.  Cylindrical 1024 x 2048, us a step, stage and KO with 4 (64) and 4 / 3 and 5 / 5
+// and 3: 449 / 492 / 459; FP64 772 / 809 / 855.
 #ifndef COFFEE_SPH_MIN_BLOCKS
 #define COFFEE_SPH_MIN_BLOCKS 6
 #endif
@@ -1026,22 +1026,23 @@ __global__ void __launch_bounds__(256, kCylStageMinBlocks) cyl_stage_kernel(cons
   const Stencil2D<true, T> st{u, o, d0};
   T R = c.R0 + c.dR * (T)(i - c.g0);
   if (fabs(R) < Tiny<T>::v) R = Tiny<T>::v;
-  // the weights of diff1_4 along R and z and of dfRdRR (:110-113): (R f)_R / R, 2 f_R
-  // on the axis
+  // dfRdRR (:110-113): (R f)_R / R, 2 f_R on the axis, as the weights of diff1_4 times
+  // R at the four points.  Factors are kept out of the weights and of the single
+  // derivatives as in sph_stage_point (E_phi of a run was 2.3 times farther from 64 bits,
+  // B_z 5%).
   const bool on_axis = fabs(R) < c.dR * T(0.25);
-  const T hR = c.inv_dR * T(1.0 / 12.0), hz = c.inv_dz * T(1.0 / 12.0), iR = T(1) / R;
-  T wR[4], wz[4], wRR[4];
+  const T iRR = on_axis ? T(2) * c.inv_dR : c.inv_dR / R;
+  T wRR[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int n = k < 2 ? k - 2 : k - 1;
-    wR[k] = diff4<T>(k) * hR;
-    wz[k] = diff4<T>(k) * hz;
-    wRR[k] = on_axis ? T(2) * wR[k] : wR[k] * ((R + T(n) * c.dR) * iR);
-  }
+  for (int k = 0; k < 4; ++k)
+    wRR[k] = diff4<T>(k) * (on_axis ? T(1) : R + T(k < 2 ? k - 2 : k - 1) * c.dR);
   // (rot E, rot B) along R, z, phi and (div E, div B)
-  const Pair<T> rot[3] = {pmul(st.dy(2, wz), both(T(-1))), st.dx(2, wRR),
-                          psub(st.dy(0, wz), st.dx(1, wR))};
-  const Pair<T> dvg = padd(st.dx(0, wRR), st.dy(1, wz));
+  Pair<T> rot[3] = {pmul(st.dy(2), both(-c.inv_dz)), pmul(st.dx(2, wRR), both(iRR)),
+                    pfma(st.dy(0), both(c.inv_dz), pmul(st.dx(1), both(-c.inv_dR)))};
+  Pair<T> dvg = pfma(st.dx(0, wRR), both(iRR), pmul(st.dy(1), both(c.inv_dz)));
+#pragma unroll
+  for (int a = 0; a < 3; ++a) rot[a] = pmul(rot[a], both(T(1.0 / 12.0)));
+  dvg = pmul(dvg, both(T(1.0 / 12.0)));
   const T divE = first(dvg), divB = second(dvg);
   Pair<T> eb[3];
 #pragma unroll
@@ -1057,7 +1058,8 @@ __global__ void __launch_bounds__(256, kCylStageMinBlocks) cyl_stage_kernel(cons
   const T J[3] = {(divE * (E[2] * B[1] - E[1] * B[2]) + Jp * B[0]) * iB2,
                   (divE * (E[0] * B[2] - E[2] * B[0]) + Jp * B[1]) * iB2,
                   (divE * (E[1] * B[0] - E[0] * B[1]) + Jp * B[2]) * iB2};
-  const T gP[3] = {st.dx1(6) * hR, st.dy1(6) * hz, T(0)};
+  const T gP[3] = {st.dx1(6) * (c.inv_dR * T(1.0 / 12.0)),
+                   st.dy1(6) * (c.inv_dz * T(1.0 / 12.0)), T(0)};
   const T dt = c.dt;
   if (flags & AX_WRITE_UN) {
 #pragma unroll
@@ -1100,30 +1102,28 @@ __global__ void __launch_bounds__(256, kCylKoMinBlocks) cyl_ko_kernel(const __gr
   const uint32_t d0 = (uint32_t)c.d0;
   const uint32_t o = (uint32_t)i + (uint32_t)j * d0;
   const Stencil2D<true, T> st{u, o, d0};
-  // the 6th differences of both axes: neighbours at distance 1, 2, 3 weigh 15, -6, 1
-  // and the point -40
+  // the 6th differences, one chain per axis as in sph_ko_point
   T v[7];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    Pair<T> t[4];
+    Pair<T> tx = st.px(a, -3), ty = st.py(a, -3);
 #pragma unroll
-    for (int n = 1; n < 4; ++n)
-      t[n] = padd(padd(st.px(a, -n), st.px(a, n)), padd(st.py(a, -n), st.py(a, n)));
-    const Pair<T> own = st.px(a, 0);
-    Pair<T> s = pfma(t[2], both(T(-6)), t[3]);
-    s = pfma(own, both(T(-40)), pfma(t[1], both(T(15)), s));
-    const Pair<T> n = pfma(s, both(c.ko_c), own);
+    for (int k = 1; k < 7; ++k) {
+      tx = pfma(st.px(a, k - 3), both(diff6<T>(k)), tx);
+      ty = pfma(st.py(a, k - 3), both(diff6<T>(k)), ty);
+    }
+    const Pair<T> n = pfma(padd(tx, ty), both(c.ko_c), st.px(a, 0));
     v[a] = first(n);
     v[3 + a] = second(n);
   }
   {
-    T t[4];
+    T tx = st.x(6, -3), ty = st.y(6, -3);
 #pragma unroll
-    for (int n = 1; n < 4; ++n)
-      t[n] = (st.x(6, -n) + st.x(6, n)) + (st.y(6, -n) + st.y(6, n));
-    const T own = st.x(6, 0);
-    const T s = sfma(own, T(-40), sfma(t[1], T(15), sfma(t[2], T(-6), t[3])));
-    v[6] = sfma(s, c.ko_c, own);
+    for (int k = 1; k < 7; ++k) {
+      tx = sfma(st.x(6, k - 3), diff6<T>(k), tx);
+      ty = sfma(st.y(6, k - 3), diff6<T>(k), ty);
+    }
+    v[6] = sfma(tx + ty, c.ko_c, st.x(6, 0));
   }
   cyl_clamps(c, v);
   cyl_finish(c, i, j, o, v, out, un, tend, false);

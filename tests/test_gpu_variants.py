@@ -379,3 +379,22 @@ def test_logsph_rounding():
     r = np.mean(r, 0)
     print(r)
     assert r[4] < 1.0 and r[6] < 0.82
+
+
+def test_cylindrical_rounding():
+    """The same of the cylindrical solver, a wave field that is smooth on the
+    axis: E_z 0.741, E_phi 0.777; with 1 / delta and 1 / R rounded into the
+    weights 0.765 and 0.804."""
+    r = []
+    for seed in range(4):
+        p = problems.cyl_pulsar_params(nR=170, nz=300, radius=0.02)
+        p.b0 = 1e-3
+        w = _waves(p, np.random.default_rng(seed))
+        R = (np.arange(p.N[0] + 2 * p.guard[0]) - p.guard[0]) * p.size[0] / p.N[0]
+        odd = R / (np.abs(R) + 2.0)
+        r.append(_rounding(FieldSolverEZCylindrical, p,
+                           [0.05 * w[0] * odd, 0.05 * w[1], 0.05 * w[2] * odd, 0.1 * w[3] * odd,
+                            1 + 0.1 * w[4], 0.1 * w[5] * odd, 0.01 * w[6]], axo.cyl_evolve, 4))
+    r = np.mean(r, 0)
+    print(r)
+    assert r[1] < 0.753 and r[2] < 0.79
