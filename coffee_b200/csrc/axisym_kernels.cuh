@@ -419,7 +419,7 @@ __device__ __forceinline__ void sph_stage_point(const SphConst<T>& c, const int 
     v[3 + a] = second(n);
   }
   {
-    T d = -dt * c.ch2 * divB - P * c.inv_tau;
+    T d = -dt * c.ch2 * divB - div_const(P, c.tau, c.inv_tau);
     if constexpr (!FIRST) d = sfma(du.p[6][o], As, d);
     du.p[6][o] = d;
     v[6] = sfma(d, Bs, P);
@@ -1080,7 +1080,7 @@ __global__ void __launch_bounds__(256, kCylStageMinBlocks) cyl_stage_kernel(cons
     v[3 + a] = second(n);
   }
   {
-    T d = -dt * c.ch2 * divB - P * c.inv_tau;
+    T d = -dt * c.ch2 * divB - div_const(P, c.tau, c.inv_tau);
     if constexpr (!FIRST) d = sfma(du.p[6][o], As, d);
     du.p[6][o] = d;
     v[6] = sfma(d, Bs, P);

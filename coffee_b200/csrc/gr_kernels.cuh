@@ -433,7 +433,7 @@ __device__ __forceinline__ void gr_stage_point(const GrConst<T>& c, Metric&& met
     db[a] = pfma(d, both(Bs), db[a]);
   }
   {
-    T d = dt * (lP - m.alpha * divB) - m.alpha * P * c.inv_tau;
+    T d = dt * (lP - m.alpha * divB) - div_const(m.alpha * P, c.tau, c.inv_tau);
     if constexpr (!FIRST) d = sfma(du.p[6][o], As, d);
     du.p[6][o] = d;
     P = sfma(d, Bs, P);

@@ -398,3 +398,31 @@ def test_cylindrical_rounding():
     r = np.mean(r, 0)
     print(r)
     assert r[1] < 0.753 and r[2] < 0.79
+
+
+@pytest.mark.parametrize("tau", [0.83, 1.3])
+@pytest.mark.parametrize("solver", ["logsph", "cyl"])
+def test_p_over_tau_is_the_rounded_quotient(solver, tau):
+    """P alone, the time step too small for anything else to reach it: five
+    stages of dP = A dP - P / tau, P += B dP in FP32 with fused sums and a
+    correctly rounded quotient, bit for bit."""
+    if solver == "logsph":
+        p, cls, box = problems.sph_pulsar_params(nr=64, nth=40), FieldSolverEZSpherical, (8, 24)
+        f = problems.sph_pulsar_fields(p, np.float32)
+    else:
+        p, cls, box = problems.cyl_pulsar_params(nR=64, nz=60), FieldSolverEZCylindrical, (16, 30)
+        f = problems.cyl_pulsar_fields(p, np.float32)
+    p.tau, p.dt, p.KOeps = float(np.float32(tau)), 1e-12, 0.0
+    f[6] = np.random.default_rng(1).uniform(1, 2, f[6].shape).astype(np.float32)
+    A = [0, -0.4178904745, -1.192151694643, -1.697784692471, -1.514183444257]
+    B = [0.1496590219993, 0.3792103129999, 0.8229550293869, 0.6994504559488, 0.1530572479681]
+    # (an FMA through FP64: the products are exact, and a sum that rounds twice is one in 1e8)
+    fma = lambda x, y, z: (x.astype(np.float64) * np.float64(np.float32(y)) + z).astype(np.float32)
+    P = f[6].copy()
+    d = np.zeros_like(P)
+    for a, b in zip(A, B):
+        d = fma(d, a, -(P / np.float32(tau)))
+        P = fma(d, b, P)
+    out, _ = _run_ours(cls, p, list(f), 1)
+    sl = (0, slice(box[0], -box[0]), slice(box[1], -box[0]))
+    assert np.array_equal(out[6][sl], P[sl]), int((out[6][sl] != P[sl]).sum())
