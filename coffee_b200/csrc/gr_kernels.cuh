@@ -343,8 +343,10 @@ __device__ __forceinline__ void gr_stage_point(const GrConst<T>& c, Metric&& met
   using I2 = std::integral_constant<int, 2>;
   using QP = std::integral_constant<int, 12>;
   using QS = std::integral_constant<int, 13>;
-  // diff1_4 of the pair (E_q, H_q) along an axis, times 12 / inv_delta; the
-  // factor is applied once per curl and divergence
+  // diff1_4 of the pair (E_q, H_q) along an axis, times 12 / inv_delta.  1 / 12 goes
+  // with the 1 / sqrt(gamma) of a whole curl or divergence: its terms cancel, and
+  // 1 / 12 rounded into inv_delta of each axis would change their ratio where the
+  // spacings differ (P of such a run 1% farther from 64 bits)
   auto d1 = [&](auto qc, auto ac) {
     constexpr int q = decltype(qc)::value;
     using H = std::integral_constant<int, q + 3>;
@@ -353,15 +355,14 @@ __device__ __forceinline__ void gr_stage_point(const GrConst<T>& c, Metric&& met
     t = pfma(v(-1), both((T)-8), t);
     return pfma(v(1), both((T)8), t);
   };
-  const T w12[3] = {c.inv_delta[0] * T(1.0 / 12.0), c.inv_delta[1] * T(1.0 / 12.0),
-                    c.inv_delta[2] * T(1.0 / 12.0)};
+  const T* w = c.inv_delta;
   // the curls and divergences before their 1 / sqrt(gamma) factor: the
   // metric is evaluated after the stencil sums, so that its values do not
   // take registers while those are formed (the same operations either way)
   Pair<T> rot[3];  // (rot E, rot H)
-  rot[0] = pfma(d1(I2{}, I1{}), both(w12[1]), pmul(d1(I1{}, I2{}), both(-w12[2])));
-  rot[1] = pfma(d1(I0{}, I2{}), both(w12[2]), pmul(d1(I2{}, I0{}), both(-w12[0])));
-  rot[2] = pfma(d1(I1{}, I0{}), both(w12[0]), pmul(d1(I0{}, I1{}), both(-w12[1])));
+  rot[0] = pfma(d1(I2{}, I1{}), both(w[1]), pmul(d1(I1{}, I2{}), both(-w[2])));
+  rot[1] = pfma(d1(I0{}, I2{}), both(w[2]), pmul(d1(I2{}, I0{}), both(-w[0])));
+  rot[2] = pfma(d1(I1{}, I0{}), both(w[0]), pmul(d1(I0{}, I1{}), both(-w[1])));
   // div4 (:44-86): each neighbour weighted by sqrt(gamma) there (the
   // per-solver table; the reference evaluates it at the shifted coordinates)
   Pair<T> dvg = both((T)0);  // (div D, div B)
@@ -374,19 +375,19 @@ __device__ __forceinline__ void gr_stage_point(const GrConst<T>& c, Metric&& met
     t = pfma(v(-1), both(T(-8) * f(QS{}, ac, -1)), t);
     t = pfma(v(1), both(T(8) * f(QS{}, ac, 1)), t);
     t = pfma(v(2), both(-f(QS{}, ac, 2)), t);
-    dvg = pfma(t, both(w12[ax]), dvg);
+    dvg = pfma(t, both(w[ax]), dvg);
   });
   T Pd[3];
   static_for<3>([&](auto ac) {
     constexpr int ax = decltype(ac)::value;
     const T t = sfma(f(QP{}, ac, -1), (T)-8, f(QP{}, ac, -2) - f(QP{}, ac, 2));
-    Pd[ax] = sfma(f(QP{}, ac, 1), (T)8, t) * w12[ax];
+    Pd[ax] = sfma(f(QP{}, ac, 1), (T)8, t) * (w[ax] * T(1.0 / 12.0));
   });
   const Cks<T> m = metric();
-  const T igms = metric_rcp(m.sg);
+  const T igms = metric_rcp(m.sg), igms12 = igms * T(1.0 / 12.0);
 #pragma unroll
-  for (int a = 0; a < 3; ++a) rot[a] = pmul(rot[a], both(igms));
-  dvg = pmul(dvg, both(igms));
+  for (int a = 0; a < 3; ++a) rot[a] = pmul(rot[a], both(igms12));
+  dvg = pmul(dvg, both(igms12));
   const T divD = first(dvg), divB = second(dvg);
   Pair<T> db[3];  // (D, B)
 #pragma unroll
@@ -652,44 +653,37 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? COFFEE_GR_KO_MIN_BLOCKS 
   if (i >= c.hi[0] || j >= c.hi[1] || k >= c.hi[2]) return;
   const uint32_t sy = (uint32_t)c.d[0], sz = sy * (uint32_t)c.d[1];
   const uint32_t o = (uint32_t)i + sy * (uint32_t)j + sz * (uint32_t)k;
-  // 6th difference of all three axes: the weights of a neighbour at distance
-  // 1, 2, 3 are 15, -6, 1 and the point's own -60
   auto at = [&](const T* p, int ax, int n) {
     if (ax == 0) return __ldg(p + o + n);
     return __ldg(p + (uint32_t)(o + (uint32_t)n * (ax == 1 ? sy : sz)));
   };
+  // the 6th differences, one chain per axis from one end to the other, where the
+  // running sum stays below 10 fields (as sph_ko_point)
   Pair<T> db[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const T *pd = u.p[a], *pb = u.p[3 + a];
-    Pair<T> s1 = both((T)0), s2 = s1, s3 = s1;
+    Pair<T> t[3];
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
-      auto sum = [&](int n) {
-        return padd(pk(at(pd, ax, -n), at(pb, ax, -n)), pk(at(pd, ax, n), at(pb, ax, n)));
-      };
-      s1 = padd(s1, sum(1));
-      s2 = padd(s2, sum(2));
-      s3 = padd(s3, sum(3));
+      t[ax] = pk(at(pd, ax, -3), at(pb, ax, -3));
+#pragma unroll
+      for (int n = 1; n < 7; ++n)
+        t[ax] = pfma(pk(at(pd, ax, n - 3), at(pb, ax, n - 3)), both(diff6<T>(n)), t[ax]);
     }
-    const Pair<T> own = pk(__ldg(pd + o), __ldg(pb + o));
-    Pair<T> t = pfma(s2, both((T)-6), s3);
-    t = pfma(s1, both((T)15), t);
-    t = pfma(own, both((T)-60), t);
-    db[a] = pfma(t, both(c.ko_c), own);
+    db[a] = pfma(padd(padd(t[0], t[1]), t[2]), both(c.ko_c), pk(__ldg(pd + o), __ldg(pb + o)));
   }
   T P;
   {
     const T* p = u.p[6];
-    T s1 = 0, s2 = 0, s3 = 0;
+    T t[3];
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
-      s1 += at(p, ax, -1) + at(p, ax, 1);
-      s2 += at(p, ax, -2) + at(p, ax, 2);
-      s3 += at(p, ax, -3) + at(p, ax, 3);
+      t[ax] = at(p, ax, -3);
+#pragma unroll
+      for (int n = 1; n < 7; ++n) t[ax] = sfma(at(p, ax, n - 3), diff6<T>(n), t[ax]);
     }
-    const T own = __ldg(p + o);
-    P = sfma(sfma(own, (T)-60, sfma(s1, (T)15, sfma(s2, (T)-6, s3))), c.ko_c, own);
+    P = sfma(t[0] + t[1] + t[2], c.ko_c, __ldg(p + o));
   }
   const Cks<T> m =
       metric_at(c, mt, i, j, k, gr_pos(c, 0, i), gr_pos(c, 1, j), gr_pos(c, 2, k));
