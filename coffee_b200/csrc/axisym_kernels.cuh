@@ -25,15 +25,19 @@ enum AxiFlags { AX_LAST = 1, AX_AUX = 2, AX_WRITE_UN = 4 };
 // the kernels are latency-bound on their stencil loads, so more warps help,
 // until spilling costs more).  Measured, us a step: log-spherical 2048 x 1024 with 8
 // (32 registers) / 6 / 5 / 4: 554 / 496 / 506 / 522, 512 x 256 67 / 66 / 63 / 55; FP64
-// with 8 / 6 / 5 / 4 / 3: 1748 / 1203 / 987 / 893 / 984.  Batched runs (whose parameters
-// come from shared memory), us for four steps of eight, with 4 (64) / 5 / 6: 5053 / 4868
-// / 4924.  Cylindrical 1024 x 2048, us a step, stage and KO with 4 (64) and 4 / 3 and 5 / 5
-// and 3: 449 / 492 / 459; FP64 772 / 809 / 855.
+// with 8 / 6 / 5 / 4 / 3: 1748 / 1203 / 987 / 893 / 984.  Four batched runs (whose
+// parameters come from shared memory) with 4 (64) / 5 / 6: 863 / 832 / 809, the persistent
+// launch 1038 / 1056 / 1086; FP64 with 5 / 4 / 3 / 2: 1532 / 1425 / 1487 / 1711.
+// Cylindrical 1024 x 2048, stage and KO with 4 (64) and 4 / 3 and 5 / 5 and 3: 449 / 492
+// / 459; FP64 772 / 809 / 855.
 #ifndef COFFEE_SPH_MIN_BLOCKS
 #define COFFEE_SPH_MIN_BLOCKS 6
 #endif
 #ifndef COFFEE_SPH_MIN_BLOCKS_F64
 #define COFFEE_SPH_MIN_BLOCKS_F64 4
+#endif
+#ifndef COFFEE_SPH_BATCH_MIN_BLOCKS_F64
+#define COFFEE_SPH_BATCH_MIN_BLOCKS_F64 4
 #endif
 #ifndef COFFEE_SPH_BATCH_MIN_BLOCKS
 #define COFFEE_SPH_BATCH_MIN_BLOCKS 5
@@ -46,7 +50,9 @@ enum AxiFlags { AX_LAST = 1, AX_AUX = 2, AX_WRITE_UN = 4 };
 #endif
 template <typename T>
 constexpr int kSphMinBlocks = sizeof(T) == 4 ? COFFEE_SPH_MIN_BLOCKS : COFFEE_SPH_MIN_BLOCKS_F64;
-constexpr int kSphBatchMinBlocks = COFFEE_SPH_BATCH_MIN_BLOCKS;
+template <typename T>
+constexpr int kSphBatchMinBlocks =
+    sizeof(T) == 4 ? COFFEE_SPH_BATCH_MIN_BLOCKS : COFFEE_SPH_BATCH_MIN_BLOCKS_F64;
 constexpr int kCylStageMinBlocks = COFFEE_CYL_STAGE_MIN_BLOCKS;
 constexpr int kCylKoMinBlocks = COFFEE_CYL_KO_MIN_BLOCKS;
 
@@ -631,7 +637,7 @@ __device__ __forceinline__ const SphBatchEntry<T>& sph_batch_entry(
 }
 
 template <typename T, bool FIRST>
-__global__ void __launch_bounds__(256, kSphBatchMinBlocks) sph_stage_batch_kernel(
+__global__ void __launch_bounds__(256, kSphBatchMinBlocks<T>) sph_stage_batch_kernel(
     const SphBatchEntry<T>* __restrict__ tab, const int n, const int to_b,
     const T* __restrict__ tnow, const T* __restrict__ tdt, const T cs, const T As, const T Bs,
     const int last) {
@@ -650,7 +656,7 @@ __global__ void __launch_bounds__(256, kSphBatchMinBlocks) sph_stage_batch_kerne
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256, kSphBatchMinBlocks) sph_ko_batch_kernel(
+__global__ void __launch_bounds__(256, kSphBatchMinBlocks<T>) sph_ko_batch_kernel(
     const SphBatchEntry<T>* __restrict__ tab, const int n, const T* __restrict__ tnow,
     const T* __restrict__ tdt) {
   __shared__ __align__(16) unsigned char buf[sizeof(SphBatchEntry<T>)];
@@ -760,7 +766,7 @@ __device__ __forceinline__ bool grid_barrier(GridSync* gs, unsigned q, long long
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256, kSphBatchMinBlocks) sph_batch_persistent_kernel(
+__global__ void __launch_bounds__(256, kSphBatchMinBlocks<T>) sph_batch_persistent_kernel(
     const SphBatchEntry<T>* __restrict__ tab, const int n, const int nblocks,
     T* __restrict__ tbuf, const T* __restrict__ tdt, const LsrkCoef<T> k, const int nsteps,
     GridSync* __restrict__ gs, const long long limit_ns, const int stall_block) {
