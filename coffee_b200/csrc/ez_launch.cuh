@@ -128,8 +128,10 @@ void build_const(const coffee_env* env, int semantics, EzConst<T>* c) {
   c->check_egb = p.check_egb;
   c->semantics = semantics;
   c->taper_lanes = (sizeof(T) == 4) ? 16 : 8;  // AVX-512 width of the reference CPU build
-  // quotients by tau stay in the range of the straight-line division
-  c->tau_mid = std::fabs((double)c->tau) > 1e-6 && std::fabs((double)c->tau) < 1e6;
+  // Quotients by tau stay in the range of the straight-line division: a point's |P| is
+  // below 2^50 there, so that 2^64 P / tau, which it forms in FP32, stays below 2^127.
+  // (A step with a smaller tau diverges: P's decay rate is 1 / tau per stage.)
+  c->tau_mid = std::fabs((double)c->tau) >= 1.0 / 8192 && std::fabs((double)c->tau) < 1e6;
   c->problem = p.problem;
   bool abs_any = p.shift_ghost > 0;
   for (int a = 0; a < 3; ++a) {

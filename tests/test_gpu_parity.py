@@ -16,7 +16,7 @@ import pytest
 
 from coffee_b200 import problems
 from coffee_b200.solver import run_flat
-from helpers import (count_differing, fp32_parity, golden_cases, interior, load_golden,
+from helpers import (NAMES, count_differing, fp32_parity, golden_cases, interior, load_golden,
                      rel_l2, wide_box_case)
 from oracle import oracle
 
@@ -305,3 +305,19 @@ def test_flat_fp64_and_star_of_any_size(n, star):
         out, _ = run_flat(p, f, 2)
         for c in range(7):
             assert rel_l2(out[c], ref[c]) < 2e-5, NAMES[c]
+
+
+def test_p_over_tau_beyond_the_straight_line_range():
+    """P / tau of 2^64 and more, with P and tau each in the range of the
+    straight-line division: bit for bit, and finite, as the IEEE division gives it
+    (no cleaning, so that P moves nothing else)."""
+    p = problems.alfven_params(16)
+    p.divB_clean = False
+    p.tau = float(np.float32(6e-5))
+    f = problems.alfven_fields(p, np.float32)
+    f[6] = (1.12e15 * np.linspace(0.99, 1.0, f[6].size).reshape(f[6].shape)).astype(np.float32)
+    ref, _ = oracle.run_port(p, f, 1, semantics=0, taper_lanes=16)
+    out, _ = run_flat(p, f, 1)
+    assert np.isfinite(ref[6]).all()
+    for c in range(7):
+        assert count_differing(out[c], ref[c]) == 0, NAMES[c]
