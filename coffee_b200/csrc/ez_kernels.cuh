@@ -163,6 +163,36 @@ __device__ __forceinline__ void store_with_images(const GridGeom& g, const Colum
   }
 }
 
+// The guard images of a box with a periodic axis of fewer than 2 guard points, where a
+// point may have one beyond each face and store_with_images writes one of them: a pass
+// of its own after each stage and KO pass of such a box, so that the others pay nothing
+// (in store_with_images a third target cost a box of 128^3 4%).  Every guard point of a
+// periodic axis takes the value at its wrapped coordinates if the kernels update
+// that point; one thread per point, and no source is a target.
+template <typename T>
+__global__ void __launch_bounds__(256) ez_images_kernel(const GridGeom g, const F7<T> u) {
+  const long long n = g.sz * g.dims[2];
+  for (long long q = blockIdx.x * 256LL + threadIdx.x; q < n; q += gridDim.x * 256LL) {
+    const int k = (int)(q / g.sz), r = (int)(q - k * g.sz), j = r / g.dims[0];
+    int c[3] = {r - j * g.dims[0], j, k};
+    bool image = false, updated = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      if (g.periodic[a]) {
+        const int s = c[a] < g.guard[a] ? g.N[a] : c[a] >= g.dims[a] - g.guard[a] ? -g.N[a] : 0;
+        image = image || s != 0;
+        c[a] += s;
+      } else {
+        updated = updated && c[a] >= g.lo[a] && c[a] < g.hi[a];
+      }
+    }
+    if (!image || !updated) continue;
+    const long long o = c[2] * g.sz + c[1] * g.sy + c[0];
+#pragma unroll
+    for (int f = 0; f < 7; ++f) u.p[f][q] = u.p[f][o];
+  }
+}
+
 // Curl, divergence and gradient of the fields at one point, as the stage
 // needs them (all inv_delta-scaled 4th-order differences).
 template <typename T>

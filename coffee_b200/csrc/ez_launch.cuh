@@ -216,6 +216,7 @@ struct FlatLaunch {
   bool dg;   // and its energy-change diagnostics (xa only)
   // one point per thread (not with the diagnostics)
   bool direct_stage, direct_ko;
+  bool two_images;  // N < 2 guard on a periodic axis (ez_images_kernel)
   int kchunk_stage, kchunk_ko;
   dim3 grid_stage, grid_ko;
 };
@@ -354,6 +355,9 @@ inline int flat_plan(const coffee_env* env, int semantics, FlatLaunch* L,
   L->vec = env->grid.dims[0] % 2 == 0;
   L->xa = reference_arith && semantics == SEM_CPU_REF;
   L->dg = L->xa && energy_diag;
+  L->two_images = false;
+  for (int a = 0; a < 3; ++a)
+    if (env->p.periodic_boundary[a] && env->p.N[a] < 2 * env->p.guard[a]) L->two_images = true;
   // the shared-memory limits of the four kernel sets of this arithmetic (a
   // caller may still switch the pair copies off, as coffee_noalloc.cu does)
   if (L->dg) {
@@ -420,6 +424,15 @@ struct LaunchHook {
   virtual ~LaunchHook() {}
 };
 
+template <typename T>
+inline cudaError_t flat_images(const FlatLaunch& L, const GridGeom& g, const F7<T>& u,
+                               cudaStream_t st) {
+  if (!L.two_images) return cudaSuccess;
+  const long long n = g.sz * g.dims[2];
+  ez_images_kernel<T><<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(g, u);
+  return cudaGetLastError();
+}
+
 // nsteps evolve_fields calls from `time` (reference field_solver_EZ.cpp:1007-1073):
 // 5 stages A -> B -> A -> B -> A -> B, then the KO pass B -> A, advancing
 // time by dt in field precision after each step (src/main-alfven3d.cpp:61,119).
@@ -454,6 +467,7 @@ inline int flat_steps(const EzConst<T>& c, const FlatLaunch& L, const F7<T>& A, 
                            tst, flags);
       });
       COFFEE_CUDA_TRY(cudaGetLastError());
+      COFFEE_CUDA_TRY(flat_images(L, c.g, dst, st));
       if (hook) {
         int rc = hook->after(kind);
         if (rc) return rc;
@@ -467,6 +481,7 @@ inline int flat_steps(const EzConst<T>& c, const FlatLaunch& L, const F7<T>& A, 
     }
     with_flat_kernels<T>(L, [&](auto K) { decltype(K)::ko_pass(L, st, c, srcc, A, dgv, t + dt); });
     COFFEE_CUDA_TRY(cudaGetLastError());
+    COFFEE_CUDA_TRY(flat_images(L, c.g, A, st));
     if (hook) {
       int rc = hook->after(COFFEE_KERNEL_KO);
       if (rc) return rc;

@@ -321,3 +321,25 @@ def test_p_over_tau_beyond_the_straight_line_range():
     assert np.isfinite(ref[6]).all()
     for c in range(7):
         assert count_differing(out[c], ref[c]) == 0, NAMES[c]
+
+
+@pytest.mark.parametrize("n,periodic", [((3, 4, 5), (True, True, True)),
+                                        ((5, 9, 3), (True, False, True)),
+                                        ((3, 3, 40), (True, True, True)),
+                                        ((34, 4, 6), (False, True, True))])
+@pytest.mark.parametrize("energy_diag", [False, True])
+def test_periodic_axes_of_fewer_than_two_guard_widths(n, periodic, energy_diag):
+    """A point of such an axis has guard images on both sides: every point,
+    the guards of the periodic axes included, bit for bit, with both kinds of
+    kernels."""
+    p, f = _ragged_case((6, 6, 6))
+    p.N, p.size, p.periodic_boundary = list(n), [m / 32 for m in n], list(periodic)
+    rng = np.random.default_rng(5)
+    shape = tuple(m + 6 for m in reversed(n))
+    f = [(0.05 * rng.standard_normal(shape) + (1.0 if c == 3 else 0.0)).astype(np.float32)
+         for c in range(7)]
+    ref, _ = oracle.run_port(p, f, 2, semantics=0, taper_lanes=16)
+    out, _ = run_flat(p, f, 2, energy_diag=energy_diag)
+    box = tuple(slice(None) if q else slice(3, -3) for q in reversed(periodic))
+    for c in range(7):
+        assert count_differing(out[c][box], ref[c][box]) == 0, NAMES[c]
