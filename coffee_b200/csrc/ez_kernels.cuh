@@ -417,7 +417,10 @@ __device__ __forceinline__ void stage_values_pair(const EzConst<T>& c, const Pai
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const Pair<T> da = FIRST ? both((T)0) : pmul(dold[a], both(As));
-    const Pair<T> w = pk(xa::sub(second(rot[a]), J[a]), xa::fma(gradP[a], s, first(rot[a])));
+    // without the cleaning P may be anything (XA: a point of which w is not finite is
+    // done again)
+    const T gp = XA || c.divB_clean ? gradP[a] : (T)0;
+    const Pair<T> w = pk(xa::sub(second(rot[a]), J[a]), xa::fma(gp, s, first(rot[a])));
     d[a] = pfma(pdt, w, da);
     nu[a] = pfma(d[a], both(Bs), eb[a]);
   }

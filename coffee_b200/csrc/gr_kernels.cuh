@@ -426,7 +426,7 @@ __device__ __forceinline__ void gr_stage_point(const GrConst<T>& c, Metric&& met
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const T clean = kl * m.l[a] - m.alpha * Pd[a];
+    const T clean = c.divB_clean ? kl * m.l[a] - m.alpha * Pd[a] : T(0);
     Pair<T> d = pmul(pk(second(rot[a]) - J[a], sfma(clean, shape, -first(rot[a]))), both(dt));
     if constexpr (!FIRST) d = pfma(pk(du.p[a][o], du.p[3 + a][o]), both(As), d);
     du.p[a][o] = first(d);

@@ -343,3 +343,19 @@ def test_periodic_axes_of_fewer_than_two_guard_widths(n, periodic, energy_diag):
     box = tuple(slice(None) if q else slice(3, -3) for q in reversed(periodic))
     for c in range(7):
         assert count_differing(out[c][box], ref[c][box]) == 0, NAMES[c]
+
+
+@pytest.mark.parametrize("semantics,arithmetic", [("cpu", "reference"), ("cpu", "fast"),
+                                                  ("gpu", "reference")])
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_without_cleaning_p_moves_nothing(semantics, arithmetic, value):
+    """With divB_clean off E and B do not depend on P, also where P is not a
+    finite number."""
+    p, f = _ragged_case((33, 20, 9))
+    p.divB_clean = False
+    ref, _ = run_flat(p, f, 2, semantics=semantics, arithmetic=arithmetic)
+    f[6] = f[6].copy()
+    f[6][7, 11, 20] = value
+    out, _ = run_flat(p, f, 2, semantics=semantics, arithmetic=arithmetic)
+    for c in range(6):
+        assert count_differing(out[c], ref[c]) == 0, NAMES[c]

@@ -445,3 +445,18 @@ def test_gr_rounding():
     r = np.mean(r, 0)
     print(r)
     assert r[6] < 0.9125
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_gr_without_cleaning_p_moves_nothing(value):
+    """With divB_clean off D and B do not depend on P, also where P is not a
+    finite number."""
+    p = problems.wald_params(N=24, half_size=5.0, a=0.9, pml=4)
+    p.divB_clean = False
+    f = [a.astype(np.float32) for a in problems.wald_fields(p, np.float64)]
+    ref, _ = _run_ours(FieldSolverGrEZ, p, f, 2)
+    f[6] = f[6].copy()
+    f[6][9, 14, 20] = value
+    out, _ = _run_ours(FieldSolverGrEZ, p, f, 2)
+    for c in range(6):
+        assert np.array_equal(out[c], ref[c]), c
