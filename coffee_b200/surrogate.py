@@ -238,6 +238,8 @@ class UNet:
         lib = _lib.load()
         s = self._saved
         n, d, h, w, _ = dout.shape
+        if dout.data_ptr() % 16:  # the fused passes load 16 bytes at a time
+            dout = dout.clone()
 
         def dz_like(a):
             return torch.empty(a.shape, dtype=torch.bfloat16, device=self.dev)

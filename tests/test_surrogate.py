@@ -281,6 +281,26 @@ def test_network_gradients_match_oracle():
 
 
 @pytest.mark.gpu
+def test_backward_takes_a_gradient_at_any_address():
+    """dL/dout at an address that no 16-byte load can start from gives the same
+    gradients, bit for bit."""
+    from coffee_b200 import surrogate as sg
+    torch = _torch()
+    net = sg.UNet(seed=5)
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    out = net.forward(torch.randn(1, 4, 4, 6, 16, generator=gen, device="cuda").to(torch.bfloat16))
+    dout = torch.randn(out.shape, generator=gen, device="cuda")
+    net.backward(dout)
+    ref = [(L.gw.clone(), L.gb.clone()) for L in net.layers]
+    buf = torch.empty(out.numel() + 1, device="cuda")
+    moved = buf[1:].view(out.shape)
+    moved.copy_(dout)
+    net.backward(moved)
+    for L, (gw, gb) in zip(net.layers, ref):
+        assert torch.equal(L.gw, gw) and torch.equal(L.gb, gb)
+
+
+@pytest.mark.gpu
 def test_training_lowers_the_loss():
     """Adam on the library's kernels fits a smooth synthetic map."""
     from coffee_b200 import surrogate as sg
