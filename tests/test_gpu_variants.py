@@ -460,3 +460,33 @@ def test_gr_without_cleaning_p_moves_nothing(value):
     out, _ = _run_ours(FieldSolverGrEZ, p, f, 2)
     for c in range(6):
         assert np.array_equal(out[c], ref[c]), c
+
+
+@pytest.mark.parametrize("n", [(33, 30, 21), (40, 37, 52)])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_gr_matches_the_restatement(n, dtype):
+    """Boxes with ragged edges, both layers, the near-horizon table and calls
+    of one and several steps: FP64 to 1e-12 (some hundred roundings), FP32
+    within the FP32 restatement's own distance."""
+    p = problems.wald_params(N=40, half_size=5.0, a=0.9, pml=4)
+    d = p.size[0] / 40
+    p.N = list(n)
+    p.size, p.lower = [d * m for m in n], [-d * (m // 2 + 0.5) for m in n]
+    f64 = problems.wald_fields(p, np.float64)
+    U = np.stack(f64)
+    U[:6] += 0.02 * np.stack(_waves(p, np.random.default_rng(4), 3))[:6]
+    ref = gr_oracle.gr_evolve(p, U.astype(dtype).astype(np.float64), 4)
+    env = SimEnvironment(p)
+    data = SimData(env, dtype)
+    data.upload(list(U.astype(dtype)))
+    solver = FieldSolverGrEZ(data, env)
+    solver.step(0.0, 1)
+    solver.step(0.0, 3)
+    out = data.download()
+    for o in (solver, data, env):
+        o.close()
+    if dtype == np.float64:
+        assert max(rel_l2(out[c], ref[c]) for c in range(7)) < 1e-12
+    else:
+        ok, rep = fp32_parity(out, gr_oracle.gr_evolve(p, U.astype(dtype), 4), ref)
+        assert ok, rep
