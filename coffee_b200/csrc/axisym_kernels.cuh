@@ -128,7 +128,8 @@ struct Stencil2D {
   }
   __device__ __forceinline__ Pair<T> px(int a, int k) const { return pk(x(a, k), x(3 + a, k)); }
   __device__ __forceinline__ Pair<T> py(int a, int k) const { return pk(y(a, k), y(3 + a, k)); }
-  // sum of w[k] times the pair a at the four points of diff1_4, or with its own weights
+  // sum of w[k] times the pair a at the four points of diff1_4, or its own sum (before
+  // its 1 / 12) in its order
   __device__ __forceinline__ Pair<T> dx(int a, const T w[4]) const {
     Pair<T> t = pmul(px(a, -2), both(w[0]));
     t = pfma(px(a, -1), both(w[1]), t);
@@ -142,10 +143,10 @@ struct Stencil2D {
     return pfma(py(a, 2), both(w[3]), t);
   }
   __device__ __forceinline__ Pair<T> dx(int a) const {
-    return pfma(psub(px(a, 1), px(a, -1)), both(T(8)), psub(px(a, -2), px(a, 2)));
+    return psub(pfma(px(a, 1), both(T(8)), pfma(px(a, -1), both(T(-8)), px(a, -2))), px(a, 2));
   }
   __device__ __forceinline__ Pair<T> dy(int a) const {
-    return pfma(psub(py(a, 1), py(a, -1)), both(T(8)), psub(py(a, -2), py(a, 2)));
+    return psub(pfma(py(a, 1), both(T(8)), pfma(py(a, -1), both(T(-8)), py(a, -2))), py(a, 2));
   }
   __device__ __forceinline__ T dx1(int f) const {
     return sfma(T(8), x(f, 1) - x(f, -1), x(f, -2) - x(f, 2));
@@ -1033,9 +1034,10 @@ __global__ void __launch_bounds__(256, kCylStageMinBlocks) cyl_stage_kernel(cons
   T R = c.R0 + c.dR * (T)(i - c.g0);
   if (fabs(R) < Tiny<T>::v) R = Tiny<T>::v;
   // dfRdRR (:110-113): (R f)_R / R, 2 f_R on the axis, as the weights of diff1_4 times
-  // R at the four points.  Factors are kept out of the weights and of the single
-  // derivatives as in sph_stage_point (E_phi of a run was 2.3 times farther from 64 bits,
-  // B_z 5%).
+  // R at the four points.  The factors stay out of the weights, as in sph_stage_point (B_z
+  // of a run was 5% farther from 64 bits), and each difference is rounded as diff1_4
+  // rounds it, 1 / 12 before 1 / delta: beside the dipole's singularity two points decide
+  // the error of E_phi, and with 1 / 12 taken out of the curls it was 1.9 times that.
   const bool on_axis = fabs(R) < c.dR * T(0.25);
   const T iRR = on_axis ? T(2) * c.inv_dR : c.inv_dR / R;
   T wRR[4];
@@ -1043,12 +1045,12 @@ __global__ void __launch_bounds__(256, kCylStageMinBlocks) cyl_stage_kernel(cons
   for (int k = 0; k < 4; ++k)
     wRR[k] = diff4<T>(k) * (on_axis ? T(1) : R + T(k < 2 ? k - 2 : k - 1) * c.dR);
   // (rot E, rot B) along R, z, phi and (div E, div B)
-  Pair<T> rot[3] = {pmul(st.dy(2), both(-c.inv_dz)), pmul(st.dx(2, wRR), both(iRR)),
-                    pfma(st.dy(0), both(c.inv_dz), pmul(st.dx(1), both(-c.inv_dR)))};
-  Pair<T> dvg = pfma(st.dx(0, wRR), both(iRR), pmul(st.dy(1), both(c.inv_dz)));
-#pragma unroll
-  for (int a = 0; a < 3; ++a) rot[a] = pmul(rot[a], both(T(1.0 / 12.0)));
-  dvg = pmul(dvg, both(T(1.0 / 12.0)));
+  auto r12 = [](Pair<T> t) { return pmul(t, both(T(1.0 / 12.0))); };
+  const Pair<T> rot[3] = {
+      pmul(r12(st.dy(2)), both(-c.inv_dz)), pmul(r12(st.dx(2, wRR)), both(iRR)),
+      pfma(r12(st.dy(0)), both(c.inv_dz), pmul(r12(st.dx(1)), both(-c.inv_dR)))};
+  const Pair<T> dvg =
+      pfma(r12(st.dx(0, wRR)), both(iRR), pmul(r12(st.dy(1)), both(c.inv_dz)));
   const T divE = first(dvg), divB = second(dvg);
   Pair<T> eb[3];
 #pragma unroll
