@@ -104,6 +104,7 @@ SIGNATURES = {
     "coffee_solver_set_arithmetic": (_i, [_vp, _i]),
     "coffee_solver_set_taper_lanes": (_i, [_vp, _i]),
     "coffee_solver_set_energy_diag": (_i, [_vp, _i]),
+    "coffee_solver_set_streaming": (_i, [_vp, _i]),
     "coffee_solver_set_timing": (_i, [_vp, _i]),
     "coffee_solver_last_timing": (_i, [_vp, _P(_d), _P(_i), _P(_d)]),
     "coffee_fields_init_fourier": (_i, [_vp, _P(_d), _i, _P(_d), _P(_d), _P(_d), _i, _P(_d),

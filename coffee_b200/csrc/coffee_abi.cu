@@ -67,6 +67,7 @@ struct coffee_solver {
   int arith;    // COFFEE_ARITH_* of the flat solver
   int taper_lanes;  // SIMD lanes of the CPU build's taper (0: by precision)
   int energy_diag;  // the CPU build's energy-change diagnostics kept
+  int streaming;    // the plane-streaming kernels at every size
   uint64_t synced_generation;
   FlatLaunch launch;
   void* vtab;  // tables / scratch of a non-Cartesian variant (device), or null
@@ -560,7 +561,7 @@ extern "C" int coffee_fields_fill_guards(coffee_fields* f) {
 template <typename T>
 static int configure_solver(coffee_solver* s) {
   return flat_plan<T>(s->env, s->semantics, &s->launch, s->arith == COFFEE_ARITH_REFERENCE,
-                      s->energy_diag != 0);
+                      s->energy_diag != 0, s->streaming != 0);
 }
 
 extern "C" int coffee_solver_create(coffee_env* env, coffee_fields* f, int variant,
@@ -604,6 +605,7 @@ extern "C" int coffee_solver_create(coffee_env* env, coffee_fields* f, int varia
   s->arith = COFFEE_ARITH_REFERENCE;
   s->taper_lanes = 0;
   s->energy_diag = 0;
+  s->streaming = 0;
   s->events_used = 0;
   s->synced_generation = 0;
   // the GR solver's inner absorbing region always needs the start-of-step
@@ -742,6 +744,23 @@ extern "C" int coffee_solver_set_energy_diag(coffee_solver* s, int enable) {
   return rc;
 }
 
+extern "C" int coffee_solver_set_streaming(coffee_solver* s, int enable) {
+  clear_error();
+  if (!s) return fail(COFFEE_E_INVALID, "coffee_solver_set_streaming: null argument");
+  if (s->variant != COFFEE_VARIANT_FLAT)
+    return fail(COFFEE_E_INVALID, "only the flat EZ solver has a choice of kernels");
+  enable = enable ? 1 : 0;
+  if (enable == s->streaming) return COFFEE_OK;
+  COFFEE_CUDA_TRY(cudaSetDevice(s->env->device));
+  s->streaming = enable;
+  const int rc = (s->f->elem == 4) ? configure_solver<float>(s) : configure_solver<double>(s);
+  if (rc) {
+    s->streaming = 1 - enable;
+    (void)((s->f->elem == 4) ? configure_solver<float>(s) : configure_solver<double>(s));
+  }
+  return rc;
+}
+
 extern "C" int coffee_solver_set_taper_lanes(coffee_solver* s, int lanes) {
   clear_error();
   if (!s) return fail(COFFEE_E_INVALID, "coffee_solver_set_taper_lanes: null argument");
@@ -768,7 +787,9 @@ extern "C" int coffee_solver_launches_per_step(coffee_solver* s) {
   if (s && s->variant == COFFEE_VARIANT_GRYEE)
     // E, H + rho + shell + update + clamp per substep, and the cleaning
     return 15 + (s->env->p.clean_ep ? 1 : 0);
-  return 6;  // 5 stage kernels + 1 KO kernel
+  // 5 stage kernels + 1 KO kernel (each with a pass over the guard images where a
+  // periodic axis has fewer than two guard widths)
+  return s && s->variant == COFFEE_VARIANT_FLAT && s->launch.two_images ? 12 : 6;
 }
 
 static int next_event_pair(coffee_solver* s, int kind, cudaEvent_t* a, cudaEvent_t* b) {

@@ -346,10 +346,12 @@ inline void with_flat_kernels(const FlatLaunch& L, Fn&& fn) {
 // reference_arith: the CPU semantics run in the CPU build's own arithmetic
 // (the default); false selects the regrouped, faster arithmetic.
 // energy_diag: with the reference arithmetic, also accumulate the CPU
-// build's energy-change diagnostics.
+// build's energy-change diagnostics.  streaming: the plane-streaming kernels at every
+// size (where there are any).
 template <typename T>
 inline int flat_plan(const coffee_env* env, int semantics, FlatLaunch* L,
-                     bool reference_arith = true, bool energy_diag = false) {
+                     bool reference_arith = true, bool energy_diag = false,
+                     bool streaming = false) {
   using S = Shape<T>;
   L->bc = flat_needs_bc(env->p, semantics);
   L->vec = env->grid.dims[0] % 2 == 0;
@@ -412,8 +414,8 @@ inline int flat_plan(const coffee_env* env, int semantics, FlatLaunch* L,
   L->grid_ko = dim3(kx, ky, (box[2] + L->kchunk_ko - 1) / L->kchunk_ko);
   const long long pts = (long long)box[0] * box[1] * box[2];
   const DirectPoints dp = direct_points<T>(L->bc, L->xa);
-  L->direct_stage = !L->dg && pts <= dp.stage;
-  L->direct_ko = !L->dg && pts <= dp.ko;
+  L->direct_stage = !L->dg && !streaming && pts <= dp.stage;
+  L->direct_ko = !L->dg && !streaming && pts <= dp.ko;
   return COFFEE_OK;
 }
 

@@ -114,13 +114,11 @@ __device__ __forceinline__ Pair<T> pdot3(const Pair<T> a[3], const Pair<T> b[3])
 // end.  Numerators are scaled by 2^64 first, so that their residuals are
 // exact however small they are (FP32); a quotient below 2^-124 is left to the
 // IEEE division, whose rounding of it is to a subnormal number.
-// Compared with the IEEE intrinsics on a B200: every FP32 reciprocal and root
-// mantissa; for every FP32 divisor all the quotients within 16/b of a rounding
-// boundary (7e8 of them; a quotient farther away cannot be misrounded by the
-// correction, which is off by less than 2^-23 of an ulp); 9e8 random quotients
-// and roots of both precisions: no difference.  The FP64 reciprocal of the
-// one mantissa that is all ones is an ulp off (as the paper says), and then
-// quotients within 2^-53 of a boundary are, too.
+// Compared with the IEEE operations on the GPU (tests/cuda/pair_check.cu): every FP32
+// reciprocal and root mantissa, 6e8 FP32 quotients beside rounding boundaries and 2e8
+// random ones, 3e8 roots, 1e8 FP64 quotients and 6e7 roots: no difference, but for -0 / b,
+// which is +0 here.  The FP64 reciprocal of the one mantissa that is all ones is an ulp
+// off (as the paper says), and then quotients within 2^-53 of a boundary are, too.
 template <typename T> struct MidRange;
 template <> struct MidRange<float> {
   static constexpr float den_max = 1073741824.0f;             // 2^30

@@ -219,6 +219,11 @@ class FieldSolverEZ:
         dU_KO and their _cum sums (SimData.download(_lib.ENERGY_DIAG_NAMES))."""
         check(self.lib.coffee_solver_set_energy_diag(self.handle, int(bool(enable))))
 
+    def set_streaming(self, enable: bool):
+        """Run the kernels that stream along z also on grids for which those of
+        one point per thread are the faster choice (to compare the two)."""
+        check(self.lib.coffee_solver_set_streaming(self.handle, int(bool(enable))))
+
     def set_taper_lanes(self, lanes: int):
         """SIMD width of the CPU build's P-gradient taper offsets (0: by
         precision, 16 for float and 8 for double as in the reference's two

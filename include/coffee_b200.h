@@ -246,6 +246,11 @@ COFFEE_API int coffee_solver_set_arithmetic(coffee_solver* s, int mode);
  * data_exporter.cpp:633-638).  Computed in the CPU build's own arithmetic:
  * flat solver, CPU semantics, COFFEE_ARITH_REFERENCE only. */
 COFFEE_API int coffee_solver_set_energy_diag(coffee_solver* s, int enable);
+/* Run the kernels that stream along z (1) also where the choice by grid size would
+ * take those of one point per thread (0, the default: the faster ones), so that both
+ * can be compared on one grid.  The FP32 stage of a star or absorbing layer in the
+ * reference arithmetic has one kernel at every size.  Flat solver only. */
+COFFEE_API int coffee_solver_set_streaming(coffee_solver* s, int enable);
 /* The SIMD width by which the CPU build's P-gradient taper offsets a point's
  * x, y and z (field_solver_EZ.cpp:222-224): 16 in its float build, 8 in its
  * double build (AVX-512), so the two builds differ in more than rounding.

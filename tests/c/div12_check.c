@@ -1,8 +1,10 @@
-/* Exhaustive check of the single-precision division by 12 used by the
- * reference-arithmetic kernels (coffee_b200/csrc/ez_refarith.cuh,
- * xa::div12_fast): q = t * (1/12), e = fma(q, 12, -t) (the exact residual
- * 12 q - t), q' = fma(e, -1/12, q).  For every finite float t it compares
- * q' with the IEEE quotient t / 12, bit for bit, and counts the mismatches
+/* Exhaustive check of the single-precision divisions by 12 of the
+ * reference-arithmetic kernels: q = t * (1/12), then either e = fma(q, 12, -t)
+ * (the exact residual 12 q - t) and q' = fma(e, -1/12, q) (xa::div12_fast of
+ * coffee_b200/csrc/ez_refarith.cuh, the fallback) or e = fma(q, -12, t) and q' =
+ * fma(e, 1/12, q) (pd1_4 of ez_kernels.cuh, the stages; of t = -0 it makes +0).
+ * For every finite float t it compares both with the IEEE quotient t / 12, bit
+ * for bit but for that zero, and counts the mismatches
  * inside and outside the range 0 < |t| < 2^-124 that the kernels send to
  * the IEEE division.  It also checks the kernels' integer test of that
  * range, key(t) = 2 bits(t) - 1 (mod 2^32) < 0x02FFFFFE, against the
@@ -31,10 +33,14 @@ int main(void) {
     float q = t * r12;
     const float e = fmaf(q, 12.0f, -t);
     q = fmaf(e, -r12, q);
-    uint32_t a1, a2;
+    const float q0 = t * r12;
+    const float s = fmaf(fmaf(q0, -12.0f, t), r12, q0);
+    uint32_t a1, a2, a3;
     memcpy(&a1, &ref, 4);
     memcpy(&a2, &q, 4);
-    if (a1 != a2) {
+    memcpy(&a3, &s, 4);
+    if (t == 0.0f && a3 == 0) a3 = a1;
+    if (a1 != a2 || a1 != a3) {
       if (in_range) ++inside;
       else ++outside;
     }

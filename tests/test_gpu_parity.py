@@ -15,7 +15,7 @@ import numpy as np
 import pytest
 
 from coffee_b200 import problems
-from coffee_b200.solver import run_flat
+from coffee_b200.solver import FieldSolverEZ, SimData, SimEnvironment, run_flat
 from helpers import (NAMES, count_differing, fp32_parity, golden_cases, interior, load_golden,
                      rel_l2, wide_box_case)
 from oracle import oracle
@@ -359,3 +359,55 @@ def test_without_cleaning_p_moves_nothing(semantics, arithmetic, value):
     out, _ = run_flat(p, f, 2, semantics=semantics, arithmetic=arithmetic)
     for c in range(6):
         assert count_differing(out[c], ref[c]) == 0, NAMES[c]
+
+
+def _run_kernels(p, f, streaming, semantics="cpu", arithmetic="reference"):
+    env = SimEnvironment(p)
+    data = SimData(env, f[0].dtype)
+    data.upload(f)
+    solver = FieldSolverEZ(data, env, semantics)
+    solver.set_arithmetic(arithmetic)
+    solver.set_streaming(streaming)
+    solver.set_aux(True)
+    solver.step(0.0, 2)
+    out = data.download() + data.download(("Jx", "Jy", "Jz", "divE", "divB"))
+    for o in (solver, data, env):
+        o.close()
+    return out
+
+
+# rows of odd and even length, a partial last tile in x and y, one z chunk and several
+# with a partial last group of planes
+@pytest.mark.parametrize("n", [(33, 20, 9), (40, 42, 41), (37, 17, 131), (64, 29, 72)])
+@pytest.mark.parametrize("star", [False, True])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("semantics,arithmetic", [("cpu", "reference"), ("cpu", "fast"),
+                                                  ("gpu", "reference")])
+def test_streaming_kernels_on_small_grids(n, star, dtype, semantics, arithmetic):
+    """The streaming kernels, which larger grids run, against those of one point
+    per thread, which small ones run: bit for bit in the reference arithmetic; in
+    the regrouped one within the roundings of two steps: some tens of 2^-24 or
+    2^-53, relative L2, and 100 times that for J, the divergences and P, which with
+    the star is a sum of div B from 0 on: each is a difference of terms of |B| / dx
+    that cancel to the dipole's truncation error, 1e-2 of them."""
+    p, f = _ragged_case(n, star=star, dtype=dtype)
+    a = _run_kernels(p, f, False, semantics, arithmetic)
+    b = _run_kernels(p, f, True, semantics, arithmetic)
+    eps = 2e-6 if dtype == np.float32 else 2e-14
+    for c in range(12):
+        if arithmetic == "reference" and semantics == "cpu":
+            assert count_differing(a[c], b[c]) == 0, c
+        else:
+            assert rel_l2(a[c], b[c]) < (eps if c < 6 else 100 * eps), c
+
+
+def test_energy_diagnostics_with_a_star():
+    """The FP32 stage kernel of runs with both the boundary code and the
+    diagnostics gives the fields of a run without the diagnostics, bit for bit."""
+    for n in ((40, 42, 41), (37, 30, 70)):
+        p, f = _ragged_case(n, star=True)
+        a, _ = run_flat(p, f, 2)
+        b, dg = run_flat(p, f, 2, energy_diag=True)
+        for c in range(7):
+            assert count_differing(a[c], b[c]) == 0, NAMES[c]
+        assert all(np.isfinite(d).all() for d in dg)
