@@ -50,9 +50,8 @@ __device__ __forceinline__ T d1_4(T m2, T m1, T p1, T p2, T s) {
 // The same of both fields of a pair.  XA: diff1_4 of the reference
 // (finite_diff_simd.h:15-25) before its inv_delta factor, the division by 12
 // as q = t / 12 (RN), q + (t - 12 q) / 12, its input noted in `g`: the IEEE quotient of
-// every t (tests/c/div12_check.c, tests/cuda/pair_check.cu) but -0, of which it makes +0.
-// No field can tell: a -0 enters a sum with +0 there, and the dissipation that ends a
-// step leaves no -0.
+// every t (tests/c/div12_check.c, tests/cuda/pair_check.cu) but -0, of which it makes +0
+// (where results are called the same bit for bit, 0 and -0 are one value).
 template <bool XA, typename T>
 __device__ __forceinline__ Pair<T> pd1_4(Pair<T> m2, Pair<T> m1, Pair<T> p1, Pair<T> p2,
                                          const T inv12, Guard<T>& g) {
