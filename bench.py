@@ -740,7 +740,7 @@ def run_variant(args):
                 "achieved": BYTES_STEP * cells / (step_ms / 1e3) / 1e9, "peak": peak,
                 "unit": "GB/s", "peak_kind": peak_kind, "traffic": None,
                 "algorithmic_bytes_per_step": BYTES_STEP * cells}
-        launches = 13 * args.steps + 1
+        launches = 7 * args.steps + 1
         launch_note = ("5 stage + 1 KO + 1 time-advance per step (one captured "
                        "CUDA graph, replayed per step), 1 axis per call")
         cfg["autotuned"] = batch.info()

@@ -156,12 +156,6 @@ struct Stencil2D {
   }
 };
 
-template <typename T>
-__device__ __forceinline__ T d1_4w(T a0, T a1, T a3, T a4) {
-  // diff1_4 (src/algorithms/finite_diff.h:14-19)
-  return (a0 - T(8) * a1 + T(8) * a3 - a4) * T(1.0 / 12.0);
-}
-
 // ---- log-spherical helpers ----------------------------------------------
 // wpert_sph_angle (field_solver_EZ_spherical.cu:576-595)
 template <typename T>

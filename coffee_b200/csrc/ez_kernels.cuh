@@ -49,9 +49,11 @@ __device__ __forceinline__ T d1_4(T m2, T m1, T p1, T p2, T s) {
 
 // The same of both fields of a pair.  XA: diff1_4 of the reference
 // (finite_diff_simd.h:15-25) before its inv_delta factor, the division by 12
-// as q = t / 12 (RN), q + (t - 12 q) / 12, its input noted in `g`: the IEEE quotient of
-// every t (tests/c/div12_check.c, tests/cuda/pair_check.cu) but -0, of which it makes +0
-// (where results are called the same bit for bit, 0 and -0 are one value).
+// as q = t (1/12), q + (t - 12 q) (1/12) with the exact residual, t noted in `g`.  This
+// is the IEEE quotient of every float but 0 < |t| < 2^-124, whose quotient is subnormal
+// and which the guard finds, and -0, of which it makes +0 (where results are called the
+// same bit for bit, 0 and -0 are one value): tests/c/div12_check.c,
+// tests/cuda/pair_check.cu.
 template <bool XA, typename T>
 __device__ __forceinline__ Pair<T> pd1_4(Pair<T> m2, Pair<T> m1, Pair<T> p1, Pair<T> p2,
                                          const T inv12, Guard<T>& g) {
@@ -89,8 +91,9 @@ __device__ __forceinline__ T d6_2(T m3, T m2, T m1, T c, T p1, T p2, T p3) {
   return ((m3 + p3) - (T)6 * (m2 + p2)) + ((T)15 * (m1 + p1) - (T)20 * c);
 }
 
-// The same of both fields of a pair; XA: the reference's order and fused terms
-// (xa::d6).
+// The same of both fields of a pair; XA: diff6_2 of the reference
+// (finite_diff_simd.h:41-58), each weighted term fused into the running sum, f+3 added
+// last.
 template <bool XA, typename T>
 __device__ __forceinline__ Pair<T> pd6_2(Pair<T> m3, Pair<T> m2, Pair<T> m1, Pair<T> c, Pair<T> p1,
                                          Pair<T> p2, Pair<T> p3) {
@@ -300,8 +303,7 @@ __device__ __noinline__ Derivs<T> point_derivatives_ieee(const EzConst<T>& c,
     const T* p = uin.p[f] + o;
     for (int a = 0; a < 3; ++a) {
       const long long t = st[a];
-      uint32_t unused = 0xFFFFFFFFu;
-      g[f][a] = xa::dq<true>(p[-2 * t], p[-t], p[t], p[2 * t], unused);
+      g[f][a] = xa::dq(p[-2 * t], p[-t], p[t], p[2 * t]);
     }
   }
   const T ix = c.inv_delta[0], iy = c.inv_delta[1], iz = c.inv_delta[2];
@@ -322,7 +324,8 @@ __device__ __noinline__ Derivs<T> point_derivatives_ieee(const EzConst<T>& c,
 
 // The same stage of one point from global memory, out of line: for the rare
 // points whose operands the straight-line arithmetic of stage_values_pair
-// does not cover (Guard).
+// does not cover (Guard).  Were all points of that kind (fields below 2^-124 on a uniform
+// B), a step of 512^3 would take 137 ms instead of 25, of 128^3 1.74 instead of 0.50.
 template <bool FIRST, typename T>
 __device__ __noinline__ StageValues<T> stage_point_ieee(const EzConst<T>& c, const F7<const T> uin,
                                                         const F7<T> du, const ColumnCtx<T> col,
@@ -608,8 +611,8 @@ struct PairLoader {
 // reading U from `uin` and writing U' (with guard images) to `uout`.
 //
 // This is the FP64 kernel (and the FP32 one of runs with both the boundary code and the
-// diagnostics).  The ring of 5 + PF + SPARE planes (k-2 .. k+2, the prefetch, a spare
-// that saves the second barrier) holds the whole stencil as pairs, read at
+// diagnostics: 256^3 with the star, 7345 us a step with the register window, 6230 here).
+// The ring of 5 + PF planes (k-2 .. k+2, the prefetch) holds the whole stencil as pairs, read at
 // compile-time offsets; with the z neighbours in the ring instead of a register
 // window a thread's registers hold one point only, which in FP64 lets 12 warps of 168
 // registers share an SM.  FP64 stage at 256^3: 2610 us with a register window, 4 warps
@@ -617,15 +620,14 @@ struct PairLoader {
 // dependent FP64 operations.  The old dU of a point is loaded at the top of its plane
 // and used after the derivatives.
 // ---------------------------------------------------------------------------
-template <typename T, int TX, int TY, int PF, int SPARE>
+template <typename T, int TX, int TY, int PF>
 constexpr size_t stage_smem_bytes() {
-  return (size_t)(5 + PF + SPARE) * PairLoader<T, TX, TY, 2>::SB;
+  return (size_t)(5 + PF) * PairLoader<T, TX, TY, 2>::SB;
 }
 
 // DG (with XA only): also accumulate the CPU build's energy-change
 // diagnostics of the clamps into dg.
-template <typename T, int TX, int TY, int PF, int SPARE, int MINB, bool FIRST, bool BC, bool XA,
-          bool DG>
+template <typename T, int TX, int TY, int PF, int MINB, bool FIRST, bool BC, bool XA, bool DG>
 __global__ void __launch_bounds__(TX * TY, MINB)
     ez_stage_kernel(const __grid_constant__ EzConst<T> c, const F7<const T> uin,
                     const F7<T> uout, const F7<T> du, const F7<T> un, const F5<T> aux,
@@ -633,7 +635,7 @@ __global__ void __launch_bounds__(TX * TY, MINB)
                     const int flags) {
   static_assert(XA || !DG, "the energy diagnostics need the reference arithmetic");
   using L = PairLoader<T, TX, TY, 2>;
-  constexpr int R = 5 + PF + SPARE;  // ring slots
+  constexpr int R = 5 + PF;  // ring slots
   constexpr int ES = (int)sizeof(T), SX = L::SX, PB = L::PB, SB = L::SB;
   constexpr int CEN = (2 * SX + 2) * 2 * ES;  // own pair, from the corner of its 5 x 5 patch
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -678,7 +680,6 @@ __global__ void __launch_bounds__(TX * TY, MINB)
       const uint32_t s = head + (uint32_t)(q * SB);
       return s >= (uint32_t)(R * SB) ? s - (uint32_t)(R * SB) : s;
     };
-    if constexpr (SPARE == 1) issue(k + 3 + PF, slot(5 + PF));  // into the slot of plane k-3
     if (active) {
       const uint32_t o = (uint32_t)k * sz + own;
       Pair<T> dold[3];
@@ -795,10 +796,8 @@ __global__ void __launch_bounds__(TX * TY, MINB)
         stage_finish<BC>(c, u, d7, n7, J, divE, divB, tst, flags, col, k, o, du, un, aux, uout);
       }
     }
-    if constexpr (SPARE == 0) {
-      __syncthreads();
-      issue(k + 3 + PF, slot(5 + PF));  // into the slot of plane k-2
-    }
+    __syncthreads();
+    issue(k + 3 + PF, head);  // into the slot of plane k-2
     head = slot(1);
   }
   cp_async_wait<0>();

@@ -39,9 +39,6 @@ template <typename T> struct Shape;
 #ifndef COFFEE_F32_SPF
 #define COFFEE_F32_SPF 1
 #endif
-#ifndef COFFEE_F32_SPARE
-#define COFFEE_F32_SPARE 0
-#endif
 #ifndef COFFEE_F32_SMINB
 #define COFFEE_F32_SMINB 2
 #endif
@@ -52,13 +49,13 @@ template <typename T> struct Shape;
 #define COFFEE_F32_KPF 1
 #endif
 template <> struct Shape<float> {
-  // stage tile, planes of prefetch, spare ring slots, resident CTAs per SM
+  // stage tile, planes of prefetch, resident CTAs per SM
   static constexpr int STX = 32, STY = COFFEE_F32_STY, SPF = COFFEE_F32_SPF;
-  static constexpr int SSPARE = COFFEE_F32_SPARE, SMINB = COFFEE_F32_SMINB;
+  static constexpr int SMINB = COFFEE_F32_SMINB;
   static constexpr int KTX = 32, KTY = COFFEE_F32_KTY, KPF = COFFEE_F32_KPF;  // KO tile, prefetch
 };
 template <> struct Shape<double> {
-  static constexpr int STX = 32, STY = 12, SPF = 1, SSPARE = 0, SMINB = 1;
+  static constexpr int STX = 32, STY = 12, SPF = 1, SMINB = 1;
   static constexpr int KTX = 32, KTY = 4, KPF = 1;
 };
 
@@ -193,8 +190,9 @@ inline bool flat_needs_bc(const coffee_params& p, int semantics) {
 // 128^3 76 / 76, 192^3 226 / 202; regrouped arithmetic, stage and KO 96^3 38 + 37 / 43
 // + 35, 128^3 85 + 87 / 79 + 76; FP64 stage 160^3 360 / 372, 256^3 1418 / 1320, KO
 // 256^3 978 / 1044.  With the boundary code the stage in the reference arithmetic is
-// faster at every size (192^3 298 / 421, 384^3 2264 / 2370, 512^3 5807 / 5732: the only
-// one), its KO pass up to 384^3 (1762 / 1790; 512^3 4538 / 3793), the regrouped ones
+// faster up to 450^3 (192^3 298 / 421, 384^3 2264 / 2370) and within the runs' spread at
+// 512^3 (5807 / 5732; whole steps 32.4 / 32.2 ms, +- 0.4): the only one.  Its KO pass is
+// faster up to 384^3 (1762 / 1790; 512^3 4538 / 3793), the regrouped ones
 // below 256^3 (192^3 300 + 271 / 334 + 317, 256^3 681 + 619 / 586 + 521).
 struct DirectPoints {
   long long stage, ko;
@@ -224,8 +222,9 @@ struct FlatLaunch {
 template <typename T, bool BC, int V, bool XA, bool DG = false>
 struct FlatKernels {
   using S = Shape<T>;
-  // the stage kernel: the register window in FP32 without the boundary code and
-  // the diagnostics, else the plane ring
+  // the stage kernel: in FP32 the register window, but for the boundary code in the
+  // reference arithmetic, which has one point per thread at every size and, with the
+  // diagnostics, the plane ring; in FP64 the plane ring
   static constexpr bool kFloat = std::is_same<T, float>::value;
   static constexpr bool kDirectOnly = kFloat && BC && XA && !DG;  // the stage kernel
   static constexpr bool kWindow = kFloat && !(BC && XA);
@@ -237,11 +236,11 @@ struct FlatKernels {
     if constexpr (kWindow)
       return ez_stage_window_kernel<T, kTileX, kTileY, S::SPF, kZU, FIRST, BC, V, XA, DG>;
     else
-      return ez_stage_kernel<T, S::STX, S::STY, S::SPF, S::SSPARE, S::SMINB, FIRST, BC, XA, DG>;
+      return ez_stage_kernel<T, S::STX, S::STY, S::SPF, S::SMINB, FIRST, BC, XA, DG>;
   }
   static constexpr size_t stage_bytes(bool first) {
     if constexpr (kWindow) return window_smem_bytes<T, kTileX, kTileY, S::SPF, V>(first);
-    else return stage_smem_bytes<T, S::STX, S::STY, S::SPF, S::SSPARE>();
+    else return stage_smem_bytes<T, S::STX, S::STY, S::SPF>();
   }
   static constexpr auto ko_fn() {
     return ez_ko_kernel<T, S::KTX, S::KTY, S::KPF, BC, V, XA, DG>;

@@ -405,7 +405,7 @@ __device__ __forceinline__ int periodic_targets(const GridGeom& g, int axis, int
   if (self) { out[0] = i; n = 1; }
   if (up) { if (n == 0) out[0] = i + N; else out[1] = i + N; ++n; }
   if (down) { if (n == 0) out[0] = i - N; else out[1] = i - N; ++n; }
-  return n < 2 ? n : 2;  // (three only where N < 2 guard)
+  return n < 2 ? n : 2;  // (three where N < 2 guard: ez_images_kernel, yee_guard_kernel)
 }
 
 // True when index i along `axis` has no periodic guard image and is not a

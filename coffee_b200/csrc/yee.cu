@@ -148,7 +148,7 @@ int yee_steps_t(const coffee_env* env, void* const A[7], void* const B0[3], void
   T t = (T)time;
   // with every axis periodic each guard point is the image of an interior
   // point, which the clamp pass writes: nothing is left for a guard pass
-  // (256^3: 0.70 ms a call saved).  On an axis of fewer than 2 guard points a
+  // (256^3: 0.70 ms a call saved).  On an axis of fewer than two guard widths a
   // point has images on both sides, of which that pass writes one: there the
   // guard pass follows every substep.
   bool guards_synced = a.g.periodic[0] && a.g.periodic[1] && a.g.periodic[2];

@@ -94,7 +94,9 @@ COFFEE_API int coffee_bias_grad(const float* dz, long long npts, int k, float* d
  * 16-byte aligned.  up2: da is the gradient of a 2x nearest upsampling, channels
  * off .. off + c of dy (cy channels at twice the grid n, d, h, w).  skip_pool2:
  * da is channels off .. off + c of dcat (ccat channels) plus the gradient of a 2x
- * average pooling, dp at half the grid. */
+ * average pooling, dp at half the grid.  All three keep their partial sums in the
+ * device's one array of coffee_bias_grad: calls of any of the four that could overlap
+ * on the GPU (other streams, other host threads) must not share a device. */
 COFFEE_API int coffee_leaky_bias_backward(const float* da, const void* a, long long npts, int c,
                                           float slope, void* dz_bf16, float* db, void* stream);
 COFFEE_API int coffee_up2_leaky_bias_backward(const float* dy, int n, int d, int h, int w, int c,

@@ -1,8 +1,9 @@
 /* Exhaustive check of the single-precision divisions by 12 of the
- * reference-arithmetic kernels: q = t * (1/12), then either e = fma(q, 12, -t)
- * (the exact residual 12 q - t) and q' = fma(e, -1/12, q) (xa::div12_fast of
- * coffee_b200/csrc/ez_refarith.cuh, the fallback) or e = fma(q, -12, t) and q' =
- * fma(e, 1/12, q) (pd1_4 of ez_kernels.cuh, the stages; of t = -0 it makes +0).
+ * reference-arithmetic kernels: q = t * (1/12), then either e = fma(q, -12, t)
+ * (the exact residual t - 12 q) and q' = fma(e, 1/12, q) (pd1_4 of
+ * coffee_b200/csrc/ez_kernels.cuh, the stages; of t = -0 it makes +0) or e =
+ * fma(q, 12, -t) and q' = fma(e, -1/12, q) (xa::div12 of ez_refarith.cuh, the
+ * points outside the stages' range).
  * For every finite float t it compares both with the IEEE quotient t / 12, bit
  * for bit but for that zero, and counts the mismatches
  * inside and outside the range 0 < |t| < 2^-124 that the kernels send to
@@ -30,16 +31,14 @@ int main(void) {
     if (in_range != key_says) ++key;
     if (!isfinite(t)) continue;
     const float ref = t / 12.0f;
-    float q = t * r12;
-    const float e = fmaf(q, 12.0f, -t);
-    q = fmaf(e, -r12, q);
-    const float q0 = t * r12;
-    const float s = fmaf(fmaf(q0, -12.0f, t), r12, q0);
+    const float q = t * r12;
+    const float s = fmaf(fmaf(q, -12.0f, t), r12, q);
+    const float d = fmaf(fmaf(q, 12.0f, -t), -r12, q);
     uint32_t a1, a2, a3;
     memcpy(&a1, &ref, 4);
-    memcpy(&a2, &q, 4);
-    memcpy(&a3, &s, 4);
-    if (t == 0.0f && a3 == 0) a3 = a1;
+    memcpy(&a2, &s, 4);
+    memcpy(&a3, &d, 4);
+    if (t == 0.0f && a2 == 0) a2 = a1;
     if (a1 != a2 || a1 != a3) {
       if (in_range) ++inside;
       else ++outside;

@@ -446,3 +446,54 @@ def test_fused_backward_passes_match_torch(c, shape):
     for ax in (1, 2, 3):
         x = x.repeat_interleave(2, ax)
     assert torch.equal(y, torch.cat([x, a], -1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c,shape", [(8, (1, 2, 2, 2)), (16, (2, 4, 6, 10)), (5, (1, 2, 4, 6))])
+def test_single_elementwise_passes_match_torch(c, shape):
+    """The library's elementwise passes that the network runs fused: copies and
+    sums of two values exact, sums of eight within 8 roundings of 2^-24."""
+    import torch
+
+    from coffee_b200 import _lib
+    from coffee_b200 import surrogate as sg
+
+    lib = _lib.load()
+    n, d, h, w = shape
+    gen = torch.Generator(device="cuda").manual_seed(c)
+    ptr, stream, npts = sg._ptr, sg._stream(), n * d * h * w
+
+    def rnd(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+
+    da, z = rnd(n, d, h, w, c), rnd(n, d, h, w, c)
+    dz, dzb = torch.empty_like(da), torch.empty(da.shape, dtype=torch.bfloat16, device="cuda")
+    sg.check(lib.coffee_leaky_backward(ptr(da), ptr(z), da.numel(), 0.1, ptr(dz), ptr(dzb), stream))
+    ref = da * torch.where(z > 0, 1.0, 0.1)
+    assert torch.equal(dz, ref) and torch.equal(dzb, ref.to(torch.bfloat16))
+    dp, dx = rnd(n, d // 2, h // 2, w // 2, c), rnd(n, d, h, w, c)
+    ref = dx.clone()
+    sg.check(lib.coffee_pool2_backward_add(ptr(dp), n, d, h, w, c, ptr(dx), stream))
+    up = dp
+    for ax in (1, 2, 3):
+        up = up.repeat_interleave(2, ax)
+    assert torch.equal(dx, ref + up * 0.125)
+    x = rnd(n, d, h, w, c).to(torch.bfloat16)
+    y = torch.zeros(n, 2 * d, 2 * h, 2 * w, c + 3, dtype=torch.bfloat16, device="cuda")
+    sg.check(lib.coffee_up2_forward(ptr(x), n, d, h, w, c, ptr(y), c + 3, 2, stream))
+    up = x
+    for ax in (1, 2, 3):
+        up = up.repeat_interleave(2, ax)
+    assert torch.equal(y[..., 2:2 + c], up) and not y[..., :2].any() and not y[..., 2 + c:].any()
+    dy = rnd(n, 2 * d, 2 * h, 2 * w, c + 3)
+    sg.check(lib.coffee_up2_backward(ptr(dy), n, d, h, w, c, c + 3, 2, ptr(dx), stream))
+    parts = dy[..., 2:2 + c].double().reshape(n, d, 2, h, 2, w, 2, c)
+    assert bool(((dx - parts.sum((2, 4, 6))).abs() <=
+                 8 * 2 ** -24 * parts.abs().sum((2, 4, 6))).all())
+    dst = torch.zeros(n, d, h, w, c + 4, dtype=torch.bfloat16, device="cuda")
+    sg.check(lib.coffee_channels_copy(ptr(x), npts, c, ptr(dst), c + 4, 3, stream))
+    assert torch.equal(dst[..., 3:3 + c], x) and not dst[..., :3].any() and not dst[..., 3 + c:].any()
+    src = rnd(n, d, h, w, c + 4)
+    ref = dx.clone()
+    sg.check(lib.coffee_channels_add(ptr(src), npts, c + 4, 1, c, ptr(dx), stream))
+    assert torch.equal(dx, ref + src[..., 1:1 + c])
