@@ -314,11 +314,12 @@ __device__ __noinline__ V7<T> gr_absorb(const GrConst<T>& c, V7<T> v, V7<T> n, T
 // the absorbing layers: order of :876-893).  u: D, B, P of the current
 // buffer; eh: E, H of the same buffer.
 // Minimum resident 256-thread CTAs per SM of the stage and KO kernels: bound by the
-// latency of their stencil loads, they want warps until spilling costs more.  256^3
-// Wald run, one step, with (stage, KO) CTAs of (7, 6) / (6, 4) / (5, 5) / (4, 4): 6118
-// / 5555 / 5337 / 5335 us.
+// latency of their stencil loads, they want warps until spilling costs more.  Stage with
+// 4 / 5 / 6, us: 64^3 19.1 / 20.3 / 21.5, 128^3 129 / 131 / 130, 192^3 399 / 402 / 396,
+// 256^3 910 / 915 / 910; KO 14.7 / 15.4 / 18.0, 86 / 84 / 88, 258 / 250 / 255, 586 / 569
+// / 577.
 #ifndef COFFEE_GR_STAGE_MIN_BLOCKS
-#define COFFEE_GR_STAGE_MIN_BLOCKS 5
+#define COFFEE_GR_STAGE_MIN_BLOCKS 4
 #endif
 #ifndef COFFEE_GR_KO_MIN_BLOCKS
 #define COFFEE_GR_KO_MIN_BLOCKS 5
